@@ -19,6 +19,7 @@
 #include <thread>
 
 #include "ogx_harmonics.cuh"
+#include "ogx_m2l64.cuh"
 #include "ogx_sm100.cuh"
 
 namespace ogx {
@@ -69,40 +70,48 @@ struct HostOps {
     std::vector<double> m2l, m2m, l2l;
 };
 static std::mutex g_ops_mu;
-static std::map<int, std::shared_ptr<HostOps>> g_ops;
+static std::map<std::pair<int, bool>, std::shared_ptr<HostOps>> g_ops;
 
-static std::shared_ptr<HostOps> host_ops(int p) {
+// M2M and L2L of order p, or (m2l) its 343 M2L operators, which only the plain form reads
+static std::shared_ptr<HostOps> host_ops(int p, bool m2l) {
     std::lock_guard<std::mutex> lk(g_ops_mu);
-    auto it = g_ops.find(p);
+    auto it = g_ops.find({p, m2l});
     if (it != g_ops.end()) return it->second;
     const int K = num_dofs(p);
     auto ops = std::make_shared<HostOps>();
     std::vector<double> tmp((size_t)K * K);
-    auto put = [&](std::vector<double>& dst, int count, int kind) {
-        dst.assign((size_t)count * K * K, 0.0);
+    // k-major, rows of ld doubles, `rows` rows per operator (zero padded)
+    auto put = [&](std::vector<double>& dst, int count, int kind, int rows, int ld) {
+        dst.assign((size_t)count * rows * ld, 0.0);
         for (int idx = 0; idx < count; ++idx) {
             build_operator(kind, p, idx, tmp.data());
-            double* o = dst.data() + (size_t)idx * K * K;
+            double* o = dst.data() + (size_t)idx * rows * ld;
             for (int j = 0; j < K; ++j)
-                for (int k = 0; k < K; ++k) o[(size_t)k * K + j] = tmp[(size_t)j * K + k];
+                for (int k = 0; k < K; ++k) o[(size_t)k * ld + j] = tmp[(size_t)j * K + k];
         }
     };
-    put(ops->m2m, 8, 0);
-    put(ops->l2l, 8, 1);
-    put(ops->m2l, 343, 2);
-    g_ops[p] = ops;
+    if (m2l) {
+        put(ops->m2l, 343, 2, m2l64_pad_rows(p), m2l64_pad_cols(p));
+    } else {
+        put(ops->m2m, 8, 0, K, K);
+        put(ops->l2l, 8, 1, K, K);
+    }
+    g_ops[{p, m2l}] = ops;
     return ops;
 }
 
 int ensure_operator_tables(Handle& h) {
     if (h.ops_p == h.prm.p) return OGX_OK;
-    auto ops = host_ops(h.prm.p);
-    OGX_TRY(arena_get(h.ws, S_OPS_M2L, ops->m2l.size(), &h.d_m2l));
+    auto ops = host_ops(h.prm.p, false);
     OGX_TRY(arena_get(h.ws, S_OPS_M2M, ops->m2m.size(), &h.d_m2m));
     OGX_TRY(arena_get(h.ws, S_OPS_L2L, ops->l2l.size(), &h.d_l2l));
-    OGX_CUDA(upload_now(h.d_m2l, ops->m2l.data(), ops->m2l.size() * sizeof(double)));
     OGX_CUDA(upload_now(h.d_m2m, ops->m2m.data(), ops->m2m.size() * sizeof(double)));
     OGX_CUDA(upload_now(h.d_l2l, ops->l2l.data(), ops->l2l.size() * sizeof(double)));
+    if (h.prm.precision == OGX_PREC_FP64) {
+        auto m2l = host_ops(h.prm.p, true);
+        OGX_TRY(arena_get(h.ws, S_OPS_M2L, m2l->m2l.size(), &h.d_m2l));
+        OGX_CUDA(upload_now(h.d_m2l, m2l->m2l.data(), m2l->m2l.size() * sizeof(double)));
+    }
     h.ops_p = h.prm.p;
     return OGX_OK;
 }

@@ -7,11 +7,8 @@
 //   M2M           bottom-up in one launch (groups of parents taken level by level,
 //                 each waiting for its children), warp per child octant,
 //                 level-independent matrices MM_s (:62-71)
-//   M2L           all levels in one launch: targets grouped by their octant in
-//                 the parent, 64 per CTA; for each of the 189 (colleague slot,
-//                 child) combinations the sources of all 64 targets are gathered
-//                 into shared memory and multiplied by the offset's matrix T_o
-//                 (:78-81; V list implicit in the colleague slots)
+//   M2L           all levels in one launch on the FP64 matrix instructions
+//                 (ogx_m2l64.cu; :78-81; V list implicit in the colleague slots)
 //   P2L           warp per box over its X list (:82, :117-128)
 //   L2L           top-down in one launch, the same way (:75-77)
 //   leaf far      warp per leaf: L2P through gradient coefficients of L, M2P
@@ -28,6 +25,7 @@
 #include "ogx_harmonics.cuh"
 #include "ogx_expansion_kernels.cuh"
 #include "ogx_mixed_kernels.cuh"
+#include "ogx_m2l64.cuh"
 
 namespace ogx {
 
@@ -359,92 +357,6 @@ int launch_l2l(Handle& h, double* L, const double* Lown) {
     return launch_translate<P, 1>(h, S_TR_READY_L, nullptr, L, Lown);
 }
 
-// ---- M2L (structured, FP64) -----------------------------------------------------------
-constexpr int M2L_TGT = 64;
-constexpr int M2L_THREADS = 256;
-
-// One CTA = up to 64 targets that share their octant t inside the parent.
-template <int P>
-__global__ void __launch_bounds__(M2L_THREADS) k_m2l_fp64(TreeView tv, const uint32_t* tgt_key, const uint32_t* tgt_box,
-                                                         const double* opsT, const double* mpole, double* lown) {
-    constexpr int K = (P + 1) * (P + 1);
-    constexpr int LD = K | 1;
-    constexpr int NR = (K + 15) / 16;
-    extern __shared__ double s_m[];                      // [64][LD]
-    __shared__ int s_pcol[M2L_TGT][27];
-    __shared__ int s_src[M2L_TGT];
-    __shared__ int s_tgt[M2L_TGT];
-    __shared__ int s_t;
-    const int tid = threadIdx.x;
-    const int base = blockIdx.x * M2L_TGT;
-    if (tv_over(tv)) return;
-    // the padded target layout never mixes octants inside a tile
-    if (tid == 0) s_t = (tgt_key[base] == 0xFFFFFFFFu) ? -1 : (int)tgt_key[base];
-    __syncthreads();
-    const int t = s_t;
-    if (t < 0) return;
-    if (tid < M2L_TGT) {
-        const int i = base + tid;
-        const int b = ((int)tgt_key[i] == t) ? (int)tgt_box[i] : -1;
-        s_tgt[tid] = b;
-        const int P_ = (b >= 0) ? tv.parent[b] : -1;
-        for (int d = 0; d < 27; ++d) s_pcol[tid][d] = (P_ >= 0) ? tv.col[27 * P_ + d] : -1;
-    }
-    __syncthreads();
-    const int tx = t & 1, ty = (t >> 1) & 1, tz = (t >> 2) & 1;
-    const int tg = tid & 15, rg = tid >> 4;
-    double acc[4][NR];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int i = 0; i < NR; ++i) acc[a][i] = 0.0;
-    for (int D = 0; D < 27; ++D) {
-        const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
-        for (int s = 0; s < 8; ++s) {
-            const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
-            if (max(abs(ox), max(abs(oy), abs(oz))) <= 1) continue;  // adjacent: not in V
-            int mysrc = -1;
-            if (tid < M2L_TGT) {
-                const int Q = s_pcol[tid][D];
-                mysrc = (Q >= 0) ? tv.child[8 * Q + s] : -1;
-                s_src[tid] = mysrc;
-            }
-            if (!__syncthreads_or(mysrc >= 0)) continue;
-            for (int idx = tid; idx < M2L_TGT * K; idx += M2L_THREADS) {
-                const int r = idx / K, kk = idx - r * K;
-                const int src = s_src[r];
-                s_m[r * LD + kk] = (src >= 0) ? mpole[(size_t)src * K + kk] : 0.0;
-            }
-            __syncthreads();
-            const double* T = opsT + (size_t)((ox + 3) + 7 * (oy + 3) + 49 * (oz + 3)) * K * K;
-            for (int kk = 0; kk < K; ++kk) {
-                double mv[4];
-#pragma unroll
-                for (int a = 0; a < 4; ++a) mv[a] = s_m[(tg + 16 * a) * LD + kk];
-#pragma unroll
-                for (int i = 0; i < NR; ++i) {
-                    const int j = rg + 16 * i;
-                    const double tv_ = (j < K) ? __ldg(T + (size_t)kk * K + j) : 0.0;
-#pragma unroll
-                    for (int a = 0; a < 4; ++a) acc[a][i] = fma(tv_, mv[a], acc[a][i]);
-                }
-            }
-            __syncthreads();
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int b = s_tgt[tg + 16 * a];
-        if (b < 0) continue;
-        const double inv = 1.0 / (2.0 * tv.center[4 * b + 3]);
-#pragma unroll
-        for (int i = 0; i < NR; ++i) {
-            const int j = rg + 16 * i;
-            if (j < K) lown[(size_t)b * K + j] += acc[a][i] * inv;
-        }
-    }
-}
-
 // ---- leaf near field (P2P over U) + final combine ----------------------------------------
 // the leaf and first target of near-field work item w (leaf, chunk of 32 targets):
 // chunk_off[lf] <= w < chunk_off[lf + 1]; false past the last item
@@ -608,7 +520,6 @@ namespace {
 template <int P>
 int run_fp64(Handle& h, double* d_acc, double* d_pot) {
     constexpr int K = (P + 1) * (P + 1);
-    constexpr int LD = K | 1;
     const cudaStream_t st = h.stream;
     TreeView& tv = h.tv;
     OGX_TRY(harm_tables_ready(h.device));
@@ -631,10 +542,7 @@ int run_fp64(Handle& h, double* d_acc, double* d_pot) {
         // third form: the same V pairs through the rotation-factored operators (ogx_m2l_rot.cu)
         OGX_TRY(m2l_rot_launch(h, M, Lown));
     } else if (h.ntgt > 0) {
-        const size_t m2l_smem = (size_t)M2L_TGT * LD * sizeof(double);
-        OGX_CUDA(smem_optin((const void*)k_m2l_fp64<P>, (int)m2l_smem));
-        const int ntiles = h.ntgt_pad / M2L_TGT;
-        k_m2l_fp64<P><<<ntiles, M2L_THREADS, m2l_smem, st>>>(tv, h.tgt_tile_key, h.tgt_tile_box, h.d_m2l, M, Lown); ++h.launches;
+        OGX_TRY(m2l_fp64_launch(h, M, Lown));   // ogx_m2l64.cu
     }
     OGX_CUDA(timing_record(h, h.ev[4], st));
     // P2L
@@ -795,7 +703,6 @@ template <int P>
 int run_mixed_m2l(Handle& h, bool pot) {
     using C = mixed::TcCfg<P>;
     constexpr int K = (P + 1) * (P + 1);
-    constexpr int LD = K | 1;
     const cudaStream_t sm = h.m2l;
     TreeView& tv = h.tv;
     double *M, *Lown;
@@ -811,20 +718,13 @@ int run_mixed_m2l(Handle& h, bool pot) {
     OGX_CUDA(timing_record(h, h.ev[3], sm));
     OGX_CUDA(cudaMemsetAsync(Lown, 0, sizeof(double) * (size_t)tv.nb * K, sm));
     if (h.ntgt > 0) {
-        if constexpr (C::SUPPORTED) {
-            OGX_CUDA(smem_optin((const void*)mixed::k_m2l_tc<P>, C::SMEM));
-            mixed::k_m2l_tc<P><<<dim3(h.ntgt_pad / 128, C::NSPLIT), C::THREADS, C::SMEM, sm>>>(
-                tv, h.tgt_tile_key, h.tgt_tile_box, mhi, mlo, mus, h.d_tc_img, h.d_tc_ounscale, Lown, h.d_err); ++h.launches;
-            if (pot) {
-                mixed::k_m2l_dof0<P><<<(h.ntgt_pad + 127) / 128, 128, 0, sm>>>(tv, h.ntgt_pad, h.tgt_tile_key, h.tgt_tile_box,
-                                                                             h.d_tc_row0, M, Lown); ++h.launches;
-            }
-        } else {
-            // an order whose operand would not fit TMEM even in slices: the FP64 M2L serves it
-            const size_t m2l_smem = (size_t)M2L_TGT * LD * sizeof(double);
-            OGX_CUDA(smem_optin((const void*)k_m2l_fp64<P>, (int)m2l_smem));
-            k_m2l_fp64<P><<<h.ntgt_pad / M2L_TGT, M2L_THREADS, m2l_smem, sm>>>(tv, h.tgt_tile_key, h.tgt_tile_box, h.d_m2l, M,
-                                                                           Lown); ++h.launches;
+        static_assert(C::SUPPORTED, "every order's operand fits TMEM, in slices if need be");
+        OGX_CUDA(smem_optin((const void*)mixed::k_m2l_tc<P>, C::SMEM));
+        mixed::k_m2l_tc<P><<<dim3(h.ntgt_pad / 128, C::NSPLIT), C::THREADS, C::SMEM, sm>>>(
+            tv, h.tgt_tile_key, h.tgt_tile_box, mhi, mlo, mus, h.d_tc_img, h.d_tc_ounscale, Lown, h.d_err); ++h.launches;
+        if (pot) {
+            mixed::k_m2l_dof0<P><<<(h.ntgt_pad + 127) / 128, 128, 0, sm>>>(tv, h.ntgt_pad, h.tgt_tile_key, h.tgt_tile_box,
+                                                                         h.d_tc_row0, M, Lown); ++h.launches;
         }
     }
     OGX_CUDA(timing_record(h, h.ev[4], sm));

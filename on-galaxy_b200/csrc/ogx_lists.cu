@@ -23,6 +23,7 @@
 
 #include "ogx_tree_common.cuh"
 #include "ogx_softening.cuh"
+#include "ogx_m2l64.cuh"
 
 namespace ogx {
 namespace {
@@ -285,7 +286,7 @@ __global__ void k_tgt_keys(int cap, const int* __restrict__ level_off, const int
 // padded per-octant layout of the M2L targets (sorted by k_tgt_keys' key, octant in
 // bits 27-29): every octant group starts on a multiple of `tile`, so a tile never
 // mixes octants.  gs[0..8] = group starts,
-// gs[9..17] = padded group starts.
+// gs[9..17] = padded group starts, then the FP64 M2L's work split (ogx_m2l64.cuh).
 __global__ void k_target_groups(const uint32_t* key, const DevCounts* counts, int tile, int fill, int* gs) {
     __shared__ int lo_s[9];
     const int g = threadIdx.x;
@@ -306,6 +307,12 @@ __global__ void k_target_groups(const uint32_t* key, const DevCounts* counts, in
             gs[9 + q] = pad;
             if (q < 8) pad += ((lo_s[q + 1] - lo_s[q] + fill - 1) / fill) * tile;
         }
+        int tiles64 = 0;
+        for (int q = 0; q < 8; ++q) tiles64 += (lo_s[q + 1] - lo_s[q] + M2L64_TGT - 1) / M2L64_TGT;
+        gs[GS_SPLIT] = max(1, min(M2L64_MAXSPLIT, (M2L64_ITEMS + tiles64 - 1) / max(tiles64, 1)));
+        gs[GS_TILES] = pad / M2L64_TGT;
+        gs[GS_TICKET] = 0;
+        gs[GS_FILL] = fill;
     }
 }
 // slot q of a padded group holds target (q - start) / tile * fill + (q - start) % tile
@@ -478,6 +485,7 @@ int lists_build_targets(Handle& h) {
     OGX_TRY(arena_get(h.ws, S_TGT_PBOX, npad, &pb));
     k_target_groups<<<1, 32, 0, h.aux>>>(tk_s, dc, tile, fill, gs); ++h.launches;
     k_target_pad<<<grid_for(npad, 256), 256, 0, h.aux>>>(tb_s, gs, npad, tile, fill, pk, pb); ++h.launches;
+    h.tgt_groups = gs;
     h.tgt_tile_key = pk;
     h.tgt_tile_box = pb;
     h.ntgt_pad = npad;

@@ -7,18 +7,18 @@
 // slot, child) combinations as the plain form's k_m2l_fp64.  Kept in a file of its
 // own: the fully unrolled blocks of twelve orders take minutes to compile, and the
 // build then runs it beside the other units.
+#include <algorithm>
 #include <memory>
 #include <mutex>
 #include <utility>
 #include <vector>
 
-#include "ogx_internal.cuh"
+#include "ogx_m2l64.cuh"
 
 namespace ogx {
 namespace {
 
-// targets per CTA; the target tiles are padded to multiples of 128, so 64 divides them
-constexpr int ROT_TGT = 64;
+constexpr int ROT_TGT = M2L64_TGT;   // targets per CTA
 
 // ---- M2L by rotations (the third form) ------------------------------------------------
 // T_o = Q_o^-1 Z_|o| Q_o (build_rot_pack): per tile of ROT_TGT targets sharing octant t
@@ -147,80 +147,91 @@ __device__ __forceinline__ void rot_ord_stage(std::integer_sequence<int, Ms...>,
     ((RotCfg<P>::ord_group(Ms) == g ? rot_ord_block<P, Ms>(Z, y_in, z_out) : void()), ...);
 }
 
+// Work items and split sums as in the plain form (ogx_m2l64.cuh): a small tree's tiles are
+// cut into ranges of colleague slots so that they fill the SMs.
 template <int P>
-__global__ void __launch_bounds__(RotCfg<P>::THREADS) k_m2l_rot(TreeView tv, const uint32_t* tgt_key, const uint32_t* tgt_box,
-                                                        const double* __restrict__ pack, const double* __restrict__ mpole,
-                                                        double* lown) {
+__global__ void __launch_bounds__(RotCfg<P>::THREADS) k_m2l_rot(TreeView tv, M2L64Args ar, const double* __restrict__ pack,
+                                                        const double* __restrict__ mpole, double* lown) {
     using R = RotCfg<P>;
     constexpr int K = R::K, LD = R::LD, RB = R::RB, TH = R::THREADS;
     extern __shared__ double s_rot[];
     double* s_m = s_rot;                    // [64][LD] sources, later z
     double* s_y = s_rot + ROT_TGT * LD;     // [64][LD] y = Q m
-    __shared__ int s_pcol[ROT_TGT][27];
+    __shared__ int s_pcol[27][ROT_TGT];
     __shared__ int s_src[ROT_TGT];
     __shared__ int s_tgt[ROT_TGT];
-    __shared__ int s_t;
+    __shared__ int s_item;
     const int tid = threadIdx.x;
     const int ga = tid / R::ROWS, ra = tid % R::ROWS;   // block group; rows ra, ra + ROWS, ...
-    const int base = blockIdx.x * ROT_TGT;
     if (tv_over(tv)) return;
-    if (tid == 0) s_t = (tgt_key[base] == 0xFFFFFFFFu) ? -1 : (int)tgt_key[base];
-    __syncthreads();
-    const int t = s_t;
-    if (t < 0) return;
-    if (tid < ROT_TGT) {
-        const int i = base + tid;
-        const int b = ((int)tgt_key[i] == t) ? (int)tgt_box[i] : -1;
-        s_tgt[tid] = b;
-        const int P_ = (b >= 0) ? tv.parent[b] : -1;
-        for (int d = 0; d < 27; ++d) s_pcol[tid][d] = (P_ >= 0) ? tv.col[27 * P_ + d] : -1;
-    }
-    __syncthreads();
-    const int tx = t & 1, ty = (t >> 1) & 1, tz = (t >> 2) & 1;
-    double acc[RB][R::NACC];
-#pragma unroll
-    for (int q = 0; q < RB; ++q)
-#pragma unroll
-        for (int i = 0; i < R::NACC; ++i) acc[q][i] = 0.0;
-    using Seq = std::make_integer_sequence<int, P + 1>;
-    for (int D = 0; D < 27; ++D) {
-        const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
-        for (int s = 0; s < 8; ++s) {
-            const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
-            if (max(abs(ox), max(abs(oy), abs(oz))) <= 1) continue;  // adjacent: not in V
-            int mysrc = -1;
-            if (tid < ROT_TGT) {
-                const int Q = s_pcol[tid][D];
-                mysrc = (Q >= 0) ? tv.child[8 * Q + s] : -1;
-                s_src[tid] = mysrc;
-            }
-            if (!__syncthreads_or(mysrc >= 0)) continue;
-            for (int idx = tid; idx < ROT_TGT * K; idx += TH) {
-                const int r = idx / K, kk = idx - r * K;
-                const int src = s_src[r];
-                s_m[r * LD + kk] = (src >= 0) ? mpole[(size_t)src * K + kk] : 0.0;
-            }
-            __syncthreads();
-            const double* pk = pack + (size_t)((ox + 3) + 7 * (oy + 3) + 49 * (oz + 3)) * R::PACK;
-            rot_deg_stage<P, true>(Seq{}, ga, pk, s_m + ra * LD, s_y + ra * LD, acc);              // y = Q m
-            __syncthreads();
-            rot_ord_stage<P>(Seq{}, ga, pk + 2 * R::QSZ, s_y + ra * LD, s_m + ra * LD);            // z = Z y
-            __syncthreads();
-            rot_deg_stage<P, false>(Seq{}, ga, pk + R::QSZ, s_m + ra * LD, nullptr, acc);          // acc += Q^-1 z
-            __syncthreads();
+    const int S = ar.gs[GS_SPLIT], tiles = ar.gs[GS_TILES];
+    const int ntgt = tv.cnt->ntgt32;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s_item = atomicAdd(ar.gs + GS_TICKET, 1);
+        __syncthreads();
+        const int item = s_item;
+        if (item >= tiles * S) return;
+        const int zr = item / tiles, base = (item - zr * tiles) * ROT_TGT;
+        const int t = (int)ar.tgt_key[base];
+        if (t < 0) continue;
+        const int D0 = m2l64_first_slot(zr, S, t), D1 = m2l64_first_slot(zr + 1, S, t);
+        if (tid < ROT_TGT) s_tgt[tid] = ((int)ar.tgt_key[base + tid] == t) ? (int)ar.tgt_box[base + tid] : -1;
+        __syncthreads();
+        for (int i = tid; i < (D1 - D0) * ROT_TGT; i += TH) {
+            const int D = D0 + i / ROT_TGT, r = i % ROT_TGT, b = s_tgt[r];
+            s_pcol[D][r] = b >= 0 ? tv.col[27 * (size_t)tv.parent[b] + D] : -1;
         }
-    }
+        __syncthreads();
+        const int tx = t & 1, ty = (t >> 1) & 1, tz = (t >> 2) & 1;
+        double acc[RB][R::NACC];
 #pragma unroll
-    for (int q = 0; q < RB; ++q) {
-        const int b = s_tgt[ra + q * R::ROWS];
-        if (b < 0) continue;
-        const double inv = 1.0 / (2.0 * tv.center[4 * b + 3]);
+        for (int q = 0; q < RB; ++q)
 #pragma unroll
-        for (int n = 0; n <= P; ++n) {
-            if (R::deg_group(n) != ga) continue;
-            const int pos = R::deg_pos(n);
+            for (int i = 0; i < R::NACC; ++i) acc[q][i] = 0.0;
+        using Seq = std::make_integer_sequence<int, P + 1>;
+        for (int D = D0; D < D1; ++D) {
+            const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
+            for (int s = 0; s < 8; ++s) {
+                const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
+                if (max(abs(ox), max(abs(oy), abs(oz))) <= 1) continue;  // adjacent: not in V
+                int mysrc = -1;
+                if (tid < ROT_TGT) {
+                    const int Q = s_pcol[D][tid];
+                    mysrc = (Q >= 0) ? tv.child[8 * Q + s] : -1;
+                    s_src[tid] = mysrc;
+                }
+                if (!__syncthreads_or(mysrc >= 0)) continue;
+                for (int idx = tid; idx < ROT_TGT * K; idx += TH) {
+                    const int r = idx / K, kk = idx - r * K;
+                    const int src = s_src[r];
+                    s_m[r * LD + kk] = (src >= 0) ? mpole[(size_t)src * K + kk] : 0.0;
+                }
+                __syncthreads();
+                const double* pk = pack + (size_t)((ox + 3) + 7 * (oy + 3) + 49 * (oz + 3)) * R::PACK;
+                rot_deg_stage<P, true>(Seq{}, ga, pk, s_m + ra * LD, s_y + ra * LD, acc);              // y = Q m
+                __syncthreads();
+                rot_ord_stage<P>(Seq{}, ga, pk + 2 * R::QSZ, s_y + ra * LD, s_m + ra * LD);            // z = Z y
+                __syncthreads();
+                rot_deg_stage<P, false>(Seq{}, ga, pk + R::QSZ, s_m + ra * LD, nullptr, acc);          // acc += Q^-1 z
+                __syncthreads();
+            }
+        }
 #pragma unroll
-            for (int r = 0; r < 2 * n + 1; ++r) lown[(size_t)b * K + n * n + r] += acc[q][pos + r] * inv;
+        for (int q = 0; q < RB; ++q) {
+            const int r0 = ra + q * R::ROWS, b = s_tgt[r0];
+            if (b < 0) continue;
+            const int pq = base + r0 - ar.gs[9 + t];
+            const int64_t j = ar.gs[t] + (int64_t)(pq / 128) * ar.gs[GS_FILL] + pq % 128;   // sorted target
+            double* o = S == 1 ? lown + (size_t)b * K : ar.part + ((size_t)zr * ntgt + j) * K;
+            const double sc = S == 1 ? 1.0 / (2.0 * tv.center[4 * b + 3]) : 1.0;
+#pragma unroll
+            for (int n = 0; n <= P; ++n) {
+                if (R::deg_group(n) != ga) continue;
+                const int pos = R::deg_pos(n);
+#pragma unroll
+                for (int r = 0; r < 2 * n + 1; ++r) o[n * n + r] = acc[q][pos + r] * sc;
+            }
         }
     }
 }
@@ -256,11 +267,20 @@ int launch_rot(Handle& h, const double* M, double* Lown) {
     OGX_TRY(ensure_rot_tables<P>(h));
     constexpr size_t rsm = RotCfg<P>::SMEM;
     OGX_CUDA(smem_optin((const void*)k_m2l_rot<P>, (int)rsm));
-    k_m2l_rot<P><<<h.ntgt_pad / ROT_TGT, RotCfg<P>::THREADS, rsm, h.stream>>>(h.tv, h.tgt_tile_key, h.tgt_tile_box,
-                                                                               h.d_rot, M, Lown);
+    M2L64Args a;
+    OGX_TRY(m2l64_args(h, &a));
+    static const int per_sm = [] {
+        int b = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_m2l_rot<P>, RotCfg<P>::THREADS, rsm) != cudaSuccess) {
+            cudaGetLastError();
+            b = 1;
+        }
+        return std::max(1, b);
+    }();
+    const int grid = (int)std::min<int64_t>((int64_t)(h.ntgt_pad / ROT_TGT) * M2L64_MAXSPLIT, (int64_t)per_sm * h.num_sms);
+    k_m2l_rot<P><<<grid, RotCfg<P>::THREADS, rsm, h.stream>>>(h.tv, a, h.d_rot, M, Lown);
     ++h.launches;
-    OGX_CUDA(cudaGetLastError());
-    return OGX_OK;
+    return m2l64_sum_launch(h, a, Lown, h.stream);
 }
 
 }  // namespace
