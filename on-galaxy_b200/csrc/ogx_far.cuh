@@ -1,0 +1,539 @@
+// ogx_far.cuh -- the leaf far field: L2P and, over the W lists, M2P (float in the mixed
+// form, double in the plain form).
+//
+// Replaces fmm::localField / fmm::multipoleField per body (src3d/FmmExpansions3D.hpp:180-235,
+// called in src3d/AdaptiveFMM3D.hpp:92-93).  The gradient of an expansion is a sum of solid
+// harmonics with three coefficient sets H^x, H^y, H^z, and a solid harmonic of order m is a
+// complex factor of m alone times a REAL polynomial of z and r^2:
+//   R_n^m = s_nm (x+iy)^m T_nm(z, r^2)             S_n^m(u) = R_n^m(u / r^2) / r
+//   T_mm = 1, T_{m+1,m} = z, T_nm = z T_{n-1,m} - b_nm r^2 T_{n-2,m},
+//   b_nm = ((n-1)^2 - m^2) / ((2n-1)(2n-3))        (the recurrences of ogx_harmonics.cuh
+// with the constants A_nm collected in s_nm).  The constants s_nm are folded into the
+// coefficient records, so per (n, m) an evaluation takes three operations for T_nm and two
+// per axis (real and imaginary coefficient); the complex factor is applied once per m.
+// With complex harmonics it took six, and an M2P evaluation at p = 8 about 800 instructions.
+// In FP32 two columns m, m + 1 go together in packed pairs (f32x2: the FMA pipe's rate at
+// half the issue slots): step i of the pair is T_{m+i,m} and T_{m+1+i,m+1}.
+// Bound: FP32 issue slots (the records come from shared memory as warp-wide broadcasts).
+// M2P + L2P of the 1M merger (p = 8, 14.4M evaluations, serialised): 1.33 -> 0.79 ms; in
+// FP64 the 262,144-body galaxy: 1.30 -> 0.41 ms (one warp per leaf had walked the W list
+// of a leaf in turn, 199 boxes at most).
+#pragma once
+
+#include "ogx_harmonics.cuh"
+#include "ogx_sm100.cuh"
+
+namespace ogx {
+namespace far {
+
+// largest degree of a record: M2P gradients reach P + 1, L2P gradients P - 1 (potential P)
+template <int P, int MODE, bool POT>
+constexpr int rec_degree() { return MODE == 0 ? P + 1 : (POT ? P : P - 1); }
+
+// values of a record: FP32 steps of column pairs (12 or 16 floats), FP64 entries per (n, m)
+// column by column (6 or 8 doubles): {gx.re, gx.im, gy.re, gy.im, gz.re, gz.im(, phi.re, phi.im)}
+template <class T, int L, bool POT>
+struct Rec {
+    static constexpr bool PAIR = sizeof(T) == 4;
+    static constexpr int V = POT ? 8 : 6;
+    static constexpr int entries() {
+        if (!PAIR) return (L + 1) * (L + 2) / 2;
+        int s = 0;
+        for (int m = 0; m <= L; m += 2) s += L - m + 1;
+        return s;
+    }
+    static constexpr int STEPS = entries();
+    static constexpr int SIZE = STEPS * V * (PAIR ? 2 : 1);      // values of T
+    static constexpr int F4 = SIZE * (int)sizeof(T) / 16;        // 16-byte pieces
+    static_assert(SIZE * sizeof(T) % 16 == 0, "records are copied in 16-byte pieces");
+};
+
+// Both parts (re, im) of entry (n, m) of a gradient coefficient set (FmmExpansions3D.hpp:111-129)
+//   MODE 0: multipole set H from M_{n-1} (dz_S / dp_S / dm_S)
+//   MODE 1: local set G from L_{n+1}     (cz_R / cp_R / cm_R)
+// (constants from global memory: the lanes hold different (n, m))
+template <int MODE>
+__device__ __forceinline__ void grad_entry(const double* c, int n, int m, double gr[3], double gi[3]) {
+    if (MODE == 0 && n == 0) return;
+    const int N = MODE == 0 ? n - 1 : n + 1;
+    double lr, li, pr, pi, mr, mi;
+    coef_get(c, N, m, lr, li);
+    coef_get(c, N, m - 1, mr, mi);
+    coef_get(c, N, m + 1, pr, pi);
+    const double cz = __ldg(MODE == 0 ? &g_harm.hz[n][m] : &g_harm.gz[n][m]);
+    const double cp = __ldg(MODE == 0 ? &g_harm.hp[n][m] : &g_harm.gp[n][m]);
+    const double cm = __ldg(MODE == 0 ? &g_harm.hm[n][m] : &g_harm.gm[n][m]);
+    const double xr = 0.5 * (cp * mr + cm * pr), xi = 0.5 * (cp * mi + cm * pi);
+    const double dr = cp * mr - cm * pr, di = cp * mi - cm * pi;
+    gr[0] = xr; gr[1] = 0.5 * di; gr[2] = cz * lr;
+    if (m > 0) { gi[0] = xi; gi[1] = -0.5 * dr; gi[2] = cz * li; }
+}
+
+// Coefficient records, warp per box (MODE 0, boxes of some W list) or leaf (MODE 1).  The
+// weights are folded in (m = 0: (c.re, 0); m > 0: (2 c.re, -2 c.im)), so that
+// sum_nm Re(c_nm z_nm) = sum re' z.re + im' z.im.
+template <int P, int MODE, bool POT, class T>
+__global__ void __launch_bounds__(128) k_far_rec(TreeView tv, int count, const double* __restrict__ coef, T* __restrict__ rec) {
+    constexpr int K = (P + 1) * (P + 1), L = rec_degree<P, MODE, POT>();
+    using R = Rec<T, L, POT>;
+    const int lane = threadIdx.x & 31;
+    const int k = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (k >= count || k >= (MODE == 0 ? tv_nb(tv) : tv_nleaf(tv)) || tv_over(tv)) return;
+    const int b = (MODE == 0) ? k : tv.leafbox[k];
+    if (MODE == 0 && tv.x_off[b] == tv.x_off[b + 1]) return;   // never an M2P source
+    const double* c = coef + (size_t)b * K;
+    T* o = rec + (size_t)k * R::SIZE;
+    for (int e = lane; e < R::STEPS * (R::PAIR ? 2 : 1); e += 32) {
+        // entry e: column m, step i (n = m + i); FP32: half of column pair m0
+        const int half = R::PAIR ? (e & 1) : 0;
+        int i = R::PAIR ? (e >> 1) : e, m = 0;
+        while (i > L - m) { i -= L - m + 1; m += R::PAIR ? 2 : 1; }
+        m += half;
+        const int n = m + i;
+        double gr[3] = {0.0, 0.0, 0.0}, gi[3] = {0.0, 0.0, 0.0}, pr = 0.0, pi = 0.0;
+        if (n <= L) {
+            if (MODE == 0 || n < P) grad_entry<MODE>(c, n, m, gr, gi);
+            if (POT && n <= P) {
+                pr = c[dof_re(n, m)];
+                if (m > 0) pi = c[dof_re(n, m) + 1];
+            }
+        }
+        const double s = n <= L ? __ldg(&g_harm.s[n][m]) : 0.0;
+        const double wr = m == 0 ? s : 2.0 * s, wi = m == 0 ? 0.0 : -2.0 * s;
+        const double v[8] = {wr * gr[0], wi * gi[0], wr * gr[1], wi * gi[1], wr * gr[2], wi * gi[2], wr * pr, wi * pi};
+        constexpr int ST = R::PAIR ? 2 : 1;
+        T* q = o + (size_t)(R::PAIR ? (e >> 1) : e) * R::V * ST + half;
+#pragma unroll
+        for (int a = 0; a < R::V; ++a) q[a * ST] = (T)v[a];
+    }
+}
+
+__host__ __device__ constexpr double rec_b(int n, int m) {
+    return (double)((n - 1) * (n - 1) - m * m) / (double)((2 * n - 1) * (2 * n - 3));
+}
+
+// ---- packed FP32 pairs
+struct f2 { unsigned long long v; };
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float sum2(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return x + y;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
+// out = {sum_axis x, y, z(, phi)} of one body at scaled offset (x, y, z) for a record in
+// shared memory; SING: singular harmonics (M2P), else regular (L2P)
+template <int L, bool POT, bool SING>
+__device__ __forceinline__ void eval(const float4* rec, float x, float y, float z, float (&out)[4]) {
+    using R = Rec<float, L, POT>;
+    float kap = x * x + y * y + z * z, d0 = 1.f;
+    if (SING) {
+        d0 = rsqrtf(kap);
+        kap = d0 * d0;
+        x *= kap; y *= kap; z *= kap;
+    }
+    const f2 z2 = pack2(z, z), nk2 = pack2(-kap, -kap);
+    // (x + iy)^2 carries a column pair to the next
+    const float qr = x * x - y * y, qi = 2.f * x * y;
+    const f2 qr2 = pack2(qr, qr), qi2 = pack2(qi, qi), nqi2 = pack2(-qi, -qi);
+    f2 dr = pack2(d0, d0 * x), di = pack2(0.f, d0 * y);
+    f2 o[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) o[a].v = 0ull;
+    const ulonglong2* r = reinterpret_cast<const ulonglong2*>(rec);
+    int e = 0;
+#pragma unroll
+    for (int m = 0; m <= L; m += 2) {
+        f2 s[R::V], t0 = pack2(1.f, 1.f), t1 = z2;
+#pragma unroll
+        for (int i = 0; i <= L - m; ++i, ++e) {
+            f2 c[R::V], t = t1;
+#pragma unroll
+            for (int a = 0; a < R::V / 2; ++a) {
+                const ulonglong2 w = r[e * (R::V / 2) + a];
+                c[2 * a].v = w.x;
+                c[2 * a + 1].v = w.y;
+            }
+            if (i == 0) {
+#pragma unroll
+                for (int a = 0; a < R::V; ++a) s[a] = c[a];
+                continue;
+            }
+            if (i >= 2) {
+                const f2 b = pack2((float)rec_b(m + i, m), (float)rec_b(m + 1 + i, m + 1));
+                t = fma2(z2, t1, mul2(mul2(b, nk2), t0));
+                t0 = t1;
+                t1 = t;
+            }
+#pragma unroll
+            for (int a = 0; a < R::V; ++a) s[a] = fma2(c[a], t, s[a]);
+        }
+#pragma unroll
+        for (int a = 0; a < R::V / 2; ++a) o[a] = fma2(s[2 * a], dr, fma2(s[2 * a + 1], di, o[a]));
+        if (m + 2 <= L) {
+            const f2 nr = fma2(dr, qr2, mul2(di, nqi2));
+            di = fma2(dr, qi2, mul2(di, qr2));
+            dr = nr;
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) out[a] = a < R::V / 2 ? sum2(o[a]) : 0.f;
+}
+
+template <int L, bool POT, bool SING>
+__device__ __forceinline__ void eval(const float4* rec, double x, double y, double z, double (&out)[4]) {
+    using R = Rec<double, L, POT>;
+    double kap = x * x + y * y + z * z, dr = 1.0, di = 0.0;
+    if (SING) {
+        dr = rsqrt(kap);
+        kap = dr * dr;
+        x *= kap; y *= kap; z *= kap;
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) out[a] = 0.0;
+    const double2* r = reinterpret_cast<const double2*>(rec);
+    int e = 0;
+#pragma unroll
+    for (int m = 0; m <= L; ++m) {
+        double s[R::V], t0 = 1.0, t1 = z;
+#pragma unroll
+        for (int i = 0; i <= L - m; ++i, ++e) {
+            double c[R::V], t = t1;
+#pragma unroll
+            for (int a = 0; a < R::V / 2; ++a) {
+                const double2 w = r[e * (R::V / 2) + a];
+                c[2 * a] = w.x;
+                c[2 * a + 1] = w.y;
+            }
+            if (i == 0) {
+#pragma unroll
+                for (int a = 0; a < R::V; ++a) s[a] = c[a];
+                continue;
+            }
+            if (i >= 2) {
+                t = fma(z, t1, -(rec_b(m + i, m) * kap) * t0);
+                t0 = t1;
+                t1 = t;
+            }
+#pragma unroll
+            for (int a = 0; a < R::V; ++a)
+                if (m > 0 || !(a & 1)) s[a] = fma(c[a], t, s[a]);   // order 0 is real
+        }
+#pragma unroll
+        for (int a = 0; a < R::V / 2; ++a) out[a] = fma(s[2 * a], dr, m > 0 ? fma(s[2 * a + 1], di, out[a]) : out[a]);
+        if (m < L) {
+            const double nr = dr * x - di * y;
+            di = dr * y + di * x;
+            dr = nr;
+        }
+    }
+}
+
+// ---- tasks: the (body, W box) pairs of a block of at most 64 bodies, W-major, taken in
+// rounds of at most 32 (lane = task).  A round covers at most RW W boxes, whose records
+// one warp stages in shared memory.
+template <class T> struct Res;
+template <> struct Res<float> { using V = float4; };
+template <> struct Res<double> { using V = double4; };
+
+constexpr int FAR_RW = 3;          // boxes of a round: 32 tasks of leaves of 16 bodies and more span at most 3
+constexpr int FAR_HW = 8;          // warps of a heavy leaf's CTA
+
+// Leaves with more M2P tasks (bodies x W boxes) than this are taken by a CTA of FAR_HW
+// warps (k_leaf_far_heavy), so that one leaf with a long W list does not decide the
+// kernel's length.  In small trees (fewer leaves than warps the GPU holds) and in FP64 a
+// task costs more of the kernel's length, so the line is lower.
+template <class T>
+__device__ __forceinline__ int64_t heavy_line(const TreeView& tv) { return sizeof(T) == 8 || tv_nleaf(tv) < 4096 ? 256 : 1024; }
+
+// shared memory of one warp
+template <int P, bool POT, class T>
+struct alignas(16) WarpSmem {
+    static constexpr int RF4 = Rec<T, P + 1, POT>::F4;
+    float4 rec[FAR_RW * RF4];
+    typename Res<T>::V res[32];
+    double hdr[FAR_RW][4];       // FP64: box centre, 1 / side; FP32: floats {offset xyz, scale, 1 / side}
+};
+
+// bodies of a block relative to the leaf centre: FP64 (x - c); FP32 ((x - c) / side) as hi + lo
+template <class T> struct Bodies;
+template <> struct Bodies<double> { double x[3][64]; };
+template <> struct Bodies<float> { float h[3][64], l[3][64]; };
+
+__device__ __forceinline__ void put_body(Bodies<double>& s, int j, double x, double y, double z, double) {
+    s.x[0][j] = x; s.x[1][j] = y; s.x[2][j] = z;
+}
+__device__ __forceinline__ void put_body(Bodies<float>& s, int j, double x, double y, double z, double inv) {
+    const double v[3] = {x * inv, y * inv, z * inv};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float h = (float)v[a];
+        s.h[a][j] = h;
+        s.l[a][j] = (float)(v[a] - (double)h);
+    }
+}
+
+// W box header, written by one lane per box.  FP32: the box's centre offset from the leaf in
+// its own side (a small dyadic number, exact), and the ratio of the sides (a power of two)
+__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double,
+                                           double) {
+    h[0] = cx - c01.x; h[1] = cy - c01.y; h[2] = cz - c23.x; h[3] = 1.0 / (2.0 * c23.y);
+}
+__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double side,
+                                           float) {
+    float* f = reinterpret_cast<float*>(h);
+    const double winv = 1.0 / (2.0 * c23.y);
+    f[0] = (float)((cx - c01.x) * winv);
+    f[1] = (float)((cy - c01.y) * winv);
+    f[2] = (float)((cz - c23.x) * winv);
+    f[3] = (float)(side * winv);
+    f[4] = (float)winv;
+}
+
+template <int L, bool POT>
+__device__ __forceinline__ double4 m2p_task(const float4* rec, const double (&h)[4], const Bodies<double>& s, int j) {
+    const double w = h[3];
+    double o[4];
+    eval<L, POT, true>(rec, (s.x[0][j] + h[0]) * w, (s.x[1][j] + h[1]) * w, (s.x[2][j] + h[2]) * w, o);
+    const double w2 = w * w;
+    return make_double4(o[0] * w2, o[1] * w2, o[2] * w2, POT ? o[3] * w : 0.0);
+}
+template <int L, bool POT>
+__device__ __forceinline__ float4 m2p_task(const float4* rec, const double (&hd)[4], const Bodies<float>& s, int j) {
+    const float* h = reinterpret_cast<const float*>(hd);
+    const float sc = h[3], w = h[4];
+    float u[3], o[4];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) u[a] = fmaf(s.l[a][j], sc, fmaf(s.h[a][j], sc, h[a]));
+    eval<L, POT, true>(rec, u[0], u[1], u[2], o);
+    const float w2 = w * w;
+    return make_float4(o[0] * w2, o[1] * w2, o[2] * w2, POT ? o[3] * w : 0.f);
+}
+
+// The rounds first, first + stride, ... of a block of nbk bodies and nw W boxes; every body
+// sums its own task results in task order into acc (FP64; lane owns bodies lane, lane + 32).
+template <int P, bool POT, class T>
+__device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restrict__ hrec, int64_t w0, int nw, int nbk, int first,
+                                           int stride, const Bodies<T>& sb, double cx, double cy, double cz, double side,
+                                           WarpSmem<P, POT, T>& sm, int lane, double (&acc)[2][4]) {
+    using R = Rec<T, P + 1, POT>;
+    constexpr int RF4 = R::F4;
+    const int total = nbk * nw;
+    // tasks of a round: at most FAR_RW boxes (whole ones for leaves of fewer than 16 bodies)
+    const int Q = nbk >= 16 ? 32 : (FAR_RW * nbk <= 32 ? FAR_RW : FAR_RW - 1) * nbk;
+    int b0 = first * Q;
+    // this lane's task: box w, body j
+    int w = (b0 + lane) / nbk, j = b0 + lane - w * nbk;
+    const int dq = stride * Q / nbk, dr = stride * Q - dq * nbk;
+    for (; b0 < total; b0 += stride * Q) {
+        const int nt = min(Q, total - b0);
+        const int wa = __shfl_sync(0xffffffffu, w, 0), nrec = __shfl_sync(0xffffffffu, w, nt - 1) - wa + 1;
+        const int ja = __shfl_sync(0xffffffffu, j, 0);
+        int c = 0;
+        if (lane < nrec) c = tv.w_idx[w0 + wa + lane];
+        for (int q = 0; q < nrec; ++q) {
+            const float4* src = reinterpret_cast<const float4*>(hrec + (size_t)__shfl_sync(0xffffffffu, c, q) * R::SIZE);
+#pragma unroll
+            for (int i = 0; i < (RF4 + 31) / 32; ++i)
+                if (32 * i + lane < RF4) sm100::cp_async16(sm.rec + q * RF4 + 32 * i + lane, src + 32 * i + lane);
+        }
+        if (lane < nrec) {
+            const double2 c01 = __ldg(reinterpret_cast<const double2*>(tv.center) + 2 * (size_t)c);
+            const double2 c23 = __ldg(reinterpret_cast<const double2*>(tv.center) + 2 * (size_t)c + 1);
+            put_header(sm.hdr[lane], c01, c23, cx, cy, cz, side, T(0));
+        }
+        sm100::cp_async_wait_all();
+        __syncwarp();
+        if (lane < nt) sm.res[lane] = m2p_task<P + 1, POT>(sm.rec + (w - wa) * RF4, sm.hdr[w - wa], sb, j);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int jo = lane + 32 * q;
+            if (jo < nbk) {
+                for (int k = jo >= ja ? jo - ja : jo - ja + nbk; k < nt; k += nbk) {
+                    const auto v = sm.res[k];
+                    acc[q][0] += v.x; acc[q][1] += v.y; acc[q][2] += v.z;
+                    if (POT) acc[q][3] += v.w;
+                }
+            }
+        }
+        __syncwarp();   // the next round's copies overwrite the records and results
+        w += dq;
+        j += dr;
+        if (j >= nbk) { j -= nbk; ++w; }
+    }
+}
+
+// L2P of the block's bodies (lane owns bodies lane and lane + 32)
+template <int P, bool POT, class T>
+__device__ __forceinline__ void l2p_block(const T* __restrict__ g, int nbk, const Bodies<T>& sb, double inv, float4* srec, int lane,
+                                          double (&acc)[2][4]) {
+    constexpr int L = rec_degree<P, 1, POT>();
+    using R = Rec<T, L, POT>;
+    __syncwarp();
+    for (int i = lane; i < R::F4; i += 32) srec[i] = __ldg(reinterpret_cast<const float4*>(g) + i);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int j = lane + 32 * q;
+        if (j < nbk) {
+            T o[4];
+            if constexpr (sizeof(T) == 4) eval<L, POT, false>(srec, sb.h[0][j], sb.h[1][j], sb.h[2][j], o);
+            else eval<L, POT, false>(srec, sb.x[0][j] * inv, sb.x[1][j] * inv, sb.x[2][j] * inv, o);
+            acc[q][0] += (double)o[0] * inv;
+            acc[q][1] += (double)o[1] * inv;
+            acc[q][2] += (double)o[2] * inv;
+            if (POT) acc[q][3] += (double)o[3];
+        }
+    }
+    __syncwarp();
+}
+
+// Warp per leaf (one warp per block, so a block's resources return as soon as its leaf is
+// done), bodies in blocks of 64.  The mixed form runs the two parts apart: M2P (DO_M2P,
+// multipoles only) beside the M2L and the downward pass, L2P (DO_L2P) after it.  With
+// DO_M2P, heavy leaves are left to k_leaf_far_heavy.
+template <int P, bool POT, bool DO_L2P, bool DO_M2P, class T>
+__global__ void __launch_bounds__(32, sizeof(T) == 4 ? 20 : 12) k_leaf_far(TreeView tv, const T* __restrict__ hrec,
+                                                                           const T* __restrict__ grec, double* __restrict__ far) {
+    using GR = Rec<T, rec_degree<P, 1, POT>(), POT>;
+    extern __shared__ __align__(16) unsigned char s_far_dyn[];
+    __shared__ Bodies<T> sb;
+    const int lane = threadIdx.x;
+    const int lf = blockIdx.x;
+    if (lf >= tv.nleaf || lf >= tv_nleaf(tv) || tv_over(tv)) return;
+    const int b = tv.leafbox[lf];
+    const int f0 = tv.pfirst[b], cnt = tv.pcount[b];
+    const int64_t w0 = DO_M2P ? tv.w_off[lf] : 0;
+    const int nw = DO_M2P ? (int)(tv.w_off[lf + 1] - w0) : 0;
+    if (DO_M2P && (int64_t)cnt * nw > heavy_line<T>(tv)) return;
+    const double cx = tv.center[4 * b], cy = tv.center[4 * b + 1], cz = tv.center[4 * b + 2];
+    const double side = 2.0 * tv.center[4 * b + 3], inv = 1.0 / side;
+    for (int jb = 0; jb < cnt; jb += 64) {
+        const int nbk = min(64, cnt - jb);
+        double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+        if (DO_L2P || nw > 0) {
+            __syncwarp();
+            for (int j = lane; j < nbk; j += 32) {
+                const int i = f0 + jb + j;
+                put_body(sb, j, tv.px[i] - cx, tv.py[i] - cy, tv.pz[i] - cz, inv);
+            }
+            __syncwarp();
+        }
+        if constexpr (DO_L2P)
+            l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, inv, reinterpret_cast<float4*>(s_far_dyn), lane, acc);
+        if constexpr (DO_M2P)
+            if (nw > 0)
+                m2p_rounds<P, POT, T>(tv, hrec, w0, nw, nbk, 0, 1, sb, cx, cy, cz, side,
+                                      *reinterpret_cast<WarpSmem<P, POT, T>*>(s_far_dyn), lane, acc);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int j = lane + 32 * q;
+            if (j < nbk) {
+                double2* o = reinterpret_cast<double2*>(far + 4 * (size_t)(f0 + jb + j));
+                o[0] = make_double2(acc[q][0], acc[q][1]);
+                o[1] = make_double2(acc[q][2], acc[q][3]);
+            }
+        }
+    }
+}
+// shared memory of k_leaf_far: the M2P stage, or the L2P record
+template <int P, bool POT, bool DO_M2P, class T>
+constexpr size_t leaf_far_smem() {
+    constexpr size_t a = sizeof(float4) * Rec<T, rec_degree<P, 1, POT>(), POT>::F4;
+    return DO_M2P ? (sizeof(WarpSmem<P, POT, T>) > a ? sizeof(WarpSmem<P, POT, T>) : a) : a;
+}
+
+// list of the heavy leaves (order irrelevant: every leaf's result is computed
+// independently); *count zero before the launch
+template <class T>
+__global__ void k_far_heavy_list(TreeView tv, int* __restrict__ list, int* count) {
+    const int lf = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lf >= tv.nleaf || lf >= tv_nleaf(tv) || tv_over(tv)) return;
+    if ((int64_t)tv.pcount[tv.leafbox[lf]] * (tv.w_off[lf + 1] - tv.w_off[lf]) > heavy_line<T>(tv)) list[atomicAdd(count, 1)] = lf;
+}
+
+// Heavy leaves: a CTA of FAR_HW warps per leaf, leaves taken from the list through a shared
+// counter (ctr[1], zero before the launch; ctr[0] = list length) so the CTAs balance
+// themselves.  Warp w runs the rounds w, w + FAR_HW, ...; warp 0 also the L2P; the warps'
+// per-body partial sums are added in warp order through shared memory (deterministic).
+template <int P, bool POT, bool DO_L2P, class T>
+__global__ void __launch_bounds__(32 * FAR_HW, sizeof(T) == 4 ? 3 : 2) k_leaf_far_heavy(TreeView tv, const T* __restrict__ hrec,
+                                                                                       const T* __restrict__ grec,
+                                                                                       double* __restrict__ far,
+                                                                                       const int* __restrict__ list, int* ctr) {
+    using GR = Rec<T, rec_degree<P, 1, POT>(), POT>;
+    extern __shared__ __align__(16) unsigned char s_far_dyn[];
+    __shared__ Bodies<T> sb;
+    __shared__ int s_lf;
+    double* s_part = reinterpret_cast<double*>(s_far_dyn);   // [FAR_HW][64][4], over the records once the rounds are done
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    WarpSmem<P, POT, T>& sm = reinterpret_cast<WarpSmem<P, POT, T>*>(s_far_dyn)[wid];
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int k = atomicAdd(&ctr[1], 1);
+            s_lf = (k < ctr[0]) ? list[k] : -1;
+        }
+        __syncthreads();
+        const int lf = s_lf;
+        if (lf < 0) return;
+        const int b = tv.leafbox[lf];
+        const int f0 = tv.pfirst[b], cnt = tv.pcount[b];
+        const int64_t w0 = tv.w_off[lf];
+        const int nw = (int)(tv.w_off[lf + 1] - w0);
+        const double cx = tv.center[4 * b], cy = tv.center[4 * b + 1], cz = tv.center[4 * b + 2];
+        const double side = 2.0 * tv.center[4 * b + 3], inv = 1.0 / side;
+        for (int jb = 0; jb < cnt; jb += 64) {
+            const int nbk = min(64, cnt - jb);
+            __syncthreads();
+            for (int j = threadIdx.x; j < nbk; j += blockDim.x) {
+                const int i = f0 + jb + j;
+                put_body(sb, j, tv.px[i] - cx, tv.py[i] - cy, tv.pz[i] - cz, inv);
+            }
+            __syncthreads();
+            double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+            if constexpr (DO_L2P)
+                if (wid == 0) l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, inv, sm.rec, lane, acc);
+            m2p_rounds<P, POT, T>(tv, hrec, w0, nw, nbk, wid, FAR_HW, sb, cx, cy, cz, side, sm, lane, acc);
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int j = lane + 32 * q;
+                if (j < nbk) {
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) s_part[(wid * 64 + j) * 4 + a] = acc[q][a];
+                }
+            }
+            __syncthreads();
+            for (int t = threadIdx.x; t < 4 * nbk; t += blockDim.x) {
+                double v = 0.0;
+#pragma unroll
+                for (int w = 0; w < FAR_HW; ++w) v += s_part[w * 256 + t];
+                far[4 * (size_t)(f0 + jb) + t] = v;
+            }
+        }
+    }
+}
+template <int P, bool POT, class T>
+constexpr size_t leaf_far_heavy_smem() {
+    constexpr size_t a = FAR_HW * sizeof(WarpSmem<P, POT, T>), b = sizeof(double) * FAR_HW * 64 * 4;
+    return a > b ? a : b;
+}
+
+}  // namespace far
+}  // namespace ogx

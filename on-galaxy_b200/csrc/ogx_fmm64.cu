@@ -24,6 +24,7 @@
 
 #include "ogx_harmonics.cuh"
 #include "ogx_expansion_kernels.cuh"
+#include "ogx_far.cuh"
 #include "ogx_mixed_kernels.cuh"
 #include "ogx_m2l64.cuh"
 
@@ -33,63 +34,58 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// ---- leaf far field: coefficient records, then L2P + M2P -------------------------
-template <int P, class T>
-int launch_far(Handle& h, const double* M, const double* L, double* far, bool pot) {
-    using Lo = EvalLayout<P>;
-    const cudaStream_t st = h.stream;
+// ---- leaf far field (ogx_far.cuh): coefficient records, then M2P over the W lists and L2P.
+// The mixed form's M2P part (L2P = false) needs only the multipoles, so it runs on the side
+// stream beside the M2L and the downward pass; the plain form takes both parts in one.
+template <int P, bool POT, bool L2P, class T>
+int launch_m2p(Handle& h, const double* M, const T* grec, double* out, cudaStream_t st) {
+    using R = far::Rec<T, P + 1, POT>;
     TreeView& tv = h.tv;
-    T *hrec, *grec;
-    OGX_TRY(arena_get(h.ws, S_EVAL_H, (size_t)tv.nb * Lo::HREC, &hrec));
-    OGX_TRY(arena_get(h.ws, S_EVAL_G, (size_t)tv.nleaf * Lo::GREC, &grec));
-    k_eval_coeffs<P, 0, T><<<(tv.nb + 3) / 4, 128, 0, st>>>(tv, tv.nb, M, hrec); ++h.launches;
-    k_eval_coeffs<P, 1, T><<<(tv.nleaf + 3) / 4, 128, 0, st>>>(tv, tv.nleaf, L, grec); ++h.launches;
-    if (pot) { k_leaf_far<P, true, T><<<(tv.nleaf + 3) / 4, 128, 0, st>>>(tv, hrec, grec, far); ++h.launches; }
-    else { k_leaf_far<P, false, T><<<(tv.nleaf + 3) / 4, 128, 0, st>>>(tv, hrec, grec, far); ++h.launches; }
-    return OGX_OK;
-}
-
-// mixed form: FP32 records with folded weights, flat (body, W box) M2P tasks.  The M2P
-// part needs only the multipoles, so it runs on the side stream beside the M2L and the
-// downward pass (into far_m); the L2P part runs after the downward pass (into far).
-template <int P>
-int launch_far32_m2p(Handle& h, const double* M, double* far_m, bool pot, cudaStream_t st) {
-    using R = mixed::FarRec32<P>;
-    TreeView& tv = h.tv;
-    float4* hrec;
-    OGX_TRY(arena_get(h.ws, S_EVAL_H, (size_t)tv.nb * 2 * R::NEH, &hrec));
-    mixed::k_far_rec32<P, 0><<<(tv.nb + 3) / 4, 128, 0, st>>>(tv, tv.nb, M, hrec); ++h.launches;
-    // heavy leaves: list, then one CTA of FAR_HW warps per leaf
+    T* hrec;
+    OGX_TRY(arena_get(h.ws, S_EVAL_H, (size_t)tv.nb * R::SIZE, &hrec));
+    far::k_far_rec<P, 0, POT, T><<<(tv.nb + 3) / 4, 128, 0, st>>>(tv, tv.nb, M, hrec); ++h.launches;
     int* heavy;
     OGX_TRY(arena_get(h.ws, S_FAR_HEAVY, (size_t)tv.nleaf + 2, &heavy));
     int* ctr = heavy + tv.nleaf;
     OGX_CUDA(cudaMemsetAsync(ctr, 0, 2 * sizeof(int), st));
-    mixed::k_far_heavy_list<<<(tv.nleaf + 255) / 256, 256, 0, st>>>(tv, heavy, ctr); ++h.launches;
-    const size_t hsmem = mixed::far_heavy_smem_bytes<P>();
-    const size_t smem = mixed::far_smem_bytes<P>();
-    const int lgrid = (tv.nleaf + mixed::FAR_WARPS - 1) / mixed::FAR_WARPS, lblock = 32 * mixed::FAR_WARPS;
-    auto heavyk = pot ? mixed::k_leaf_far32_heavy<P, true, false> : mixed::k_leaf_far32_heavy<P, false, false>;
-    auto lightk = pot ? mixed::k_leaf_far32<P, true, false, true> : mixed::k_leaf_far32<P, false, false, true>;
+    far::k_far_heavy_list<T><<<(tv.nleaf + 255) / 256, 256, 0, st>>>(tv, heavy, ctr); ++h.launches;
+    constexpr size_t hsmem = far::leaf_far_heavy_smem<P, POT, T>(), smem = far::leaf_far_smem<P, POT, true, T>();
+    auto heavyk = far::k_leaf_far_heavy<P, POT, L2P, T>;
+    auto lightk = far::k_leaf_far<P, POT, L2P, true, T>;
     OGX_CUDA(smem_optin((const void*)heavyk, (int)hsmem));
     OGX_CUDA(smem_optin((const void*)lightk, (int)smem));
-    heavyk<<<2 * h.num_sms, 32 * mixed::FAR_HW, hsmem, st>>>(tv, hrec, nullptr, far_m, heavy, ctr); ++h.launches;
-    lightk<<<lgrid, lblock, smem, st>>>(tv, hrec, nullptr, far_m); ++h.launches;
+    // two CTAs per SM: a third finishes the 1M merger no sooner (4.03 ms either way) and takes
+    // the shared memory that another system's M2L tiles need (three 262,144-body galaxies at
+    // p = 4 in turn: 1.51 -> 1.79 ms each)
+    heavyk<<<2 * h.num_sms, 32 * far::FAR_HW, hsmem, st>>>(tv, hrec, grec, out, heavy, ctr); ++h.launches;
+    lightk<<<tv.nleaf, 32, smem, st>>>(tv, hrec, grec, out); ++h.launches;
+    OGX_CUDA(cudaGetLastError());
     return OGX_OK;
 }
 
-template <int P>
-int launch_far32_l2p(Handle& h, const double* L, double* far, bool pot) {
-    using R = mixed::FarRec32<P>;
-    const cudaStream_t st = h.stream;
-    TreeView& tv = h.tv;
-    float4* grec;
-    OGX_TRY(arena_get(h.ws, S_EVAL_G, (size_t)tv.nleaf * 2 * R::NEG, &grec));
-    mixed::k_far_rec32<P, 1><<<(tv.nleaf + 3) / 4, 128, 0, st>>>(tv, tv.nleaf, L, grec); ++h.launches;
-    const size_t smem = mixed::far_smem_bytes<P>();
-    const int lgrid = (tv.nleaf + mixed::FAR_WARPS - 1) / mixed::FAR_WARPS, lblock = 32 * mixed::FAR_WARPS;
-    auto l2pk = pot ? mixed::k_leaf_far32<P, true, true, false> : mixed::k_leaf_far32<P, false, true, false>;
-    OGX_CUDA(smem_optin((const void*)l2pk, (int)smem));
-    l2pk<<<lgrid, lblock, smem, st>>>(tv, nullptr, grec, far); ++h.launches;
+template <int P, bool POT, class T>
+int launch_local_rec(Handle& h, const double* L, T** grec) {
+    using R = far::Rec<T, far::rec_degree<P, 1, POT>(), POT>;
+    OGX_TRY(arena_get(h.ws, S_EVAL_G, (size_t)h.tv.nleaf * R::SIZE, grec));
+    far::k_far_rec<P, 1, POT, T><<<(h.tv.nleaf + 3) / 4, 128, 0, h.stream>>>(h.tv, h.tv.nleaf, L, *grec); ++h.launches;
+    return OGX_OK;
+}
+
+// plain form: L2P + M2P in FP64, on h.stream
+template <int P, bool POT>
+int launch_far64(Handle& h, const double* M, const double* L, double* out) {
+    double* grec;
+    OGX_TRY((launch_local_rec<P, POT, double>(h, L, &grec)));
+    return launch_m2p<P, POT, true, double>(h, M, grec, out, h.stream);
+}
+
+// mixed form: the L2P, after the downward pass
+template <int P, bool POT>
+int launch_l2p32(Handle& h, const double* L, double* out) {
+    float* grec;
+    OGX_TRY((launch_local_rec<P, POT, float>(h, L, &grec)));
+    constexpr size_t smem = far::leaf_far_smem<P, POT, false, float>();
+    far::k_leaf_far<P, POT, true, false, float><<<h.tv.nleaf, 32, smem, h.stream>>>(h.tv, nullptr, grec, out); ++h.launches;
     return OGX_OK;
 }
 
@@ -553,7 +549,8 @@ int run_fp64(Handle& h, double* d_acc, double* d_pot) {
     OGX_CUDA(timing_record(h, h.ev[6], st));
     // leaves
     const bool pot = d_pot != nullptr;
-    OGX_TRY((launch_far<P, double>(h, M, L, far, pot)));
+    if (pot) OGX_TRY((launch_far64<P, true>(h, M, L, far)));
+    else OGX_TRY((launch_far64<P, false>(h, M, L, far)));
     const double G = h.prm.G, eps2 = h.prm.eps * h.prm.eps;
     int64_t* chunk_off;
     OGX_TRY(near_items(h, &chunk_off));
@@ -765,7 +762,8 @@ int run_mixed(Handle& h, double* d_acc, double* d_pot) {
         OGX_TRY(arena_get(h.ws, S_MIX_POS4, 2 * (size_t)tv.n, &rel));
         OGX_CUDA(cudaStreamWaitEvent(h.side, h.ev_fork, 0));
         // the far field's M2P part (multipoles only) first, then the near field
-        OGX_TRY(launch_far32_m2p<P>(h, M, far_m, d_pot != nullptr, h.side));
+        if (d_pot) OGX_TRY((launch_m2p<P, true, false, float>(h, M, nullptr, far_m, h.side)));
+        else OGX_TRY((launch_m2p<P, false, false, float>(h, M, nullptr, far_m, h.side)));
         mixed::k_near_prep<<<(tv.n + 255) / 256, 256, 0, h.side>>>(tv, rel, rel + tv.n); ++h.launches;
         // one block per work item: the leaves' chunks number at most nleaf + n / 32 (a
         // bounded grid left the far chain waiting)
@@ -799,7 +797,8 @@ int run_mixed(Handle& h, double* d_acc, double* d_pot) {
     OGX_TRY(launch_l2l<P>(h, L, Lown));
     OGX_CUDA(timing_record(h, h.ev[6], st));
     const bool pot = d_pot != nullptr;
-    OGX_TRY(launch_far32_l2p<P>(h, L, far, pot));
+    if (pot) OGX_TRY((launch_l2p32<P, true>(h, L, far)));
+    else OGX_TRY((launch_l2p32<P, false>(h, L, far)));
     // join the side stream (M2P, near field), then acc = G (far + near) in the caller's order
     OGX_CUDA(cudaStreamWaitEvent(st, h.ev_join, 0));
     const double G = h.prm.G;

@@ -35,6 +35,8 @@ struct HarmTables {
     // gradient-coefficient constants (derivative recurrences of FmmExpansions3D.hpp:111-129)
     double gz[kTab][kTab], gp[kTab][kTab], gm[kTab][kTab];  // local  -> degree n (from degree n+1)
     double hz[kTab][kTab], hp[kTab][kTab], hm[kTab][kTab];  // mpole  -> degree n (from degree n-1)
+    // R_n^m = s[n][m] (x+iy)^m T_nm: the product of the recurrence constants (ogx_far.cuh)
+    double s[kTab][kTab];
     // FP32 copies of the recurrence constants for the FP32 kernels (no conversion per use)
     float fa[kTab], fb[kTab], fA[kTab][kTab], fB[kTab][kTab];
 };
@@ -86,6 +88,16 @@ static inline void fill_harm_tables(HarmTables& t) {
                 }
             }
         }
+    double am = 1.0;
+    for (int m = 0; m < kTab; ++m) {
+        am *= t.a[m];
+        double v = am;
+        for (int n = m; n < kTab; ++n) {
+            if (n == m + 1) v *= t.b[m];
+            else if (n > m + 1) v *= t.A[n][m];
+            t.s[n][m] = v;
+        }
+    }
 }
 
 static inline int harm_tables_ready(int device) {
@@ -204,58 +216,6 @@ __device__ __forceinline__ void coef_get(const T* c, int n, int m, T& re, T& im)
     re = c[n * n + 2 * am - 1];
     im = c[n * n + 2 * am];
     if (m < 0) im = -im;
-}
-
-__device__ __forceinline__ void dof_decode(int d, int& n, int& m, int& part) {
-    n = (int)floorf(sqrtf((float)d) + 1e-4f);
-    const int r = d - n * n;
-    m = (r + 1) >> 1;
-    part = (r == 0) ? 0 : ((r - 1) & 1);
-}
-
-// Gradient coefficients of a local expansion (degree P -> P-1), in the real
-// layout, for the three axes.  From the derivative recurrences of
-// FmmExpansions3D.hpp:111-119 as used by localField (:215-235):
-//   Gz_n^m = cz_R(n+1,m) L_{n+1}^m
-//   Gx_n^m = (cp_R(n+1,m-1) L_{n+1}^{m-1} + cm_R(n+1,m+1) L_{n+1}^{m+1}) / 2
-//   Gy_n^m = -i (cp_R(n+1,m-1) L_{n+1}^{m-1} - cm_R(n+1,m+1) L_{n+1}^{m+1}) / 2
-// Every returned value is for one real dof index `d` of degree <= P-1.
-template <class Tin, class T>
-__device__ __forceinline__ void local_grad_dof(const Tin* L, int d, T g[3]) {
-    int n, m, part;
-    dof_decode(d, n, m, part);
-    const int N = n + 1;
-    Tin lr, li, pr, pi, mr, mi;
-    coef_get(L, N, m, lr, li);
-    coef_get(L, N, m - 1, mr, mi);
-    coef_get(L, N, m + 1, pr, pi);
-    const double czr = c_harm.gz[n][m], cpr = c_harm.gp[n][m], cmr = c_harm.gm[n][m];
-    const double xr = 0.5 * (cpr * mr + cmr * pr), xi = 0.5 * (cpr * mi + cmr * pi);
-    const double dr = cpr * mr - cmr * pr, di = cpr * mi - cmr * pi;  // -i/2 (a - b)
-    if (part == 0) { g[0] = (T)xr; g[1] = (T)(0.5 * di); g[2] = (T)(czr * lr); }
-    else { g[0] = (T)xi; g[1] = (T)(-0.5 * dr); g[2] = (T)(czr * li); }
-}
-
-// Gradient coefficients of a multipole expansion (degree P -> P+1), from
-// dz_S/dp_S/dm_S (FmmExpansions3D.hpp:121-129) as used by multipoleField (:180-200):
-//   Hz_n^m = dz_S(n-1,m) M_{n-1}^m
-//   Hx_n^m = (dp_S(n-1,m-1) M_{n-1}^{m-1} + dm_S(n-1,m+1) M_{n-1}^{m+1}) / 2
-//   Hy_n^m = -i (dp_S(n-1,m-1) M_{n-1}^{m-1} - dm_S(n-1,m+1) M_{n-1}^{m+1}) / 2
-template <class Tin, class T>
-__device__ __forceinline__ void mpole_grad_dof(const Tin* M, int d, T g[3]) {
-    int n, m, part;
-    dof_decode(d, n, m, part);
-    if (n == 0) { g[0] = g[1] = g[2] = 0; return; }
-    const int N = n - 1;
-    Tin lr, li, pr, pi, mr, mi;
-    coef_get(M, N, m, lr, li);
-    coef_get(M, N, m - 1, mr, mi);
-    coef_get(M, N, m + 1, pr, pi);
-    const double dzs = c_harm.hz[n][m], dps = c_harm.hp[n][m], dms = c_harm.hm[n][m];
-    const double xr = 0.5 * (dps * mr + dms * pr), xi = 0.5 * (dps * mi + dms * pi);
-    const double dr = dps * mr - dms * pr, di = dps * mi - dms * pi;
-    if (part == 0) { g[0] = (T)xr; g[1] = (T)(0.5 * di); g[2] = (T)(dzs * lr); }
-    else { g[0] = (T)xi; g[1] = (T)(-0.5 * dr); g[2] = (T)(dzs * li); }
 }
 
 }  // namespace ogx
