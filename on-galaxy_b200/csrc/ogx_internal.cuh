@@ -358,5 +358,6 @@ int radix_sort_u32(Handle& h, Slot kin, Slot vin, Slot kalt, Slot valt, int64_t 
 // by levels 1..16 only)
 int radix_sort_key72(Handle& h, int64_t n, int first_pass, uint64_t** khi, uint32_t** klo, uint32_t** idx);
 int scan_i32_to_i64(Handle& h, const int* in, int64_t* out, int64_t n);  // exclusive, out[n] = total
+int scan2_i32_to_i64(Handle& h, const int* in_a, int64_t* out_a, const int* in_b, int64_t* out_b, int64_t n);   // both at once
 
 }  // namespace ogx

@@ -517,8 +517,7 @@ int lists_build_uwx(Handle& h) {
     k_uw_warp<false><<<grid_for(nleaf, 4), 128, 0, st>>>(nleaf, tv.leafbox, tv.parent, tv.child, tv.leafid, col, tv.center,
                                                          tv.pcount, tv.root, lane_u, lane_w, ucnt, wcnt, nullptr, nullptr,
                                                          nullptr, nullptr, dc); ++h.launches;
-    OGX_TRY(scan_i32_to_i64(h, ucnt, uoff, nleaf));
-    OGX_TRY(scan_i32_to_i64(h, wcnt, woff, nleaf));
+    OGX_TRY(scan2_i32_to_i64(h, ucnt, uoff, wcnt, woff, nleaf));
     int64_t nu, nw;
     if (h.cap_mode) {
         nu = h.cap.u;

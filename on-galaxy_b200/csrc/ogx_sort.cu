@@ -5,19 +5,25 @@
 //   1. bodies by their 72-bit octant path (9 passes of 8 bits),
 //   2. bodies by leaf id, starting from the original order, so that inside a
 //      leaf the bodies keep their original index order (2-3 passes).
-// Each pass: per-tile digit histogram -> one exclusive scan over
-// (digit, tile) -> stable scatter.  The scatter ranks keys inside a warp with
-// __match_any_sync, keeps per-warp digit counters in shared memory and
-// orders warps by their contiguous sub-tiles, so the pass is stable.
+// Ranking is the same everywhere: a warp ranks 32 keys with __match_any_sync,
+// keeps per-warp digit counters in shared memory and warps are ordered by their
+// contiguous sub-tiles, so a pass is stable.
+//
+// Up to 131,072 items, all passes run in ONE launch of a thread-block cluster: every CTA
+// keeps its items in registers and shared memory, digit counts are exchanged and items
+// scattered through distributed shared memory, with two cluster barriers per pass.  These
+// sizes are bound by latency, not by memory: as four launches per pass (histogram, two
+// scans, scatter) a pass took 35-40 us whatever its size, and an evaluation runs 15 passes.
+// Above, each pass is three launches: per-tile digit histogram -> scan over the tiles of
+// every digit -> scatter (which scans the 256 digit totals itself).
+#include <cooperative_groups.h>
+
 #include "ogx_internal.cuh"
 
 namespace ogx {
 namespace {
 
-constexpr int RS_THREADS = 256;
-constexpr int RS_IPT = 16;
-constexpr int RS_TILE = RS_THREADS * RS_IPT;
-constexpr int RS_WARPS = RS_THREADS / 32;
+namespace cg = cooperative_groups;
 constexpr unsigned FULL = 0xffffffffu;
 
 struct Key32 {
@@ -26,6 +32,14 @@ struct Key32 {
     __device__ __forceinline__ T load(int64_t i) const { return k[i]; }
     __device__ __forceinline__ void store(int64_t i, T v) const { k[i] = v; }
     __device__ __forceinline__ static uint32_t digit(T v, int pass) { return (v >> (8 * pass)) & 0xFFu; }
+    // a tile's keys in shared memory (rs_cluster)
+    static constexpr int BYTES = 4;
+    using Smem = uint32_t*;
+    __device__ __forceinline__ static Smem smem(unsigned char* p, int) { return reinterpret_cast<uint32_t*>(p); }
+    __device__ __forceinline__ static void put(Smem s, const cg::cluster_group& cl, unsigned c, unsigned o, T v) {
+        cl.map_shared_rank(s, c)[o] = v;
+    }
+    __device__ __forceinline__ static T get(Smem s, int i) { return s[i]; }
 };
 
 struct K72 {
@@ -44,36 +58,181 @@ struct Key72 {
         if (pass == 1) return ((v.lo >> 8) & 1u) | (uint32_t)((v.hi & 0x7Full) << 1);
         return (uint32_t)((v.hi >> (8 * pass - 9)) & 0xFFull);
     }
+    static constexpr int BYTES = 12;
+    struct Smem {
+        uint64_t* hi;
+        uint32_t* lo;
+    };
+    __device__ __forceinline__ static Smem smem(unsigned char* p, int tile) {
+        return Smem{reinterpret_cast<uint64_t*>(p), reinterpret_cast<uint32_t*>(p + (size_t)tile * 8)};
+    }
+    __device__ __forceinline__ static void put(Smem s, const cg::cluster_group& cl, unsigned c, unsigned o, T v) {
+        cl.map_shared_rank(s.hi, c)[o] = v.hi;
+        cl.map_shared_rank(s.lo, c)[o] = v.lo;
+    }
+    __device__ __forceinline__ static T get(Smem s, int i) { return K72{s.hi[i], s.lo[i]}; }
 };
 
-template <class KO>
+// ---- one launch, all passes: a cluster of CTAs ------------------------------------------
+constexpr int RC_THREADS = 1024;
+constexpr int RC_WARPS = RC_THREADS / 32;
+constexpr int RC_MAX_CTAS = 16;
+constexpr int RC_MAX = RC_MAX_CTAS * RC_THREADS * 8;   // 131,072 items
+
+template <class KO, int IPT>
+constexpr int rc_smem() { return RC_THREADS * IPT * (int)(KO::BYTES + 4) + RC_WARPS * 256 * 4; }
+
+template <class KO, int IPT>
+__global__ void __launch_bounds__(RC_THREADS) rs_cluster(KO kin, KO kout, const uint32_t* vin, uint32_t* vout, int n,
+                                                         int first_pass, int npasses) {
+    constexpr int TILE = RC_THREADS * IPT;
+    extern __shared__ __align__(16) unsigned char rc_raw[];
+    __shared__ uint32_t s_cnt[256], s_base[256], s_quarter[4][256], s_warp[8];
+    typename KO::Smem sk = KO::smem(rc_raw, TILE);
+    uint32_t* sv = reinterpret_cast<uint32_t*>(rc_raw + (size_t)TILE * KO::BYTES);
+    uint32_t(*wcnt)[256] = reinterpret_cast<uint32_t(*)[256]>(sv + TILE);
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), me = (int)cl.block_rank();
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int local0 = w * 32 * IPT + lane;      // this thread's items: local0 + 32 r
+    const int left = min(max(n - me * TILE, 0), TILE);   // items of this CTA
+    typename KO::T key[IPT];
+    uint32_t val[IPT];
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        const int i = local0 + 32 * r;
+        if (i < left) {
+            key[r] = kin.load((int64_t)me * TILE + i);
+            val[r] = vin[(int64_t)me * TILE + i];
+        }
+    }
+    for (int pass = first_pass; pass < npasses; ++pass) {
+        for (int i = t; i < RC_WARPS * 256; i += RC_THREADS) (&wcnt[0][0])[i] = 0;
+        __syncthreads();
+        uint32_t loc[IPT];
+#pragma unroll
+        for (int r = 0; r < IPT; ++r) {
+            const bool valid = local0 + 32 * r < left;
+            const uint32_t d = valid ? KO::digit(key[r], pass) : 0xFFFFFFFFu;
+            const unsigned peers = __match_any_sync(FULL, d);
+            uint32_t c = 0;
+            if (valid) c = wcnt[w][d];
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1) wcnt[w][d] = c + __popc(peers);
+            __syncwarp();
+            loc[r] = c + __popc(peers & lt);
+        }
+        __syncthreads();
+        {   // counters -> offsets inside the CTA's digit, a quarter of the warps per thread
+            const int d = t & 255, q = t >> 8;
+            uint32_t run = 0;
+#pragma unroll
+            for (int k = 0; k < RC_WARPS / 4; ++k) {
+                const uint32_t c = wcnt[q * (RC_WARPS / 4) + k][d];
+                wcnt[q * (RC_WARPS / 4) + k][d] = run;
+                run += c;
+            }
+            s_quarter[q][d] = run;
+        }
+        __syncthreads();
+        if (t < 256) {
+            uint32_t run = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t c = s_quarter[q][t];
+                s_quarter[q][t] = run;
+                run += c;
+            }
+            s_cnt[t] = run;
+        }
+        cl.sync();
+        uint32_t tot = 0, before = 0, x = 0;
+        if (t < 256) {
+            for (int c = 0; c < C; ++c) {
+                const uint32_t v = cl.map_shared_rank(s_cnt, c)[t];
+                if (c < me) before += v;
+                tot += v;
+            }
+            x = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) s_warp[w] = x;
+        }
+        __syncthreads();
+        if (t < 256) {
+            uint32_t pre = 0;
+            for (int k = 0; k < w; ++k) pre += s_warp[k];
+            s_base[t] = pre + x - tot + before;
+        }
+        __syncthreads();
+        const bool last = pass + 1 == npasses;
+#pragma unroll
+        for (int r = 0; r < IPT; ++r) {
+            if (local0 + 32 * r < left) {
+                const uint32_t d = KO::digit(key[r], pass);
+                const uint32_t pos = s_base[d] + s_quarter[w / (RC_WARPS / 4)][d] + wcnt[w][d] + loc[r];
+                if (last) {
+                    kout.store(pos, key[r]);
+                    vout[pos] = val[r];
+                } else {
+                    const unsigned c = pos / TILE, o = pos % TILE;
+                    KO::put(sk, cl, c, o, key[r]);
+                    cl.map_shared_rank(sv, c)[o] = val[r];
+                }
+            }
+        }
+        cl.sync();   // every item is in place (and, after the last pass, no CTA exits while its counts are read)
+        if (!last) {
+#pragma unroll
+            for (int r = 0; r < IPT; ++r) {
+                const int i = local0 + 32 * r;
+                if (i < left) {
+                    key[r] = KO::get(sk, i);
+                    val[r] = sv[i];
+                }
+            }
+        }
+    }
+}
+
+// ---- three launches per pass ----------------------------------------------------------
+constexpr int RS_THREADS = 512;
+constexpr int RS_WARPS = RS_THREADS / 32;
+
+template <class KO, int IPT>
 __global__ void __launch_bounds__(RS_THREADS) rs_hist(KO keys, int64_t n, int pass, uint32_t* hist, int nblocks) {
     __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
+    if (threadIdx.x < 256) h[threadIdx.x] = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int64_t start = (int64_t)blockIdx.x * RS_TILE;
-    for (int k = threadIdx.x; k < RS_TILE; k += RS_THREADS) {
-        const int64_t i = start + k;
-        const bool valid = i < n;
-        const uint32_t d = valid ? KO::digit(keys.load(i), pass) : 0xFFFFFFFFu;
-        const unsigned peers = __match_any_sync(FULL, d);
-        if (valid && lane == __ffs(peers) - 1) atomicAdd(&h[d], (uint32_t)__popc(peers));
+    const int64_t start = (int64_t)blockIdx.x * (RS_THREADS * IPT) + threadIdx.x;
+    uint32_t d[IPT];
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        const int64_t i = start + r * RS_THREADS;
+        d[r] = i < n ? KO::digit(keys.load(i), pass) : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        const unsigned peers = __match_any_sync(FULL, d[r]);
+        if (d[r] < 256 && lane == __ffs(peers) - 1) atomicAdd(&h[d[r]], (uint32_t)__popc(peers));
     }
     __syncthreads();
-    hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+    if (threadIdx.x < 256) hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
 // Digit-major histogram hist[d * nblocks + b] -> exclusive offsets within each digit
 // (one CTA per digit, coalesced over the tiles), digit totals into tot[d].
-__global__ void __launch_bounds__(1024) rs_scan_digit(uint32_t* hist, int nblocks, uint32_t* tot) {
-    __shared__ uint32_t warp_sum[32];
-    __shared__ uint32_t carry;
+__global__ void __launch_bounds__(256) rs_scan_digit(uint32_t* hist, int nblocks, uint32_t* tot) {
+    __shared__ uint32_t warp_sum[8];
     uint32_t* a = hist + (size_t)blockIdx.x * nblocks;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if (t == 0) carry = 0;
-    __syncthreads();
-    for (int b0 = 0; b0 < nblocks; b0 += 1024) {
+    uint32_t carry = 0;
+    for (int b0 = 0; b0 < nblocks; b0 += 256) {
         const int i = b0 + t;
         const uint32_t v = (i < nblocks) ? a[i] : 0u;
         uint32_t x = v;
@@ -84,90 +243,84 @@ __global__ void __launch_bounds__(1024) rs_scan_digit(uint32_t* hist, int nblock
         }
         if (lane == 31) warp_sum[w] = x;
         __syncthreads();
-        if (w == 0) {
-            uint32_t s = warp_sum[lane];
+        uint32_t pre = 0, all = 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, s, o);
-                if (lane >= o) s += y;
-            }
-            warp_sum[lane] = s;
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t s = warp_sum[k];
+            if (k < w) pre += s;
+            all += s;
         }
-        __syncthreads();
-        const uint32_t ex = carry + (w > 0 ? warp_sum[w - 1] : 0u) + x - v;
-        if (i < nblocks) a[i] = ex;
-        __syncthreads();
-        if (t == 0) carry += warp_sum[31];
+        if (i < nblocks) a[i] = carry + pre + x - v;
+        carry += all;
         __syncthreads();
     }
     if (t == 0) tot[blockIdx.x] = carry;
 }
 
-// exclusive scan of the 256 digit totals (in place)
-__global__ void __launch_bounds__(256) rs_scan_totals(uint32_t* tot) {
-    __shared__ uint32_t s[256];
-    const int t = threadIdx.x;
-    const uint32_t v = tot[t];
-    s[t] = v;
-    __syncthreads();
-    for (int o = 1; o < 256; o <<= 1) {
-        const uint32_t y = (t >= o) ? s[t - o] : 0u;
-        __syncthreads();
-        s[t] += y;
-        __syncthreads();
-    }
-    tot[t] = s[t] - v;
-}
-
-template <class KO>
+template <class KO, int IPT>
 __global__ void __launch_bounds__(RS_THREADS) rs_scatter(KO kin, KO kout, const uint32_t* vin, uint32_t* vout, int64_t n,
-                                                         int pass, const uint32_t* scanned, int nblocks, const uint32_t* digit_base) {
+                                                         int pass, const uint32_t* scanned, int nblocks, const uint32_t* tot) {
     __shared__ uint32_t wcnt[RS_WARPS][256];
-    __shared__ uint32_t gbase[256];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&wcnt[0][0])[i] = 0;
-    __syncthreads();
+    __shared__ uint32_t gbase[256], s_warp[8];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const int64_t base = (int64_t)blockIdx.x * RS_TILE + (int64_t)w * 32 * RS_IPT;
-    typename KO::T key[RS_IPT];
-    uint32_t val[RS_IPT], loc[RS_IPT], dig[RS_IPT];
+    const int64_t base = (int64_t)blockIdx.x * (RS_THREADS * IPT) + (int64_t)w * 32 * IPT + lane;
+    // every load of the tile is in flight before the first rank
+    typename KO::T key[IPT];
+    uint32_t val[IPT], loc[IPT];
 #pragma unroll
-    for (int r = 0; r < RS_IPT; ++r) {
-        const int64_t i = base + r * 32 + lane;
-        const bool valid = i < n;
-        uint32_t d = 0xFFFFFFFFu;
-        if (valid) {
+    for (int r = 0; r < IPT; ++r) {
+        const int64_t i = base + r * 32;
+        if (i < n) {
             key[r] = kin.load(i);
             val[r] = vin[i];
-            d = KO::digit(key[r], pass);
         }
-        const unsigned peers = __match_any_sync(FULL, d);
-        uint32_t l = 0;
-        if (valid) l = wcnt[w][d] + __popc(peers & lt);
-        __syncwarp();
-        if (valid && lane == __ffs(peers) - 1) wcnt[w][d] += __popc(peers);
-        __syncwarp();
-        loc[r] = l;
-        dig[r] = d;
+    }
+    uint32_t tv = 0, x = 0, sc = 0;
+    if (t < 256) {
+        x = tv = tot[t];
+        sc = scanned[(int64_t)t * nblocks + blockIdx.x];
+    }
+    for (int i = t; i < RS_WARPS * 256; i += RS_THREADS) (&wcnt[0][0])[i] = 0;
+    if (t < 256) {   // exclusive scan of the 256 digit totals
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_warp[w] = x;
     }
     __syncthreads();
-    {
-        const int d = threadIdx.x;  // RS_THREADS == 256 bins
+#pragma unroll
+    for (int r = 0; r < IPT; ++r) {
+        const bool valid = base + r * 32 < n;
+        const uint32_t d = valid ? KO::digit(key[r], pass) : 0xFFFFFFFFu;
+        const unsigned peers = __match_any_sync(FULL, d);
+        uint32_t c = 0;
+        if (valid) c = wcnt[w][d];
+        __syncwarp();
+        if (valid && lane == __ffs(peers) - 1) wcnt[w][d] = c + __popc(peers);
+        __syncwarp();
+        loc[r] = c + __popc(peers & lt);
+    }
+    __syncthreads();
+    if (t < 256) {
         uint32_t run = 0;
 #pragma unroll
-        for (int ww = 0; ww < RS_WARPS; ++ww) {
-            const uint32_t c = wcnt[ww][d];
-            wcnt[ww][d] = run;
+        for (int k = 0; k < RS_WARPS; ++k) {
+            const uint32_t c = wcnt[k][t];
+            wcnt[k][t] = run;
             run += c;
         }
-        gbase[d] = digit_base[d] + scanned[(int64_t)d * nblocks + blockIdx.x];
+        uint32_t pre = 0;
+        for (int k = 0; k < w; ++k) pre += s_warp[k];
+        gbase[t] = pre + x - tv + sc;
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < RS_IPT; ++r) {
-        const int64_t i = base + r * 32 + lane;
-        if (i < n) {
-            const uint32_t d = dig[r];
+    for (int r = 0; r < IPT; ++r) {
+        if (base + r * 32 < n) {
+            const uint32_t d = KO::digit(key[r], pass);
             const int64_t pos = (int64_t)gbase[d] + wcnt[w][d] + loc[r];
             kout.store(pos, key[r]);
             vout[pos] = val[r];
@@ -176,9 +329,19 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(KO kin, KO kout, const 
 }
 
 // ---- generic exclusive scan int32 -> int64 (out has n+1 entries) --------------
+// Two arrays of one length at a time (grid y); up to SC_ONE entries in one launch (one
+// CTA walks them, its loads a chunk ahead), else per-tile sums and a second launch in
+// which every tile adds the sums before it.
 constexpr int SC_THREADS = 1024;
 constexpr int SC_IPT = 4;
 constexpr int SC_TILE = SC_THREADS * SC_IPT;
+constexpr int64_t SC_ONE = 8 * SC_TILE;
+
+struct ScanPair {
+    const int* in[2];
+    int64_t* out[2];
+    int64_t* part[2];
+};
 
 __device__ __forceinline__ int64_t block_excl_scan_i64(int64_t v, int64_t* sh, int64_t* total) {
     // sh: 32 int64 scratch
@@ -208,68 +371,142 @@ __device__ __forceinline__ int64_t block_excl_scan_i64(int64_t v, int64_t* sh, i
     return wpre + x - v;
 }
 
-__global__ void __launch_bounds__(SC_THREADS) sc_partials(const int* in, int64_t n, int64_t* part) {
-    __shared__ int64_t sh[32];
-    const int64_t b = (int64_t)blockIdx.x * SC_TILE + (int64_t)threadIdx.x * SC_IPT;
-    int64_t s = 0;
+__device__ __forceinline__ void sc_load(const int* in, int64_t b, int64_t n, int (&v)[SC_IPT]) {
 #pragma unroll
-    for (int k = 0; k < SC_IPT; ++k)
-        if (b + k < n) s += in[b + k];
-    int64_t tot;
+    for (int k = 0; k < SC_IPT; ++k) v[k] = b + k < n ? in[b + k] : 0;
+}
+
+__global__ void __launch_bounds__(SC_THREADS) sc_one(ScanPair sp, int64_t n) {
+    __shared__ int64_t sh[32];
+    const int* in = sp.in[blockIdx.y];
+    int64_t* out = sp.out[blockIdx.y];
+    int64_t carry = 0;
+    int v[SC_IPT];
+    sc_load(in, (int64_t)threadIdx.x * SC_IPT, n, v);
+    for (int64_t t0 = 0; t0 < n; t0 += SC_TILE) {
+        const int64_t b = t0 + (int64_t)threadIdx.x * SC_IPT;
+        int nx[SC_IPT];
+        sc_load(in, b + SC_TILE, n, nx);
+        int64_t s = 0, tot;
+#pragma unroll
+        for (int k = 0; k < SC_IPT; ++k) s += v[k];
+        int64_t run = carry + block_excl_scan_i64(s, sh, &tot);
+#pragma unroll
+        for (int k = 0; k < SC_IPT; ++k) {
+            if (b + k < n) out[b + k] = run;
+            run += v[k];
+            v[k] = nx[k];
+        }
+        carry += tot;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
+__global__ void __launch_bounds__(SC_THREADS) sc_partials(ScanPair sp, int64_t n) {
+    __shared__ int64_t sh[32];
+    int v[SC_IPT];
+    sc_load(sp.in[blockIdx.y], (int64_t)blockIdx.x * SC_TILE + (int64_t)threadIdx.x * SC_IPT, n, v);
+    int64_t s = 0, tot;
+#pragma unroll
+    for (int k = 0; k < SC_IPT; ++k) s += v[k];
     block_excl_scan_i64(s, sh, &tot);
-    if (threadIdx.x == 0) part[blockIdx.x] = tot;
+    if (threadIdx.x == 0) sp.part[blockIdx.y][blockIdx.x] = tot;
 }
 
-__global__ void __launch_bounds__(SC_THREADS) sc_scan_partials(int64_t* part, int64_t m) {
+__global__ void __launch_bounds__(SC_THREADS) sc_finish(ScanPair sp, int64_t n) {
     __shared__ int64_t sh[32];
-    __shared__ int64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int64_t b = 0; b < m; b += SC_THREADS) {
-        const int64_t i = b + threadIdx.x;
-        const int64_t v = (i < m) ? part[i] : 0;
-        int64_t tot;
-        const int64_t ex = block_excl_scan_i64(v, sh, &tot);
-        if (i < m) part[i] = carry + ex;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[m] = carry;
-}
-
-__global__ void __launch_bounds__(SC_THREADS) sc_finish(const int* in, int64_t n, const int64_t* part, int64_t* out, int nparts) {
-    __shared__ int64_t sh[32];
+    const int64_t* part = sp.part[blockIdx.y];
+    int64_t* out = sp.out[blockIdx.y];
     const int64_t b = (int64_t)blockIdx.x * SC_TILE + (int64_t)threadIdx.x * SC_IPT;
-    int64_t v[SC_IPT];
-    int64_t s = 0;
+    int v[SC_IPT];
+    sc_load(sp.in[blockIdx.y], b, n, v);
+    int64_t pre = 0, base;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += SC_THREADS) pre += part[k];
+    block_excl_scan_i64(pre, sh, &base);   // the sum of the tiles before this one
+    int64_t s = 0, tot;
 #pragma unroll
-    for (int k = 0; k < SC_IPT; ++k) {
-        v[k] = (b + k < n) ? in[b + k] : 0;
-        s += v[k];
-    }
-    int64_t run = part[blockIdx.x] + block_excl_scan_i64(s, sh, nullptr);
+    for (int k = 0; k < SC_IPT; ++k) s += v[k];
+    int64_t run = base + block_excl_scan_i64(s, sh, &tot);
 #pragma unroll
     for (int k = 0; k < SC_IPT; ++k) {
         if (b + k < n) out[b + k] = run;
         run += v[k];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = part[nparts];
+    if (blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) out[n] = base + tot;
 }
 
 }  // namespace
 
-int scan_i32_to_i64(Handle& h, const int* in, int64_t* out, int64_t n) {
-    const int nparts = (int)((n + SC_TILE - 1) / SC_TILE);
-    int64_t* part;
-    OGX_TRY(arena_get(h.ws, S_SCAN_TMP, (size_t)nparts + 1, &part));
+static int scan_arrays(Handle& h, ScanPair sp, int count, int64_t n) {
     if (n == 0) {
-        OGX_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), h.stream));
+        for (int a = 0; a < count; ++a) OGX_CUDA(cudaMemsetAsync(sp.out[a], 0, sizeof(int64_t), h.stream));
         return OGX_OK;
     }
-    sc_partials<<<nparts, SC_THREADS, 0, h.stream>>>(in, n, part); ++h.launches;
-    sc_scan_partials<<<1, SC_THREADS, 0, h.stream>>>(part, nparts); ++h.launches;
-    sc_finish<<<nparts, SC_THREADS, 0, h.stream>>>(in, n, part, out, nparts); ++h.launches;
+    if (n <= SC_ONE) {
+        sc_one<<<dim3(1, count), SC_THREADS, 0, h.stream>>>(sp, n); ++h.launches;
+    } else {
+        const int nparts = (int)((n + SC_TILE - 1) / SC_TILE);
+        OGX_TRY(arena_get(h.ws, S_SCAN_TMP, 2 * (size_t)nparts, &sp.part[0]));
+        sp.part[1] = sp.part[0] + nparts;
+        sc_partials<<<dim3(nparts, count), SC_THREADS, 0, h.stream>>>(sp, n); ++h.launches;
+        sc_finish<<<dim3(nparts, count), SC_THREADS, 0, h.stream>>>(sp, n); ++h.launches;
+    }
+    OGX_CUDA(cudaGetLastError());
+    return OGX_OK;
+}
+
+int scan_i32_to_i64(Handle& h, const int* in, int64_t* out, int64_t n) {
+    ScanPair sp{};
+    sp.in[0] = in;
+    sp.out[0] = out;
+    return scan_arrays(h, sp, 1, n);
+}
+
+int scan2_i32_to_i64(Handle& h, const int* in_a, int64_t* out_a, const int* in_b, int64_t* out_b, int64_t n) {
+    ScanPair sp{};
+    sp.in[0] = in_a; sp.in[1] = in_b;
+    sp.out[0] = out_a; sp.out[1] = out_b;
+    return scan_arrays(h, sp, 2, n);
+}
+
+// The cluster sort: IPT items per thread and the fewest CTAs (a power of two) that hold n.
+// CTAs of 4,096 items while a cluster of 8 holds them (fewer rounds per pass), else of 8,192.
+template <class KO, int IPT>
+static int cluster_sort(Handle& h, KO a, KO b, const uint32_t* va, uint32_t* vb, int64_t n, int npasses, int first_pass) {
+    auto kern = rs_cluster<KO, IPT>;
+    constexpr int smem = rc_smem<KO, IPT>();
+    OGX_CUDA(smem_optin((const void*)kern, smem));
+    int ctas = 1;
+    while ((int64_t)ctas * RC_THREADS * IPT < n) ctas *= 2;
+    if (ctas > 8) OGX_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(RC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    OGX_CUDA(cudaLaunchKernelEx(&cfg, kern, a, b, va, vb, (int)n, first_pass, npasses)); ++h.launches;
+    return OGX_OK;
+}
+
+template <class KO, int IPT>
+static int tile_sort(Handle& h, KO src, KO dst, uint32_t* vs, uint32_t* vd, int64_t n, int npasses, int first_pass) {
+    const int nblocks = (int)((n + RS_THREADS * IPT - 1) / (RS_THREADS * IPT));
+    uint32_t* hist;
+    OGX_TRY(arena_get(h.ws, S_RS_HIST, (size_t)256 * nblocks + 256, &hist));
+    uint32_t* tot = hist + (size_t)256 * nblocks;
+    for (int pass = first_pass; pass < npasses; ++pass) {
+        rs_hist<KO, IPT><<<nblocks, RS_THREADS, 0, h.stream>>>(src, n, pass, hist, nblocks); ++h.launches;
+        rs_scan_digit<<<256, 256, 0, h.stream>>>(hist, nblocks, tot); ++h.launches;
+        rs_scatter<KO, IPT><<<nblocks, RS_THREADS, 0, h.stream>>>(src, dst, vs, vd, n, pass, hist, nblocks, tot); ++h.launches;
+        std::swap(src, dst);
+        std::swap(vs, vd);
+    }
     OGX_CUDA(cudaGetLastError());
     return OGX_OK;
 }
@@ -277,23 +514,15 @@ int scan_i32_to_i64(Handle& h, const int* in, int64_t* out, int64_t n) {
 template <class KO>
 static int radix_passes(Handle& h, KO a, KO b, uint32_t* va, uint32_t* vb, int64_t n, int npasses, int* which,
                         int first_pass = 0) {
-    const int nblocks = (int)((n + RS_TILE - 1) / RS_TILE);
-    uint32_t* hist;
-    OGX_TRY(arena_get(h.ws, S_RS_HIST, (size_t)256 * nblocks + 256, &hist));
-    uint32_t* tot = hist + (size_t)256 * nblocks;
-    KO src = a, dst = b;
-    uint32_t *vs = va, *vd = vb;
-    for (int pass = first_pass; pass < npasses; ++pass) {
-        rs_hist<KO><<<nblocks, RS_THREADS, 0, h.stream>>>(src, n, pass, hist, nblocks); ++h.launches;
-        rs_scan_digit<<<256, 1024, 0, h.stream>>>(hist, nblocks, tot); ++h.launches;
-        rs_scan_totals<<<1, 256, 0, h.stream>>>(tot); ++h.launches;
-        rs_scatter<KO><<<nblocks, RS_THREADS, 0, h.stream>>>(src, dst, vs, vd, n, pass, hist, nblocks, tot); ++h.launches;
-        std::swap(src, dst);
-        std::swap(vs, vd);
+    if (n <= RC_MAX) {
+        *which = 1;
+        if (n <= 8 * RC_THREADS * 4) return cluster_sort<KO, 4>(h, a, b, va, vb, n, npasses, first_pass);
+        return cluster_sort<KO, 8>(h, a, b, va, vb, n, npasses, first_pass);
     }
-    OGX_CUDA(cudaGetLastError());
     *which = (npasses - first_pass) & 1;  // 0: result in a, 1: result in b
-    return OGX_OK;
+    // tiles of 2,048 while 4,096 would leave SMs without one
+    if (n <= (int64_t)RS_THREADS * 8 * h.num_sms) return tile_sort<KO, 4>(h, a, b, va, vb, n, npasses, first_pass);
+    return tile_sort<KO, 8>(h, a, b, va, vb, n, npasses, first_pass);
 }
 
 int radix_sort_u32(Handle& h, Slot kin, Slot vin, Slot kalt, Slot valt, int64_t n, int bits, uint32_t** kout,

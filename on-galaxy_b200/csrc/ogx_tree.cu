@@ -435,8 +435,7 @@ int tree_build(Handle& h, const double* d_pos, const double* d_mass, int64_t n) 
         if (first_pass > 0 && n > thr) { k_deep_check<<<grid_for(n, 256), 256, 0, st>>>(khi, n, thr, dc); ++h.launches; }
         k_topo_pairs<<<grid_for(n, 256), 256, 0, st>>>(khi, klo, n, thr, dfirst, cplthr); ++h.launches;
         k_topo_levels<<<grid_for(n, WM_BLOCK), WM_BLOCK, wm_smem, st>>>(cplthr, dfirst, n, thr, root, leaflev, cnt, leafflag, dc); ++h.launches;
-        OGX_TRY(scan_i32_to_i64(h, cnt, recoff, n));
-        OGX_TRY(scan_i32_to_i64(h, leafflag, leafscan, n));
+        OGX_TRY(scan2_i32_to_i64(h, cnt, recoff, leafflag, leafscan, n));
         k_counts_finalize<<<1, 32, 0, st>>>(dc, recoff, leafscan, n, level_off_dev); ++h.launches;
         if (h.cap_mode) {
             nb = h.cap.nb;
