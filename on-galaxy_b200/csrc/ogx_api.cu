@@ -40,7 +40,10 @@ int Arena::get(Slot s, size_t bytes, void** out) {
             ptr[s] = nullptr;
             cap[s] = 0;
         }
-        size_t nb = bytes + bytes / 4;
+        // operator tables keep their size; everything else may grow with the next system
+        const bool table = s == S_OPS_M2L || s == S_OPS_M2M || s == S_OPS_L2L || s == S_MIX_TOPS || s == S_MIX_ROW0 ||
+                           s == S_ROT_PACK;
+        size_t nb = table ? bytes : bytes + bytes / 4;
         nb = (nb + 255) & ~(size_t)255;
         const cudaError_t e = cudaMalloc(&ptr[s], nb);
         if (e != cudaSuccess) {
@@ -93,8 +96,8 @@ static std::shared_ptr<HostOps> host_ops(int p, bool m2l) {
     if (m2l) {
         put(ops->m2l, 343, 2, m2l64_pad_rows(p), m2l64_pad_cols(p));
     } else {
-        put(ops->m2m, 8, 0, K, K);
-        put(ops->l2l, 8, 1, K, K);
+        put(ops->m2m, 8, 0, m2l64_pad_rows(p), m2l64_pad_cols(p));
+        put(ops->l2l, 8, 1, m2l64_pad_rows(p), m2l64_pad_cols(p));
     }
     g_ops[{p, m2l}] = ops;
     return ops;
@@ -220,7 +223,7 @@ static int eval_device_on(Handle& h, int64_t n, const double* d_pos, const doubl
     const cudaStream_t st = h.stream;
     OGX_CUDA(timing_record(h, h.ev[0], st));
     if (h.prm.solver == OGX_SOLVER_DIRECT) {
-        OGX_TRY(direct_eval(h, d_pos, d_mass, n, d_acc, d_pot, false));
+        OGX_TRY(direct_eval(h, d_pos, d_mass, n, d_acc, d_pot));
         OGX_CUDA(timing_record(h, h.ev[8], st));
         h.stats.launches = h.launches - l0;
         return OGX_OK;

@@ -21,6 +21,7 @@
 #pragma once
 
 #include "ogx_harmonics.cuh"
+#include "ogx_packed.cuh"
 #include "ogx_sm100.cuh"
 
 namespace ogx {
@@ -110,29 +111,6 @@ __global__ void __launch_bounds__(128) k_far_rec(TreeView tv, int count, const d
 
 __host__ __device__ constexpr double rec_b(int n, int m) {
     return (double)((n - 1) * (n - 1) - m * m) / (double)((2 * n - 1) * (2 * n - 3));
-}
-
-// ---- packed FP32 pairs
-struct f2 { unsigned long long v; };
-__device__ __forceinline__ f2 pack2(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float sum2(f2 a) {
-    float x, y;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
-    return x + y;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return r;
 }
 
 // out = {sum_axis x, y, z(, phi)} of one body at scaled offset (x, y, z) for a record in

@@ -20,11 +20,13 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "ogx_harmonics.cuh"
-#include "ogx_expansion_kernels.cuh"
+#include "ogx_p2x.cuh"
 #include "ogx_far.cuh"
+#include "ogx_near.cuh"
 #include "ogx_mixed_kernels.cuh"
 #include "ogx_m2l64.cuh"
 
@@ -89,271 +91,7 @@ int launch_l2p32(Handle& h, const double* L, double* out) {
     return OGX_OK;
 }
 
-// ---- M2M (MODE 0) / L2L (MODE 1): one launch per pass ---------------------------------
-// CTA = tr_pb<P>() parents x 8 warps, warp s = child octant s.  Warp s applies the
-// operator MM_s / LL_s (transposed, k-major, L2-resident) to its TR_PB parents,
-// lanes over output dofs.
-//   M2M: M'_P = sum_s MM_s M'_{child s}                (src3d/AdaptiveFMM3D.hpp:62-71)
-//        the eight partial products are summed in octant order through shared memory
-//   L2L: L'_{child s} = L'own_{child s} + LL_s L'_P     (src3d/AdaptiveFMM3D.hpp:75-77)
-// The reference walks the levels one after another (its GPU form launches once per
-// level, src3d/gpu/AdaptiveFMM3DGPU.cu:274-289).  Here one launch covers every level.
-// The CTAs take groups of TR_PB parents of one level by ticket (an atomic counter) in
-// level order: root level first for L2L, deepest level first for M2M.  A group waits
-// until its inputs are final: for L2L each parent's local, written by the group that
-// holds the parent's parent; for M2M each non-leaf child's multipole.  Those groups hold
-// earlier tickets, taken by CTAs that are already running, so every wait ends; each is
-// bounded all the same (one that runs out sets *err).  A group publishes its boxes with
-// a fence and a release store of ready[box]; data written in this launch is read
-// through L2 (ld.global.cg).  The arithmetic per box is the same in any order.
-// parents per CTA: each warp applies its operator to TR_PB parents per load of an
-// operator row (4 where the shared staging fits the 48 KB static limit)
-template <int P>
-constexpr int tr_pb() { return (P + 1) * (P + 1) <= 81 ? 4 : 2; }
-// operator rows in flight per warp (at most ~128 registers, two CTAs per SM)
-template <int P>
-constexpr int tr_kb() { return (P + 1) * (P + 1) <= 96 ? 12 : 6; }
-
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-// bounded wait until *flag != 0; false when it ran out (*err is then set) or when
-// another wait already gave up
-__device__ bool wait_ready(const int* flag, int* err, uint32_t limit = sm100::kSpinLimit) {
-    for (uint32_t it = 0; it < limit; ++it) {
-        if (ld_acquire_gpu(flag)) return true;
-        if (*(volatile int*)err) return false;
-        if (it > 16) __nanosleep(64);
-    }
-    atomicExch(err, 1);
-    return false;
-}
-
-template <int P, int MODE>
-__global__ void __launch_bounds__(256) k_translate_flow(TreeView tv, const int* __restrict__ nonleaf,
-                                                        const int* __restrict__ nl_off, int nlev, int ibeg, int iend,
-                                                        const double* __restrict__ opsT, double* mpole, double* local,
-                                                        const double* __restrict__ lown, int* ready, int* ticket,
-                                                        int* err) {
-    constexpr int K = (P + 1) * (P + 1);
-    constexpr int NPL = (K + 31) / 32;
-    constexpr int TR_PB = tr_pb<P>();
-    __shared__ double s_in[MODE == 0 ? 8 : 1][TR_PB][K];
-    __shared__ double s_part[MODE == 0 ? 8 : 1][TR_PB][MODE == 0 ? K : 1];
-    __shared__ int s_gend[kMaxDepth + 2];   // groups of the pass's first i+1 levels
-    __shared__ int s_t;
-    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
-    if (tv_over(tv) || nlev <= 0 || ibeg >= iend) return;
-    if (threadIdx.x == 0) {
-        int c = 0;
-        for (int i = 0; i < iend; ++i) {
-            const int l = MODE == 1 ? i : nlev - 1 - i;
-            c += (nl_off[l + 1] - nl_off[l] + TR_PB - 1) / TR_PB;
-            s_gend[i] = c;
-        }
-    }
-    for (;;) {
-        __syncthreads();   // s_gend is written; the previous group's shared data was read
-        // this launch's levels are pass-order indices [ibeg, iend): its tickets count from
-        // the first group of level ibeg
-        if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1) + (ibeg > 0 ? s_gend[ibeg - 1] : 0);
-        __syncthreads();
-        const int t = s_t;
-        if (t >= s_gend[iend - 1]) break;
-        int i = 0;
-        while (t >= s_gend[i]) ++i;
-        const int l = MODE == 1 ? i : nlev - 1 - i;
-        const int p0 = (t - (i > 0 ? s_gend[i - 1] : 0)) * TR_PB;
-        const int first = nl_off[l], count = nl_off[l + 1] - first;
-        int bx[TR_PB], ch[TR_PB];
-        bool any = false;
-#pragma unroll
-        for (int a = 0; a < TR_PB; ++a) {
-            bx[a] = (p0 + a < count) ? nonleaf[first + p0 + a] : -1;
-            ch[a] = (bx[a] >= 0) ? tv.child[8 * bx[a] + s] : -1;
-            any |= ch[a] >= 0;
-        }
-        // wait for this group's inputs
-        if (MODE == 1) {
-            if (l > 0 && threadIdx.x < TR_PB) {
-                int b = -1;
-#pragma unroll
-                for (int a = 0; a < TR_PB; ++a) b = (a == (int)threadIdx.x) ? bx[a] : b;
-                if (b >= 0) wait_ready(ready + b, err);   // published by the group of b's parent
-            }
-        } else if (lane < TR_PB) {
-            int c = -1;
-#pragma unroll
-            for (int a = 0; a < TR_PB; ++a) c = (a == lane) ? ch[a] : c;
-            if (c >= 0 && tv.leafid[c] < 0) wait_ready(ready + c, err);
-        }
-        __syncthreads();
-        if (MODE == 0) {
-#pragma unroll
-            for (int a = 0; a < TR_PB; ++a)
-                for (int d = lane; d < K; d += 32) s_in[s][a][d] = (ch[a] >= 0) ? __ldcg(mpole + (size_t)ch[a] * K + d) : 0.0;
-            __syncwarp();
-        } else {
-#pragma unroll
-            for (int a = 0; a < TR_PB; ++a)
-                for (int d = threadIdx.x; d < K; d += blockDim.x) s_in[0][a][d] = (bx[a] >= 0) ? __ldcg(local + (size_t)bx[a] * K + d) : 0.0;
-            __syncthreads();
-        }
-        double acc[TR_PB][NPL];
-#pragma unroll
-        for (int a = 0; a < TR_PB; ++a)
-#pragma unroll
-            for (int q = 0; q < NPL; ++q) acc[a][q] = 0.0;
-        if (any) {  // warp-uniform
-            const double* T = opsT + (size_t)s * K * K;
-            const int si = MODE == 0 ? s : 0;
-            // operator rows in batches of TR_KB, all loads of a batch issued before its
-            // FMAs (the pass is bound by the chain of L2 round trips); kk order unchanged
-            constexpr int TR_KB = tr_kb<P>();
-            for (int k0 = 0; k0 < K; k0 += TR_KB) {
-                double tq[TR_KB][NPL];
-#pragma unroll
-                for (int u = 0; u < TR_KB; ++u)
-#pragma unroll
-                    for (int q = 0; q < NPL; ++q) {
-                        const int j = lane + 32 * q;
-                        tq[u][q] = (k0 + u < K && j < K) ? __ldg(T + (size_t)(k0 + u) * K + j) : 0.0;
-                    }
-#pragma unroll
-                for (int u = 0; u < TR_KB; ++u) {
-                    if (k0 + u >= K) break;
-#pragma unroll
-                    for (int a = 0; a < TR_PB; ++a) {
-                        const double v = s_in[si][a][k0 + u];
-#pragma unroll
-                        for (int q = 0; q < NPL; ++q) acc[a][q] = fma(tq[u][q], v, acc[a][q]);
-                    }
-                }
-            }
-        }
-        if (MODE == 1) {
-#pragma unroll
-            for (int a = 0; a < TR_PB; ++a) {
-                if (ch[a] < 0) continue;
-#pragma unroll
-                for (int q = 0; q < NPL; ++q) {
-                    const int j = lane + 32 * q;
-                    if (j < K) local[(size_t)ch[a] * K + j] = lown[(size_t)ch[a] * K + j] + acc[a][q];
-                }
-            }
-            __threadfence();
-            __syncthreads();
-            if (lane < TR_PB) {
-                int c = -1;
-#pragma unroll
-                for (int a = 0; a < TR_PB; ++a) c = (a == lane) ? ch[a] : c;
-                if (c >= 0) st_release_gpu(ready + c, 1);
-            }
-        } else {
-#pragma unroll
-            for (int a = 0; a < TR_PB; ++a)
-#pragma unroll
-                for (int q = 0; q < NPL; ++q) {
-                    const int j = lane + 32 * q;
-                    if (j < K) s_part[s][a][j] = acc[a][q];
-                }
-            __syncthreads();
-#pragma unroll
-            for (int a = 0; a < TR_PB; ++a) {
-                if (bx[a] < 0) continue;
-                for (int d = threadIdx.x; d < K; d += blockDim.x) {
-                    double v = 0.0;
-#pragma unroll
-                    for (int o = 0; o < 8; ++o) v += s_part[o][a][d];
-                    mpole[(size_t)bx[a] * K + d] = v;
-                }
-            }
-            __threadfence();
-            __syncthreads();
-            if (threadIdx.x < TR_PB) {
-                int b = -1;
-#pragma unroll
-                for (int a = 0; a < TR_PB; ++a) b = (a == (int)threadIdx.x) ? bx[a] : b;
-                if (b >= 0) st_release_gpu(ready + b, 1);
-            }
-        }
-    }
-}
-
-// Groups of one level's translation: enough for the level's boxes (eager: the level
-// size is known on the host; capacity mode: the level's capacity)
-template <int P>
-int translate_groups(const Handle& h, int l) {
-    if (h.cap_mode) return (h.cap.level_boxes[l] + tr_pb<P>() - 1) / tr_pb<P>();
-    const int nbl = h.level_off[l + 1] - h.level_off[l];   // bound on the level's parents
-    return (nbl + tr_pb<P>() - 1) / tr_pb<P>();
-}
-
-// A translation pass.  A tree of at least kFlowBoxes boxes takes one launch over every
-// level: CTAs for every SM (as many as fit), at most one per group.  A smaller tree (a
-// system that shares the GPU with others, typically) takes one launch per level, each
-// with its level's groups only: its level chain would otherwise keep waiting CTAs on
-// most SMs while its few groups per level run.  Same kernel, same arithmetic per box.
-// The ready flags and the ticket counters (one per launch) are cleared first.
-constexpr int kFlowBoxes = 32768;
-template <int P, int MODE>
-int launch_translate(Handle& h, Slot slot, double* M, double* L, const double* Lown) {
-    const int nlev = h.max_level;   // parent levels 0 .. max_level-1
-    if (nlev <= 0) return OGX_OK;
-    int groups = 0;
-    for (int l = 0; l < nlev; ++l) groups += translate_groups<P>(h, l);
-    if (groups <= 0) return OGX_OK;
-    static const int per_sm = [] {
-        int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_translate_flow<P, MODE>, 256, 0) != cudaSuccess) {
-            cudaGetLastError();
-            b = 1;
-        }
-        return std::max(1, b);
-    }();
-    int* ready;
-    const size_t nready = (size_t)h.tv.nb + kMaxDepth + 2;
-    OGX_TRY(arena_get(h.ws, slot, nready, &ready));
-    OGX_CUDA(cudaMemsetAsync(ready, 0, sizeof(int) * nready, h.stream));
-    int* tickets = ready + h.tv.nb;
-    const double* ops = MODE == 0 ? h.d_m2m : h.d_l2l;
-    if (h.tv.nb >= kFlowBoxes) {
-        const int grid = std::min(groups, per_sm * h.num_sms);
-        k_translate_flow<P, MODE><<<grid, 256, 0, h.stream>>>(h.tv, h.d_nonleaf, h.d_nonleaf_off, nlev, 0, nlev, ops, M, L,
-                                                              Lown, ready, tickets, h.d_err);
-        ++h.launches;
-    } else {
-        for (int i = 0; i < nlev; ++i) {
-            const int g = translate_groups<P>(h, MODE == 1 ? i : nlev - 1 - i);
-            if (g <= 0) continue;
-            k_translate_flow<P, MODE><<<std::min(g, per_sm * h.num_sms), 256, 0, h.stream>>>(
-                h.tv, h.d_nonleaf, h.d_nonleaf_off, nlev, i, i + 1, ops, M, L, Lown, ready, tickets + i, h.d_err);
-            ++h.launches;
-        }
-    }
-    OGX_CUDA(cudaGetLastError());
-    return OGX_OK;
-}
-
-template <int P>
-int launch_m2m(Handle& h, double* M) {
-    return launch_translate<P, 0>(h, S_TR_READY_M, M, nullptr, nullptr);
-}
-
-template <int P>
-int launch_l2l(Handle& h, double* L, const double* Lown) {
-    constexpr int K = (P + 1) * (P + 1);
-    // root (no parent): its local is its own M2L/P2L part
-    OGX_CUDA(cudaMemcpyAsync(L, Lown, sizeof(double) * K, cudaMemcpyDeviceToDevice, h.stream));   // box 0 is the root
-    return launch_translate<P, 1>(h, S_TR_READY_L, nullptr, L, Lown);
-}
-
-// ---- leaf near field (P2P over U) + final combine ----------------------------------------
+// ---- work items of the near field (ogx_near.cuh) ----------------------------------------
 // the leaf and first target of near-field work item w (leaf, chunk of 32 targets):
 // chunk_off[lf] <= w < chunk_off[lf + 1]; false past the last item
 __device__ __forceinline__ bool near_item(const TreeView& tv, const int64_t* chunk_off, int64_t w, int& lf, int& j0) {
@@ -367,59 +105,6 @@ __device__ __forceinline__ bool near_item(const TreeView& tv, const int64_t* chu
     lf = lo;
     j0 = 32 * (int)(w - chunk_off[lo]);
     return true;
-}
-
-// Warp per work item (leaf, chunk of 32 targets), so a leaf held large by the eps floor
-// spreads over many warps.
-template <bool POT, bool SOFT = false>
-__global__ void __launch_bounds__(128) k_leaf_near(TreeView tv, const int64_t* __restrict__ chunk_off, double G, double eps2,
-                                                   const double* far, double* acc, double* pot, double hs = 0.0,
-                                                   double hinv = 0.0) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int lf, j0;
-    if (tv_over(tv) || !near_item(tv, chunk_off, blockIdx.x * 4 + wid, lf, j0)) return;
-    const int b = tv.leafbox[lf];
-    const int f0 = tv.pfirst[b], cnt = tv.pcount[b];
-    {
-        const int jj = j0 + lane;
-        const bool act = jj < cnt;
-        const int i = f0 + (act ? jj : 0);
-        const double x = tv.px[i], y = tv.py[i], z = tv.pz[i];
-        double ax = 0, ay = 0, az = 0, ph = 0;
-        for (int64_t e = tv.u_off[lf]; e < tv.u_off[lf + 1]; ++e) {
-            const int c = tv.u_idx[e];
-            const int s0 = tv.pfirst[c], sc = tv.pcount[c];
-            for (int j = s0; j < s0 + sc; ++j) {
-                const double dx = __ldg(tv.px + j) - x, dy = __ldg(tv.py + j) - y, dz = __ldg(tv.pz + j) - z;
-                const double mj = (j == i) ? 0.0 : __ldg(tv.pm + j);
-                if constexpr (SOFT) {
-                    const double r2 = dx * dx + dy * dy + dz * dz;
-                    double g, k;
-                    spline_gk<double>(j == i ? 1.0 : r2, hs, hinv, g, k);
-                    const double w = mj * g;
-                    if (j != i) {
-                        ax = fma(w, dx, ax); ay = fma(w, dy, ay); az = fma(w, dz, az);
-                        if (POT) ph = fma(mj, k, ph);
-                    }
-                } else {
-                    const double r2 = (dx * dx + dy * dy + dz * dz) + eps2;
-                    const double ir = rsqrt(r2);
-                    const double w = mj * ir * ir * ir;
-                    if (j != i) {
-                        ax = fma(w, dx, ax); ay = fma(w, dy, ay); az = fma(w, dz, az);
-                        if (POT) ph = fma(mj, ir, ph);
-                    }
-                }
-            }
-        }
-        if (act) {
-            const int o = tv.perm[i];
-            acc[3 * (size_t)o] = G * (far[4 * (size_t)i] + ax);
-            acc[3 * (size_t)o + 1] = G * (far[4 * (size_t)i + 1] + ay);
-            acc[3 * (size_t)o + 2] = G * (far[4 * (size_t)i + 2] + az);
-            if (POT) pot[o] = -G * (far[4 * (size_t)i + 3] + ph);
-        }
-    }
 }
 
 // ---- OGX_SOFT_SPLINE: the far field's pairs within the support ------------------------
@@ -474,19 +159,6 @@ __global__ void __launch_bounds__(128) k_soft_correct(TreeView tv, const int64_t
 
 }  // namespace
 
-// One thread runs the translation passes' bounded flag wait, with a limit of `polls`, on
-// a flag that nothing sets: the wait runs out and sets *err as in the passes.
-__global__ void k_flag_wait_probe(const int* flag, int* err, uint32_t polls) {
-    if (threadIdx.x == 0) wait_ready(flag, err, polls);
-}
-
-int flag_wait_probe(Handle& h, uint32_t polls, const int* flag, int* err) {
-    k_flag_wait_probe<<<1, 32, 0, h.stream>>>(flag, err, polls);
-    ++h.launches;
-    OGX_CUDA(cudaGetLastError());
-    return OGX_OK;
-}
-
 // work items of the near field (leaf, chunk of 32 targets), on h.stream; the grid of a
 // warp-per-item kernel needs at most nleaf + n / 32 warps
 int near_items(Handle& h, int64_t** chunk_off) {
@@ -494,7 +166,7 @@ int near_items(Handle& h, int64_t** chunk_off) {
     int* nchunk;
     OGX_TRY(arena_get(h.ws, S_NEAR_CHUNK, (size_t)tv.nleaf, &nchunk));
     OGX_TRY(arena_get(h.ws, S_NEAR_CHUNK_OFF, (size_t)tv.nleaf + 1, chunk_off));
-    mixed::k_near_chunks<<<(tv.nleaf + 255) / 256, 256, 0, h.stream>>>(tv, nchunk); ++h.launches;
+    near_field::k_near_chunks<<<(tv.nleaf + 255) / 256, 256, 0, h.stream>>>(tv, nchunk); ++h.launches;
     return scan_i32_to_i64(h, nchunk, *chunk_off, tv.nleaf);
 }
 
@@ -526,11 +198,8 @@ int run_fp64(Handle& h, double* d_acc, double* d_pot) {
     OGX_TRY(arena_get(h.ws, S_FAR, 4 * (size_t)tv.n, &far));
     OGX_CUDA(timing_record(h, h.ev[2], st));
     // upward
-    const size_t p2x_smem = p2x_smem_bytes<P, double>();
-    OGX_CUDA(smem_optin((const void*)k_p2x<P, 0, double>, (int)p2x_smem));
-    OGX_CUDA(smem_optin((const void*)k_p2x<P, 1, double>, (int)p2x_smem));
-    k_p2x<P, 0, double><<<(tv.nleaf + 3) / 4, 128, p2x_smem, st>>>(tv, tv.nleaf, M); ++h.launches;
-    OGX_TRY(launch_m2m<P>(h, M));
+    p2x::k_p2x<P, 0, double><<<tv.nleaf, 32, p2x::p2x_smem<P, double>(), st>>>(tv, tv.nleaf, M); ++h.launches;
+    OGX_TRY(m2m_launch(h, M));
     OGX_CUDA(timing_record(h, h.ev[3], st));
     // M2L
     OGX_CUDA(cudaMemsetAsync(Lown, 0, sizeof(double) * (size_t)tv.nb * K, st));
@@ -542,10 +211,10 @@ int run_fp64(Handle& h, double* d_acc, double* d_pot) {
     }
     OGX_CUDA(timing_record(h, h.ev[4], st));
     // P2L
-    k_p2x<P, 1, double><<<(tv.nb + 3) / 4, 128, p2x_smem, st>>>(tv, tv.nb, Lown); ++h.launches;
+    p2x::k_p2x<P, 1, double><<<tv.nb, 32, p2x::p2x_smem<P, double>(), st>>>(tv, tv.nb, Lown); ++h.launches;
     OGX_CUDA(timing_record(h, h.ev[5], st));
     // L2L top-down
-    OGX_TRY(launch_l2l<P>(h, L, Lown));
+    OGX_TRY(l2l_launch(h, L, Lown));
     OGX_CUDA(timing_record(h, h.ev[6], st));
     // leaves
     const bool pot = d_pot != nullptr;
@@ -554,16 +223,20 @@ int run_fp64(Handle& h, double* d_acc, double* d_pot) {
     const double G = h.prm.G, eps2 = h.prm.eps * h.prm.eps;
     int64_t* chunk_off;
     OGX_TRY(near_items(h, &chunk_off));
-    const int ngrid = (tv.nleaf + (tv.n + 31) / 32 + 3) / 4;   // a warp per work item
-    if (h.prm.softening == OGX_SOFT_SPLINE) {
-        // the far field's pairs within the support, then the spline kernel in the near field
-        OGX_TRY(soft_correct_launch(h, chunk_off, far, pot, st));
-        const double hs = spline_support(h.prm.eps), hinv = hs > 0.0 ? 1.0 / hs : 0.0;
-        if (pot) k_leaf_near<true, true><<<ngrid, 128, 0, st>>>(tv, chunk_off, G, eps2, far, d_acc, d_pot, hs, hinv);
-        else k_leaf_near<false, true><<<ngrid, 128, 0, st>>>(tv, chunk_off, G, eps2, far, d_acc, nullptr, hs, hinv);
-        ++h.launches;
-    } else if (pot) { k_leaf_near<true><<<ngrid, 128, 0, st>>>(tv, chunk_off, G, eps2, far, d_acc, d_pot); ++h.launches; }
-    else { k_leaf_near<false><<<ngrid, 128, 0, st>>>(tv, chunk_off, G, eps2, far, d_acc, nullptr); ++h.launches; }
+    double* nearb;
+    OGX_TRY(arena_get(h.ws, S_NEAR32, 4 * (size_t)tv.n, &nearb));
+    const bool soft = h.prm.softening == OGX_SOFT_SPLINE;
+    // the far field's pairs within the support, then the spline kernel in the near field
+    if (soft) OGX_TRY(soft_correct_launch(h, chunk_off, far, pot, st));
+    using near_field::Near64;
+    const double hs = soft ? spline_support(h.prm.eps) : 0.0;
+    const near_field::NearPrm<double> npr{eps2, hs, hs > 0.0 ? 1.0 / hs : 0.0};
+    const Near64::Bodies bod{tv.px, tv.py, tv.pz, tv.pm};
+    auto near = pot ? (soft ? near_field::k_leaf_near<Near64, true, 64, 1> : near_field::k_leaf_near<Near64, true, 64>)
+                    : (soft ? near_field::k_leaf_near<Near64, false, 64, 1> : near_field::k_leaf_near<Near64, false, 64>);
+    near<<<tv.nleaf + (tv.n + 31) / 32, 32, 0, st>>>(tv, chunk_off, bod, npr, nearb); ++h.launches;
+    auto combine = pot ? mixed::k_combine<true> : mixed::k_combine<false>;
+    combine<<<(tv.n + 255) / 256, 256, 0, st>>>(tv.n, tv.perm, G, far, nullptr, nearb, d_acc, d_pot, tv.cnt); ++h.launches;
     OGX_CUDA(timing_record(h, h.ev[7], st));
     OGX_CUDA(cudaGetLastError());
     return OGX_OK;
@@ -674,15 +347,13 @@ int run_mixed_upward(Handle& h) {
     OGX_TRY(arena_get(h.ws, S_MIX_MHI, (size_t)tv.nb * C::KPAD, &mhi));
     OGX_TRY(arena_get(h.ws, S_MIX_MLO, (size_t)tv.nb * C::KPAD, &mlo));
     OGX_TRY(arena_get(h.ws, S_MIX_MUNSCALE, (size_t)tv.nb, &mus));
-    const size_t p2x_smem = p2x_smem_bytes<P, float>();
-    OGX_CUDA(smem_optin((const void*)k_p2x<P, 0, float>, (int)p2x_smem));
     OGX_CUDA(cudaEventRecord(h.ev_tree, h.stream));
     const cudaStream_t main_st = h.stream, su = h.up;
     OGX_CUDA(cudaStreamWaitEvent(su, h.ev_tree, 0));
-    h.stream = su;   // launch_m2m issues on h.stream
+    h.stream = su;   // m2m_launch issues on h.stream
     OGX_CUDA(timing_record(h, h.ev[2], su));
-    k_p2x<P, 0, float><<<(tv.nleaf + 3) / 4, 128, p2x_smem, su>>>(tv, tv.nleaf, M); ++h.launches;
-    const int rc = launch_m2m<P>(h, M);
+    p2x::k_p2x<P, 0, float><<<tv.nleaf, 32, p2x::p2x_smem<P, float>(), su>>>(tv, tv.nleaf, M); ++h.launches;
+    const int rc = m2m_launch(h, M);
     h.stream = main_st;
     OGX_TRY(rc);
     if constexpr (C::SUPPORTED) {
@@ -743,8 +414,6 @@ int run_mixed(Handle& h, double* d_acc, double* d_pot) {
     double *nearb, *far_m;
     OGX_TRY(arena_get(h.ws, S_NEAR32, 4 * (size_t)tv.n, &nearb));
     OGX_TRY(arena_get(h.ws, S_FAR_M, 4 * (size_t)tv.n, &far_m));
-    const size_t p2x_smem = p2x_smem_bytes<P, float>();
-    OGX_CUDA(smem_optin((const void*)k_p2x<P, 1, float>, (int)p2x_smem));
     // near-field work items (leaf, chunk of 32 targets)
     int64_t* chunk_off;
     OGX_TRY(near_items(h, &chunk_off));
@@ -758,43 +427,38 @@ int run_mixed(Handle& h, double* d_acc, double* d_pot) {
     // SMs its last wave leaves idle, and then what P2L, L2L and the far field leave idle
     {
         const float eps2 = (float)(h.prm.eps * h.prm.eps);
-        float4* rel;
-        OGX_TRY(arena_get(h.ws, S_MIX_POS4, 2 * (size_t)tv.n, &rel));
         OGX_CUDA(cudaStreamWaitEvent(h.side, h.ev_fork, 0));
         // the far field's M2P part (multipoles only) first, then the near field
         if (d_pot) OGX_TRY((launch_m2p<P, true, false, float>(h, M, nullptr, far_m, h.side)));
         else OGX_TRY((launch_m2p<P, false, false, float>(h, M, nullptr, far_m, h.side)));
-        mixed::k_near_prep<<<(tv.n + 255) / 256, 256, 0, h.side>>>(tv, rel, rel + tv.n); ++h.launches;
         // one block per work item: the leaves' chunks number at most nleaf + n / 32 (a
         // bounded grid left the far chain waiting)
         const int ngrid = tv.nleaf + (tv.n + 31) / 32;
-        if (h.prm.softening == OGX_SOFT_SPLINE) {
-            // spline kernel in the near field; the far field's pairs within the support are
-            // corrected in FP32 into the M2P part (written above on this stream)
-            const double hs = spline_support(h.prm.eps);
-            const float hsf = (float)hs, hinvf = hs > 0.0 ? (float)(1.0 / hs) : 0.f;
-            auto near = d_pot ? (h.near_units == 32 ? mixed::k_leaf_near32<true, 32, 1> : mixed::k_leaf_near32<true, 64, 1>)
-                              : (h.near_units == 32 ? mixed::k_leaf_near32<false, 32, 1> : mixed::k_leaf_near32<false, 64, 1>);
-            near<<<ngrid, 32, 0, h.side>>>(tv, chunk_off, rel, rel + tv.n, eps2, nearb, hsf, hinvf); ++h.launches;
-            if (h.soft_pairs > 0) {
-                // the same staging over the S lists, the kernel difference added into far_m
-                auto corr = d_pot ? (h.near_units == 32 ? mixed::k_leaf_near32<true, 32, 2> : mixed::k_leaf_near32<true, 64, 2>)
-                                  : (h.near_units == 32 ? mixed::k_leaf_near32<false, 32, 2> : mixed::k_leaf_near32<false, 64, 2>);
-                corr<<<ngrid, 32, 0, h.side>>>(tv, chunk_off, rel, rel + tv.n, eps2, far_m, hsf, hinvf); ++h.launches;
-            }
-        } else {
-            auto near = d_pot ? (h.near_units == 32 ? mixed::k_leaf_near32<true, 32> : mixed::k_leaf_near32<true, 64>)
-                              : (h.near_units == 32 ? mixed::k_leaf_near32<false, 32> : mixed::k_leaf_near32<false, 64>);
-            near<<<ngrid, 32, 0, h.side>>>(tv, chunk_off, rel, rel + tv.n, eps2, nearb, 0.f, 0.f); ++h.launches;
+        // spline kernel in the near field; the far field's pairs within the support are
+        // corrected in FP32 into the M2P part (written above on this stream)
+        const bool soft = h.prm.softening == OGX_SOFT_SPLINE, p = d_pot != nullptr, u32 = h.near_units == 32;
+        const double hs = soft ? spline_support(h.prm.eps) : 0.0;
+        using near_field::Near32;
+        const near_field::NearPrm<float> npr{eps2, (float)hs, hs > 0.0 ? (float)(1.0 / hs) : 0.f};
+        const Near32::Bodies bod{tv.rhi, tv.rlo};
+        auto pick = [&](auto km) {
+            constexpr int KM = decltype(km)::value;
+            return p ? (u32 ? near_field::k_leaf_near<Near32, true, 32, KM> : near_field::k_leaf_near<Near32, true, 64, KM>)
+                     : (u32 ? near_field::k_leaf_near<Near32, false, 32, KM> : near_field::k_leaf_near<Near32, false, 64, KM>);
+        };
+        auto near = soft ? pick(std::integral_constant<int, 1>{}) : pick(std::integral_constant<int, 0>{});
+        near<<<ngrid, 32, 0, h.side>>>(tv, chunk_off, bod, npr, nearb); ++h.launches;
+        if (soft && h.soft_pairs > 0) {
+            // the same staging over the S lists, the kernel difference added into far_m
+            pick(std::integral_constant<int, 2>{})<<<ngrid, 32, 0, h.side>>>(tv, chunk_off, bod, npr, far_m); ++h.launches;
         }
         OGX_CUDA(cudaEventRecord(h.ev_join, h.side));
     }
     // join the M2L (its end is timing event 4, recorded on h.m2l)
     OGX_CUDA(cudaStreamWaitEvent(st, h.ev_m2l, 0));
-    if constexpr (mixed::P2L32<P>::OK) { mixed::k_p2l32<P><<<tv.nb, 32, 0, st>>>(tv, Lown); ++h.launches; }
-    else { k_p2x<P, 1, float><<<(tv.nb + 3) / 4, 128, p2x_smem, st>>>(tv, tv.nb, Lown); ++h.launches; }
+    p2x::k_p2x<P, 1, float><<<tv.nb, 32, p2x::p2x_smem<P, float>(), st>>>(tv, tv.nb, Lown); ++h.launches;
     OGX_CUDA(timing_record(h, h.ev[5], st));
-    OGX_TRY(launch_l2l<P>(h, L, Lown));
+    OGX_TRY(l2l_launch(h, L, Lown));
     OGX_CUDA(timing_record(h, h.ev[6], st));
     const bool pot = d_pot != nullptr;
     if (pot) OGX_TRY((launch_l2p32<P, true>(h, L, far)));

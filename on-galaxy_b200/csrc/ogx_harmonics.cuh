@@ -37,6 +37,8 @@ struct HarmTables {
     double hz[kTab][kTab], hp[kTab][kTab], hm[kTab][kTab];  // mpole  -> degree n (from degree n-1)
     // R_n^m = s[n][m] (x+iy)^m T_nm: the product of the recurrence constants (ogx_far.cuh)
     double s[kTab][kTab];
+    // the same per real dof, negative for imaginary parts (conjugate sums, ogx_p2x.cuh)
+    double sd[(kPMax + 1) * (kPMax + 1)];
     // FP32 copies of the recurrence constants for the FP32 kernels (no conversion per use)
     float fa[kTab], fb[kTab], fA[kTab][kTab], fB[kTab][kTab];
 };
@@ -98,6 +100,12 @@ static inline void fill_harm_tables(HarmTables& t) {
             t.s[n][m] = v;
         }
     }
+    for (int n = 0; n <= kPMax; ++n)
+        for (int m = 0; m <= n; ++m) {
+            const int d = m == 0 ? n * n : n * n + 2 * m - 1;
+            t.sd[d] = t.s[n][m];
+            if (m > 0) t.sd[d + 1] = -t.s[n][m];
+        }
 }
 
 static inline int harm_tables_ready(int device) {

@@ -173,6 +173,8 @@ struct TreeView {
     const RootInfo* root;
     const double *px, *py, *pz, *pm;   // sorted bodies
     const int* perm;                   // sorted -> original
+    // mixed form: sorted bodies relative to the root centre, hi + lo FP32 (mass in rhi.w)
+    const float4 *rhi, *rlo;
     const int* level;                  // per box
     const int* coord;                  // per box: ix, iy, iz (3 ints)
     const double* center;              // per box: cx, cy, cz, half
@@ -227,9 +229,10 @@ struct Handle {
     int64_t n = 0;
     // operator tables for prm.p (host built, device resident)
     int ops_p = -1;
-    double* d_m2l = nullptr;  // 343 x K x K
-    double* d_m2m = nullptr;  // 8 x K x K
-    double* d_l2l = nullptr;  // 8 x K x K
+    // k-major, rows and columns padded with zeros (m2l64_pad_rows, m2l64_pad_cols)
+    double* d_m2l = nullptr;  // 343 operators
+    double* d_m2m = nullptr;  // 8
+    double* d_l2l = nullptr;  // 8
     // device-resident integrator state
     bool resident = false;
     bool species_set = false;       // species tags uploaded (or made by ogx_ic_merger)
@@ -338,12 +341,13 @@ int soft_lists_build(Handle& h);      // OGX_SOFT_SPLINE: the leaf pairs the far
 int soft_correct_launch(Handle& h, const int64_t* chunk_off, double* out, bool pot, cudaStream_t st);   // FP64: adds the kernel difference over them
 int fmm_fp64(Handle& h, double* d_acc, double* d_pot);
 int fmm_mixed(Handle& h, double* d_acc, double* d_pot);
+int m2m_launch(Handle& h, double* M);                       // ogx_translate.cu, on h.stream
+int l2l_launch(Handle& h, double* L, const double* Lown);
 int m2l_rot_launch(Handle& h, const double* M, double* Lown);   // third form's M2L, on h.stream
 int fmm_mixed_upward(Handle& h);   // upward pass on h.up, right after the tree (before the lists)
 int fmm_mixed_m2l(Handle& h, bool pot);   // tensor-core M2L on h.m2l, after the target tiles
 int flag_wait_probe(Handle& h, uint32_t polls, const int* flag, int* err);   // translation passes' wait, run out
-int direct_eval(Handle& h, const double* d_pos, const double* d_mass, int64_t n, double* d_acc,
-                double* d_pot, bool fp32);
+int direct_eval(Handle& h, const double* d_pos, const double* d_mass, int64_t n, double* d_acc, double* d_pot);
 int ensure_operator_tables(Handle& h);
 void drop_step_graph(Handle& h);   // ogx_api.cu
 int eval_device_shared(Handle& h, int64_t n, const double* d_pos, const double* d_mass, double* d_acc, double* d_pot);

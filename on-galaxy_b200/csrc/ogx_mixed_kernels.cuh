@@ -46,17 +46,12 @@
 // slices (2 x 72 and 3 x 56 dofs), each handled by its own CTA (grid y) in the
 // paired form with one 64- or 80-column operand; the A rows are gathered once per
 // slice.
-//
-// Near field in FP32 on leaf-centred double-float coordinates (hi + lo FP32
-// relative to the target leaf centre, shift in FP64), r^-1 from rsqrt, every
-// U-list entry's partial sum folded into a compensated (Kahan) accumulator.
 #pragma once
 
 #include <cuda_fp16.h>
 
 #include "ogx_harmonics.cuh"
 #include "ogx_sm100.cuh"
-#include "ogx_softening.cuh"
 
 namespace ogx {
 namespace mixed {
@@ -623,269 +618,6 @@ __global__ void __launch_bounds__(128) k_m2l_dof0(TreeView tv, int ntgt_pad, con
     lown[(size_t)b * K] += acc / (2.0 * tv.center[4 * b + 3]);
 }
 
-// ---- FP32 near field ------------------------------------------------------------
-// Double-float coordinates: every sorted body's position relative to the root centre
-// is held as hi + lo FP32 (hi = fp32(x - c), lo = fp32((x - c) - hi), the difference
-// taken in FP64; k_near_prep, once per evaluation).  For a close pair the two hi parts
-// lie within a factor of two of each other, so s_hi - t_hi is exact (Sterbenz) and
-// d = (s_hi - t_hi) + (s_lo - t_lo) carries the FP32 relative accuracy of |d| itself
-// (absolute error ~2^-48 of the root box), however small |d| is.  No per-leaf shift
-// is needed, so the sources of many U-list entries are staged together.
-__device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
-    const float y = v - c;
-    const float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
-constexpr int NEAR_CAP = 128;    // source bodies staged per round (several U-list entries)
-
-// work items of the near field: ceil(bodies / 32) per leaf (none for capacity padding)
-__global__ void k_near_chunks(TreeView tv, int* __restrict__ cnt) {
-    const int lf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lf >= tv.nleaf) return;
-    cnt[lf] = (lf < tv_nleaf(tv) && !tv_over(tv)) ? (tv.pcount[tv.leafbox[lf]] + 31) / 32 : 0;
-}
-
-__global__ void __launch_bounds__(256) k_near_prep(TreeView tv, float4* __restrict__ rhi, float4* __restrict__ rlo) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= tv.n || tv_over(tv)) return;
-    const double ex = tv.px[i] - tv.root->c[0], ey = tv.py[i] - tv.root->c[1], ez = tv.pz[i] - tv.root->c[2];
-    const float hx = (float)ex, hy = (float)ey, hz = (float)ez;
-    rhi[i] = make_float4(hx, hy, hz, (float)tv.pm[i]);
-    rlo[i] = make_float4((float)(ex - (double)hx), (float)(ey - (double)hy), (float)(ez - (double)hz), 0.f);
-}
-
-// softened pair sum of one target over staged sources q = q0, q0 + dq, ... < n;
-// SELF: the source at staged position self_q is the target itself and is skipped.
-// KM (kernel): 0 Plummer's (eps2); 1 the spline of support hs (ogx_softening.cuh);
-// 2 the spline minus the Newtonian kernel, zero from hs on (the far field's pairs
-// inside the support, OGX_SOFT_SPLINE)
-template <bool SELF, bool POT, int KM = 0>
-__device__ __forceinline__ void p2p_part(const float4* __restrict__ shi, const float4* __restrict__ slo, int q0, int dq, int n,
-                                         int self_q, const float (&th)[3], const float (&tl)[3], float eps2, float (&a)[4],
-                                         float hs = 0.f, float hinv = 0.f) {
-#pragma unroll 4
-    for (int q = q0; q < n; q += dq) {
-        const float4 h = shi[q];
-        const float4 l = slo[q];
-        const float dx = (h.x - th[0]) + (l.x - tl[0]);
-        const float dy = (h.y - th[1]) + (l.y - tl[1]);
-        const float dz = (h.z - th[2]) + (l.z - tl[2]);
-        const bool self = SELF && (q == self_q);
-        if constexpr (KM == 1) {
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            float g, k;
-            spline_gk<float>(self ? 1.0f : r2, hs, hinv, g, k);
-            const float m = self ? 0.0f : h.w;
-            const float w = m * g;
-            a[0] = fmaf(w, dx, a[0]);
-            a[1] = fmaf(w, dy, a[1]);
-            a[2] = fmaf(w, dz, a[2]);
-            if (POT) a[3] = fmaf(m, k, a[3]);
-        } else if constexpr (KM == 2) {
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            if (r2 < hs * hs && r2 > 0.0f) {
-                float g, k;
-                spline_gk<float>(r2, hs, hinv, g, k);
-                const float y = rsqrtf(r2);
-                const float w = h.w * (g - y * y * y);
-                a[0] = fmaf(w, dx, a[0]);
-                a[1] = fmaf(w, dy, a[1]);
-                a[2] = fmaf(w, dz, a[2]);
-                if (POT) a[3] = fmaf(h.w, k - y, a[3]);
-            }
-        } else {
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-            // rsqrtf alone (within 2 ulp): its error, ~1e-7 per pair in random directions,
-            // stays far below the form's budget
-            const float y = rsqrtf(self ? 1.0f : r2);
-            const float my = (self ? 0.0f : h.w) * y;
-            const float w = my * y * y;
-            a[0] = fmaf(w, dx, a[0]);
-            a[1] = fmaf(w, dy, a[1]);
-            a[2] = fmaf(w, dz, a[2]);
-            if (POT) a[3] += my;
-        }
-    }
-}
-
-// Number of source parts G for a chunk of T targets: units (target, part) = T G,
-// at most NU, are spread over the 32 lanes in R = ceil(T G / 32) rounds; G maximises
-// the busy fraction T G / (32 R) (ties: the smaller G).  With NU = 64 a 17-body leaf
-// gets G = 3 (80% busy; one target per lane would leave 47% of the lanes idle), a
-// 5-body leaf G = 6 (94%).
-template <int NU>
-__device__ __forceinline__ int near_parts(int T) {
-    int best = 1, bu = 0;
-    for (int G = 1; G <= 32 && T * G <= NU; ++G) {
-        const int U = T * G;
-        const int u = (U << 10) / (32 * ((U + 31) >> 5));   // busy fraction, fixed point
-        if (u > bu) { bu = u; best = G; }
-    }
-    return best;
-}
-
-// Warp per target leaf (one warp per block, so a block's resources return as soon as
-// its leaf is done).  The leaf's bodies go in chunks of up to 32 targets; in a chunk
-// of T targets, unit u = lane + 32 r (r < NU / 32) is target u mod T with source part
-// u / T, which takes every G-th source of each staged round.  The leaf itself is one
-// round (with the self pair skipped); the bodies of all other U-list entries are
-// concatenated and staged NEAR_CAP at a time.  Each unit folds every round's partial
-// sum into a compensated (Kahan) accumulator; at the end the G parts of each target
-// are added in part order in FP64 through shared memory (deterministic).  Output:
-// near[4 i] = (sum m d / r^3 xyz, sum m / r) of sorted body i, FP64.  The kernel needs
-// only the tree and the lists, so it runs beside the far-field chain.
-// KM = 1: the spline kernel (OGX_SOFT_SPLINE).  KM = 2: the far field's pairs inside the
-// spline's support instead: the leaf's S list in place of its U list (no self round),
-// the kernel difference, and the result added to near[] rather than stored.
-// Work items are (leaf, chunk of 32 targets): chunk_off[lf] is the first item of leaf lf
-// (k_near_chunks + an exclusive scan), so a leaf of many bodies (the eps floor stops
-// splitting in dense cores) spreads over as many blocks as it has chunks.
-template <bool POT, int NU, int KM = 0>
-__global__ void __launch_bounds__(32, 32) k_leaf_near32(TreeView tv, const int64_t* __restrict__ chunk_off,
-                                                        const float4* __restrict__ rhi, const float4* __restrict__ rlo,
-                                                        float eps2, double* __restrict__ near, float hs = 0.f,
-                                                        float hinv = 0.f) {
-    constexpr int R = NU / 32;
-    static_assert(R * 32 == NU && R >= 1 && R <= 2, "near-field units: 32 or 64");
-    __shared__ float4 s_hi[NEAR_CAP], s_lo[NEAR_CAP];
-    __shared__ double s_red[NU][4];
-    const int lane = threadIdx.x & 31;
-    if (tv_over(tv)) return;
-    const int64_t items = chunk_off[tv.nleaf];
-    for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
-        // the leaf of item w: chunk_off[lf] <= w < chunk_off[lf + 1] (warp-uniform search)
-        int lo = 0, hi = tv.nleaf;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (chunk_off[mid] <= w) lo = mid;
-            else hi = mid;
-        }
-        const int lf = lo;
-        const int b = tv.leafbox[lf];
-        const int f0 = tv.pfirst[b], cnt = tv.pcount[b];
-        const int64_t u0 = KM == 2 ? tv.s_off[lf] : tv.u_off[lf], u1 = KM == 2 ? tv.s_off[lf + 1] : tv.u_off[lf + 1];
-        if (KM == 2 && u0 == u1) continue;
-        {
-            const int j0 = 32 * (int)(w - chunk_off[lf]);
-            const int T = min(32, cnt - j0);
-            const int G = near_parts<NU>(T);
-            const int U = T * G;
-            // the lane's units: target tt[r] (index in the leaf), source part pp[r]
-            int tt[R], pp[R];
-            bool act[R];
-            float th[R][3], tl[R][3];
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                const int u = lane + 32 * r;
-                act[r] = u < U;
-                tt[r] = act[r] ? u % T : 0;
-                pp[r] = act[r] ? u / T : 0;
-                const float4 h = rhi[f0 + j0 + tt[r]], l = rlo[f0 + j0 + tt[r]];
-                th[r][0] = h.x; th[r][1] = h.y; th[r][2] = h.z;
-                tl[r][0] = l.x; tl[r][1] = l.y; tl[r][2] = l.z;
-            }
-            float ks[R][4], kc[R][4];
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) ks[r][k] = kc[r][k] = 0.f;
-            // round 0: the leaf itself
-            for (int k0 = 0; k0 < (KM == 2 ? 0 : cnt); k0 += NEAR_CAP) {
-                const int n = min(NEAR_CAP, cnt - k0);
-                __syncwarp();
-                for (int q = lane; q < n; q += 32) {
-                    s_hi[q] = rhi[f0 + k0 + q];
-                    s_lo[q] = rlo[f0 + k0 + q];
-                }
-                __syncwarp();
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (!act[r]) continue;
-                    float a[4] = {0.f, 0.f, 0.f, 0.f};
-                    p2p_part<true, POT, KM>(s_hi, s_lo, pp[r], G, n, j0 + tt[r] - k0, th[r], tl[r], eps2, a, hs, hinv);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < 3 || POT) kahan_add(ks[r][k], kc[r][k], a[k]);
-                }
-            }
-            // the other U-list entries, 32 at a time: lane e holds entry e's first body and
-            // count; an inclusive scan of the counts maps a flat source position to its entry
-            for (int64_t eb = u0; eb < u1; eb += 32) {
-                const int64_t e = eb + lane;
-                int pf = 0, pc = 0;
-                if (e < u1) {
-                    const int c = KM == 2 ? tv.s_idx[e] : tv.u_idx[e];
-                    if (c != b) { pf = tv.pfirst[c]; pc = tv.pcount[c]; }
-                }
-                int pre = pc;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, pre, o);
-                    if (lane >= o) pre += v;
-                }
-                const int total = __shfl_sync(0xffffffffu, pre, 31);
-                for (int base = 0; base < total; base += NEAR_CAP) {
-                    const int n = min(NEAR_CAP, total - base);
-                    __syncwarp();
-                    // warp-uniform trip count: every lane takes part in every shuffle
-                    for (int q0 = 0; q0 < n; q0 += 32) {
-                        const int q = q0 + lane;
-                        const int f = base + q;
-                        // entry of flat position f: the number of entries whose inclusive
-                        // prefix is <= f (five halving steps over the 32 prefixes)
-                        int pos = 0;
-#pragma unroll
-                        for (int step = 16; step > 0; step >>= 1)
-                            if (__shfl_sync(0xffffffffu, pre, pos + step - 1) <= f) pos += step;
-                        const int ep = __shfl_sync(0xffffffffu, pre, pos), ec = __shfl_sync(0xffffffffu, pc, pos);
-                        const int j = __shfl_sync(0xffffffffu, pf, pos) + f - (ep - ec);
-                        if (q < n) {
-                            s_hi[q] = rhi[j];
-                            s_lo[q] = rlo[j];
-                        }
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        if (!act[r]) continue;
-                        float a[4] = {0.f, 0.f, 0.f, 0.f};
-                        p2p_part<false, POT, KM>(s_hi, s_lo, pp[r], G, n, -1, th[r], tl[r], eps2, a, hs, hinv);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (k < 3 || POT) kahan_add(ks[r][k], kc[r][k], a[k]);
-                    }
-                }
-            }
-            // the parts of every target, in part order, in FP64
-            __syncwarp();
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (act[r])
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) s_red[lane + 32 * r][k] = (double)ks[r][k] - (double)kc[r][k];
-            __syncwarp();
-            if (lane < T) {
-                double v[4] = {0.0, 0.0, 0.0, 0.0};
-                for (int p = 0; p < G; ++p)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) v[k] += s_red[p * T + lane][k];
-                double2* o = reinterpret_cast<double2*>(near + 4 * (size_t)(f0 + j0 + lane));
-                if (KM == 2) {
-                    const double2 o0 = o[0], o1 = o[1];
-                    o[0] = make_double2(o0.x + v[0], o0.y + v[1]);
-                    o[1] = make_double2(o1.x + v[2], o1.y + (POT ? v[3] : 0.0));
-                } else {
-                    o[0] = make_double2(v[0], v[1]);
-                    o[1] = make_double2(v[2], POT ? v[3] : 0.0);
-                }
-            }
-        }
-        __syncwarp();
-    }
-}
-
 // acc[orig] = G (far + near), pot[orig] = -G (far + near) (AdaptiveFMM3D.hpp:104)
 // far = far_l (L2P) + far_m (M2P) when the two parts ran apart (far_m non-null)
 template <bool POT>
@@ -908,79 +640,6 @@ __global__ void k_combine(int n, const int* __restrict__ perm, double G, const d
     acc[3 * (size_t)o + 1] = G * (f0.y + n0.y);
     acc[3 * (size_t)o + 2] = G * (f1.x + n1.x);
     if (POT) pot[o] = -G * (f1.y + n1.y);
-}
-
-// ---- P2L over X lists in FP32 (p <= 9) ------------------------------------------------
-// L_b += sum over the X-list leaves c of b, bodies j of c: q_j S_n^m(x_j - c_b)
-// (AdaptiveFMM3D::p2lAccum, src3d/AdaptiveFMM3D.hpp:117-128, scaled by side^n).
-// Warp per box (one warp per block).  The bodies of all X-list leaves form one
-// flat sequence; lane l takes positions l, l + 32, ... walking the entries on its
-// own, so every lane evaluates a body each round however the leaves are sized.
-// Each lane sums its K coefficients in registers (FP32); the 32 lane sums are
-// added once per box through shared memory in FP64.
-template <int P>
-struct P2L32 {
-    static constexpr int K = (P + 1) * (P + 1);
-    static constexpr bool OK = K <= 100;   // register budget of the per-lane sums
-};
-
-template <int P>
-__global__ void __launch_bounds__(32, 16) k_p2l32(TreeView tv, double* __restrict__ lown) {
-    constexpr int K = (P + 1) * (P + 1);
-    constexpr int LD = K | 1;
-    constexpr int NPL = (K + 31) / 32;
-    __shared__ float s_red[32 * LD];
-    const int lane = threadIdx.x;
-    const int b = blockIdx.x;
-    if (b >= tv_nb(tv) || tv_over(tv)) return;
-    const int64_t e0 = tv.x_off[b], e1 = tv.x_off[b + 1];
-    if (e0 == e1) return;
-    const double cx = tv.center[4 * b], cy = tv.center[4 * b + 1], cz = tv.center[4 * b + 2];
-    const double inv = 1.0 / (2.0 * tv.center[4 * b + 3]);
-    float acc[K];
-#pragma unroll
-    for (int d = 0; d < K; ++d) acc[d] = 0.f;
-    int64_t e = e0;
-    int c = tv.x_idx[e];
-    int f0 = tv.pfirst[c], cnt = tv.pcount[c];
-    int j = lane;
-    for (;;) {
-        while (e < e1 && j >= cnt) {
-            j -= cnt;
-            if (++e < e1) {
-                c = tv.x_idx[e];
-                f0 = tv.pfirst[c];
-                cnt = tv.pcount[c];
-            }
-        }
-        const bool act = e < e1;
-        if (!__any_sync(0xffffffffu, act)) break;
-        if (act) {
-            const int i = f0 + j;
-            const float q = (float)tv.pm[i];
-            const float ux = (float)((tv.px[i] - cx) * inv), uy = (float)((tv.py[i] - cy) * inv),
-                        uz = (float)((tv.pz[i] - cz) * inv);
-            for_singular<P>(ux, uy, uz, [&](int n, int m, float re, float im) {
-                const int dr = dof_re(n, m);
-                acc[dr] = fmaf(q, re, acc[dr]);
-                if (m > 0) acc[dr + 1] = fmaf(-q, im, acc[dr + 1]);
-            });
-        }
-        j += 32;
-    }
-#pragma unroll
-    for (int d = 0; d < K; ++d) s_red[lane * LD + d] = acc[d];
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < NPL; ++q) {
-        const int d = lane + 32 * q;
-        if (d < K) {
-            double sum = 0.0;
-#pragma unroll 8
-            for (int r = 0; r < 32; ++r) sum += (double)s_red[r * LD + d];
-            lown[(size_t)b * K + d] += sum * inv;
-        }
-    }
 }
 
 }  // namespace mixed

@@ -308,14 +308,23 @@ __global__ void k_leafkey(const uint32_t* perm_key, const int64_t* leafscan, int
     leafkey[perm_key[i]] = (uint32_t)(leafscan[i + 1] - 1);  // leaf id containing sorted position i
     ident[i] = (uint32_t)i;
 }
+// rhi, rlo (mixed form): position relative to the root centre as hi + lo FP32 (hi =
+// fp32(x - c), lo = fp32((x - c) - hi), the difference taken in FP64), mass in rhi.w
 __global__ void k_gather_bodies(const uint32_t* perm, const double* pos, const double* mass, int64_t n, int* perm_out,
-                                double* px, double* py, double* pz, double* pm) {
+                                double* px, double* py, double* pz, double* pm, const RootInfo* root, float4* rhi, float4* rlo) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t j = perm[i];
     perm_out[i] = (int)j;
-    px[i] = pos[3 * j]; py[i] = pos[3 * j + 1]; pz[i] = pos[3 * j + 2];
-    pm[i] = mass[j];
+    const double x = pos[3 * j], y = pos[3 * j + 1], z = pos[3 * j + 2], m = mass[j];
+    px[i] = x; py[i] = y; pz[i] = z;
+    pm[i] = m;
+    if (rhi) {
+        const double ex = x - root->c[0], ey = y - root->c[1], ez = z - root->c[2];
+        const float hx = (float)ex, hy = (float)ey, hz = (float)ez;
+        rhi[i] = make_float4(hx, hy, hz, (float)m);
+        rlo[i] = make_float4((float)(ex - (double)hx), (float)(ey - (double)hy), (float)(ez - (double)hz), 0.f);
+    }
 }
 
 }  // namespace
@@ -524,11 +533,15 @@ int tree_build(Handle& h, const double* d_pos, const double* d_mass, int64_t n) 
         OGX_CUDA(cudaStreamWaitEvent(st, h.ev_mass, 0));
         h.mass_pending = false;
     }
-    k_gather_bodies<<<grid_for(n, 256), 256, 0, st>>>(perm_s, d_pos, d_mass, n, perm, px, py, pz, pm); ++h.launches;
+    float4* rel = nullptr;
+    if (h.prm.precision == OGX_PREC_MIXED) OGX_TRY(arena_get(h.ws, S_MIX_POS4, 2 * n, &rel));
+    k_gather_bodies<<<grid_for(n, 256), 256, 0, st>>>(perm_s, d_pos, d_mass, n, perm, px, py, pz, pm, root, rel,
+                                                      rel ? rel + n : nullptr); ++h.launches;
     OGX_CUDA(cudaGetLastError());
 
     TreeView& tv = h.tv;
     tv.n = (int)n; tv.nb = nb; tv.nleaf = nleaf; tv.root = root; tv.cnt = dc;
+    tv.rhi = rel; tv.rlo = rel ? rel + n : nullptr;
     tv.px = px; tv.py = py; tv.pz = pz; tv.pm = pm; tv.perm = perm;
     tv.level = level; tv.coord = coord; tv.center = center; tv.parent = parent; tv.child = child;
     tv.leafid = leafid; tv.pfirst = pfirst; tv.pcount = pcount; tv.leafbox = leafbox;
