@@ -251,6 +251,7 @@ static int eval_device_on(Handle& h, int64_t n, const double* d_pos, const doubl
     if (!h.cap_mode) update_capacity(h);
     if (h.prm.precision == OGX_PREC_MIXED) OGX_TRY(fmm_mixed(h, d_acc, d_pot));
     else OGX_TRY(fmm_fp64(h, d_acc, d_pot));   // the plain form, or with rotation-based M2L
+    OGX_CUDA(cudaStreamWaitEvent(st, h.ev_check, 0));   // the adjacency check's counts
     // every count of this evaluation (the overflow flag included) reaches the host with it,
     // and so does the error word of its bounded waits (tensor-core M2L, translation passes)
     OGX_CUDA(cudaMemcpyAsync(h.h_counts, h.d_counts, sizeof(DevCounts), cudaMemcpyDeviceToHost, st));
@@ -664,6 +665,7 @@ int ogx_create(const ogx_params* prm, void** handle) {
     OGX_CUDA(cudaStreamCreateWithPriority(&h->m2l, cudaStreamNonBlocking, prio_mid));
     OGX_CUDA(cudaEventCreateWithFlags(&h->ev_col, cudaEventDisableTiming));
     OGX_CUDA(cudaEventCreateWithFlags(&h->ev_tgt, cudaEventDisableTiming));
+    OGX_CUDA(cudaEventCreateWithFlags(&h->ev_check, cudaEventDisableTiming));
     OGX_CUDA(cudaEventCreateWithFlags(&h->ev_m2l, cudaEventDisableTiming));
     OGX_CUDA(cudaEventCreateWithFlags(&h->ev_mass, cudaEventDisableTiming));
     OGX_CUDA(cudaEventCreateWithFlags(&h->ev_pos, cudaEventDisableTiming));
@@ -687,7 +689,7 @@ int ogx_destroy(void* handle) {
         if (h->h_stage) cudaFreeHost(h->h_stage);
         for (auto& e : h->ev)
             if (e) cudaEventDestroy(e);
-        for (cudaEvent_t e : {h->ev_col, h->ev_tgt, h->ev_m2l, h->ev_mass, h->ev_pos})
+        for (cudaEvent_t e : {h->ev_col, h->ev_tgt, h->ev_m2l, h->ev_check, h->ev_mass, h->ev_pos})
             if (e) cudaEventDestroy(e);
         for (cudaStream_t sx : {h->main, h->side, h->up, h->aux, h->m2l})
             if (sx) {

@@ -166,7 +166,6 @@ int near_items(Handle& h, int64_t** chunk_off) {
     int* nchunk;
     OGX_TRY(arena_get(h.ws, S_NEAR_CHUNK, (size_t)tv.nleaf, &nchunk));
     OGX_TRY(arena_get(h.ws, S_NEAR_CHUNK_OFF, (size_t)tv.nleaf + 1, chunk_off));
-    near_field::k_near_chunks<<<(tv.nleaf + 255) / 256, 256, 0, h.stream>>>(tv, nchunk); ++h.launches;
     return scan_i32_to_i64(h, nchunk, *chunk_off, tv.nleaf);
 }
 
@@ -388,11 +387,17 @@ int run_mixed_m2l(Handle& h, bool pot) {
     if (h.ntgt > 0) {
         static_assert(C::SUPPORTED, "every order's operand fits TMEM, in slices if need be");
         OGX_CUDA(smem_optin((const void*)mixed::k_m2l_tc<P>, C::SMEM));
-        mixed::k_m2l_tc<P><<<dim3(h.ntgt_pad / 128, C::NSPLIT), C::THREADS, C::SMEM, sm>>>(
-            tv, h.tgt_tile_key, h.tgt_tile_box, mhi, mlo, mus, h.d_tc_img, h.d_tc_ounscale, Lown, h.d_err); ++h.launches;
+        M2L64Args a;
+        OGX_TRY(m2l64_args(h, C::NSPLIT, &a));
+        const int tiles = h.ntgt_pad / 128;
+        // ranges of slots per tile, one CTA each (the kernel's own count is exact; this one
+        // comes from a bound and may differ)
+        const int ranges = m2l_tc_split((h.ntgt + 127) / 128, C::NSPLIT);
+        mixed::k_m2l_tc<P><<<dim3(tiles, C::NSPLIT, ranges), C::THREADS, C::SMEM, sm>>>(tv, a, mhi, mlo, mus, h.d_tc_img,
+                                                                                       h.d_tc_ounscale, Lown, h.d_err); ++h.launches;
+        OGX_TRY(m2l64_sum_launch(h, a, C::NSPLIT, Lown, sm));
         if (pot) {
-            mixed::k_m2l_dof0<P><<<(h.ntgt_pad + 127) / 128, 128, 0, sm>>>(tv, h.ntgt_pad, h.tgt_tile_key, h.tgt_tile_box,
-                                                                         h.d_tc_row0, M, Lown); ++h.launches;
+            mixed::k_m2l_dof0<P><<<(h.ntgt + 3) / 4, 128, 0, sm>>>(tv, h.ntgt, h.tgt_box, h.d_tc_row0, M, Lown); ++h.launches;
         }
     }
     OGX_CUDA(timing_record(h, h.ev[4], sm));

@@ -156,7 +156,6 @@ struct DevCounts {
     int64_t v_total;
     int32_t kernel_error;  // set by kernels whose bounded waits ran out
     int32_t pad_err;       // zero: the bounded-wait probe's flag that nothing sets
-    int32_t nonleaf_level[kMaxDepth + 2];
     int32_t deep_flag;   // some level-16 box holds more than leaf_capacity bodies
     int32_t overflow;    // capacity mode: a count above its capacity (see above)
     int32_t nb32, nleaf32;   // num_boxes, num_leaves
@@ -246,7 +245,7 @@ struct Handle {
     // mixed form: the tensor-core M2L (middle priority), launched once the multipoles and
     // target tiles are ready, beside the rest of the list build
     cudaStream_t m2l = nullptr;
-    cudaEvent_t ev_col = nullptr, ev_tgt = nullptr, ev_m2l = nullptr;
+    cudaEvent_t ev_col = nullptr, ev_tgt = nullptr, ev_m2l = nullptr, ev_check = nullptr;
     // host-buffer evaluation: the masses' copy runs on `aux` beside the start of the tree
     // build, which waits for it (ev_mass) before the sorted-body gather
     cudaEvent_t ev_mass = nullptr, ev_pos = nullptr;

@@ -5,10 +5,9 @@
 //    colleagues that pass `adjacent` (:143-151).  Box centres are exact binary
 //    fractions of the root box, so for same-level boxes that test holds exactly
 //    for integer offsets in [-1,1]^3: every (box, slot) finds its colleague in
-//    one launch by a binary search of the level's boxes (Morton order) for the
-//    offset coordinates.  A second launch replays the reference's recursion over
+//    one launch through the tree's pointers.  A second launch replays the reference's recursion over
 //    the children of each parent's colleagues with the FP64 predicate and counts
-//    every disagreement with the search (expected 0);
+//    every disagreement (expected 0);
 //  - V is implicit: children of the parent's colleagues at integer offset
 //    max|o| >= 2 (:154-161); every candidate is also classified with the
 //    reference's FP64 predicate and disagreements are counted (expected 0);
@@ -31,25 +30,13 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int UW_STACK = 192;
 
-// p's highest set bit is below q's
-__device__ __forceinline__ bool msb_less(unsigned p, unsigned q) { return p < q && p < (p ^ q); }
-
-// Morton order of two boxes of one level from their integer coordinates: the
-// dimension whose coordinates first differ at the highest bit decides; at equal
-// bits z ranks above y above x (octant digit = x | y << 1 | z << 2)
-__device__ __forceinline__ bool morton_less(int ax, int ay, int az, int bx, int by, int bz) {
-    const unsigned x = (unsigned)(ax ^ bx), y = (unsigned)(ay ^ by), z = (unsigned)(az ^ bz);
-    int d = 2;
-    unsigned m = z;
-    if (msb_less(m, y)) { d = 1; m = y; }
-    if (msb_less(m, x)) d = 0;
-    return d == 0 ? ax < bx : (d == 1 ? ay < by : az < bz);
-}
-
-// colleague slot d of box b: the box of b's level at integer offset (d % 3 - 1, ...);
-// level_off[l] = first box of level l (device)
-__global__ void k_colleagues_bs(int nb_cap, const int* __restrict__ level_off, const int* __restrict__ level,
-                                const int* __restrict__ coord, int* __restrict__ col, const DevCounts* counts) {
+// colleague slot d of box b: the box of b's level at integer offset (d % 3 - 1, ...), found by
+// climbing to the first ancestor that contains both and descending by the other's octants
+// (two or three steps each way on average; a binary search of the level took a dozen steps
+// of three loads: 47 -> 20 us on the 1M merger)
+__global__ void k_colleagues(int nb_cap, const int* __restrict__ level, const int* __restrict__ coord,
+                             const int* __restrict__ parent, const int* __restrict__ child, int* __restrict__ col,
+                             const DevCounts* counts) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= 27 * (int64_t)nb_cap || counts->overflow) return;
     const int b = (int)(t / 27), d = (int)(t - 27 * (int64_t)b);
@@ -57,17 +44,15 @@ __global__ void k_colleagues_bs(int nb_cap, const int* __restrict__ level_off, c
     if (d == 13) { col[t] = b; return; }
     const int l = level[b];
     const int side = 1 << l;
-    const int nx = coord[3 * b] + d % 3 - 1, ny = coord[3 * b + 1] + (d / 3) % 3 - 1, nz = coord[3 * b + 2] + d / 9 - 1;
+    const int x = coord[3 * b], y = coord[3 * b + 1], z = coord[3 * b + 2];
+    const int nx = x + d % 3 - 1, ny = y + (d / 3) % 3 - 1, nz = z + d / 9 - 1;
     int found = -1;
-    if (l > 0 && nx >= 0 && ny >= 0 && nz >= 0 && nx < side && ny < side && nz < side) {
-        int lo = level_off[l], hi = level_off[l + 1] - 1;
-        while (lo <= hi) {
-            const int mid = (lo + hi) >> 1;
-            const int mx = coord[3 * mid], my = coord[3 * mid + 1], mz = coord[3 * mid + 2];
-            if (mx == nx && my == ny && mz == nz) { found = mid; break; }
-            if (morton_less(mx, my, mz, nx, ny, nz)) lo = mid + 1;
-            else hi = mid - 1;
-        }
+    if (nx >= 0 && ny >= 0 && nz >= 0 && nx < side && ny < side && nz < side) {
+        const int up = 32 - __clz((x ^ nx) | (y ^ ny) | (z ^ nz));   // levels to the common ancestor
+        found = b;
+        for (int i = 0; i < up; ++i) found = parent[found];
+        for (int i = up - 1; i >= 0 && found >= 0; --i)
+            found = child[8 * (size_t)found + (((nx >> i) & 1) | (((ny >> i) & 1) << 1) | (((nz >> i) & 1) << 2))];
     }
     col[t] = found;
 }
@@ -143,13 +128,17 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane) {
     return x - v;
 }
 
+// A node's descent step takes two rounds of loads: its children and centre, then the leaf
+// ids of the adjacent children (a child's centre is its parent's shifted by half the child's
+// edge, the operation k_boxes formed it with); one child after another, with its centre
+// loaded, took some twenty.  FILL also emits the transposed W pairs (X lists) and counts them.
 template <bool FILL>
 __global__ void __launch_bounds__(128) k_uw_warp(int nleaf, const int* __restrict__ leafbox, const int* __restrict__ parent,
                                                  const int* __restrict__ child, const int* __restrict__ leafid,
                                                  const int* __restrict__ col, const double* __restrict__ ctr,
                                                  const int* __restrict__ pcount, const RootInfo* root, int* lane_u, int* lane_w,
                                                  int* ucnt, int* wcnt, const int64_t* uoff, const int64_t* woff, int* uidx,
-                                                 int* widx, DevCounts* counts) {
+                                                 int* widx, uint32_t* xkey, uint32_t* xval, int* xcnt, DevCounts* counts) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int lf = blockIdx.x * 4 + wid;
     if (lf >= nleaf || lf >= counts->nleaf32 || counts->overflow) return;
@@ -157,10 +146,13 @@ __global__ void __launch_bounds__(128) k_uw_warp(int nleaf, const int* __restric
     const double tol = root->tol;
     // adjacent64(ctr, a, b, tol) with b's centre held in registers
     const double bx = ctr[4 * b], by = ctr[4 * b + 1], bz = ctr[4 * b + 2], bh = ctr[4 * b + 3];
-    auto adj_b = [&](int a) {
-        const double lim = __dadd_rn(__dadd_rn(ctr[4 * a + 3], bh), tol);
-        return fabs(__dsub_rn(ctr[4 * a], bx)) <= lim && fabs(__dsub_rn(ctr[4 * a + 1], by)) <= lim &&
-               fabs(__dsub_rn(ctr[4 * a + 2], bz)) <= lim;
+    auto adj = [&](double x, double y, double z, double h) {
+        const double lim = __dadd_rn(__dadd_rn(h, bh), tol);
+        return fabs(__dsub_rn(x, bx)) <= lim && fabs(__dsub_rn(y, by)) <= lim && fabs(__dsub_rn(z, bz)) <= lim;
+    };
+    auto centre = [&](int a, double2& c01, double2& c23) {
+        c01 = __ldg(reinterpret_cast<const double2*>(ctr) + 2 * (size_t)a);
+        c23 = __ldg(reinterpret_cast<const double2*>(ctr) + 2 * (size_t)a + 1);
     };
     int nu = 0, nw = 0;
     int64_t upairs = 0, ub = 0, wb = 0;
@@ -176,28 +168,56 @@ __global__ void __launch_bounds__(128) k_uw_warp(int nleaf, const int* __restric
     };
     if (lane < 27) {
         const int d = lane;
-        const int c = col[27 * b + d];
-        if (c >= 0 && leafid[c] >= 0) addU(c);  // same-level adjacent leaves (b itself in slot 13)
-        for (int A = parent[b]; A >= 0; A = parent[A]) {  // coarser adjacent leaves
-            const int a2 = col[27 * A + d];
-            if (a2 >= 0 && leafid[a2] >= 0 && adj_b(a2)) addU(a2);
+        const int c = col[27 * (size_t)b + d];
+        const int lc = c >= 0 ? leafid[c] : -1;
+        if (c >= 0 && lc >= 0) addU(c);  // same-level adjacent leaves (b itself in slot 13)
+        for (int A = parent[b]; A >= 0;) {  // coarser adjacent leaves
+            const int up = parent[A], a2 = col[27 * (size_t)A + d];
+            if (a2 >= 0 && leafid[a2] >= 0) {
+                double2 c01, c23;
+                centre(a2, c01, c23);
+                if (adj(c01.x, c01.y, c23.x, c23.y)) addU(a2);
+            }
+            A = up;
         }
-        if (c >= 0 && c != b && leafid[c] < 0) {  // finer: descend the non-leaf colleague
+        if (c >= 0 && c != b && lc < 0) {  // finer: descend the non-leaf colleague
             int stk[UW_STACK];
             int sp = 0;
             stk[sp++] = c;
             while (sp > 0) {
                 const int node = stk[--sp];
+                const int4 k0 = __ldg(reinterpret_cast<const int4*>(child + 8 * (size_t)node));
+                const int4 k1 = __ldg(reinterpret_cast<const int4*>(child + 8 * (size_t)node) + 1);
+                double2 c01, c23;
+                centre(node, c01, c23);
+                const int ch[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+                const double h2 = __dmul_rn(0.5, c23.y);
+                // per axis: the lower and the upper child's coordinate (k_boxes' operations)
+                const double xs[2] = {__dadd_rn(c01.x, -h2), __dadd_rn(c01.x, h2)}, ys[2] = {__dadd_rn(c01.y, -h2), __dadd_rn(c01.y, h2)},
+                             zs[2] = {__dadd_rn(c23.x, -h2), __dadd_rn(c23.x, h2)};
+                int leaf[8];
+                unsigned near = 0;
+#pragma unroll
                 for (int s = 0; s < 8; ++s) {
-                    const int ch = child[8 * node + s];
-                    if (ch < 0) continue;
-                    if (!adj_b(ch)) {
-                        if (FILL) widx[wb + nw] = ch;
+                    const bool a = ch[s] >= 0 && adj(xs[s & 1], ys[(s >> 1) & 1], zs[s >> 2], h2);
+                    leaf[s] = a ? __ldg(leafid + ch[s]) : -1;
+                    if (a) near |= 1u << s;
+                }
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    if (ch[s] < 0) continue;
+                    if (!(near >> s & 1u)) {
+                        if (FILL) {
+                            widx[wb + nw] = ch[s];
+                            xkey[wb + nw] = (uint32_t)ch[s];
+                            xval[wb + nw] = (uint32_t)b;
+                            atomicAdd(&xcnt[ch[s]], 1);
+                        }
                         ++nw;
-                    } else if (leafid[ch] >= 0) {
-                        addU(ch);
+                    } else if (leaf[s] >= 0) {
+                        addU(ch[s]);
                     } else if (sp < UW_STACK) {
-                        stk[sp++] = ch;
+                        stk[sp++] = ch[s];
                     } else {
                         overflow = true;
                     }
@@ -229,19 +249,6 @@ __global__ void __launch_bounds__(128) k_uw_warp(int nleaf, const int* __restric
     }
 }
 
-// X = transpose of W: emit (w, leaf box) in leaf order, count members per box
-__global__ void k_x_emit(int nleaf, const int* leafbox, const int64_t* woff, const int* widx, uint32_t* xkey, uint32_t* xval,
-                         int* xcnt, const DevCounts* counts) {
-    const int lf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lf >= nleaf || lf >= counts->nleaf32 || counts->overflow) return;
-    const int b = leafbox[lf];
-    for (int64_t e = woff[lf]; e < woff[lf + 1]; ++e) {
-        xkey[e] = (uint32_t)widx[e];
-        xval[e] = (uint32_t)b;
-        atomicAdd(&xcnt[widx[e]], 1);
-    }
-}
-
 // M2L targets: boxes of level >= 2 keyed by their child octant
 // Sort key of an M2L target: its octant t inside the parent (bits 27-29; a tensor-core
 // tile holds targets of one octant) and, below it, which of the parent's 27 colleague
@@ -251,36 +258,42 @@ __global__ void k_x_emit(int nleaf, const int* leafbox, const int64_t* woff, con
 // order of a tile's targets does not change any target's result.
 // Launched over the capacity of boxes: the targets are boxes level_off[2] .. nb - 1
 // (device counts); slots behind them get key 1 << 30 and sort after every target.
-__global__ void k_tgt_keys(int cap, const int* __restrict__ level_off, const int* __restrict__ coord,
-                           const int* __restrict__ parent, const int* __restrict__ col, const int* __restrict__ child,
-                           uint32_t* key, uint32_t* val, DevCounts* counts) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Warp per target, lane = colleague slot.
+__global__ void __launch_bounds__(128) k_tgt_keys(int cap, const int* __restrict__ level_off, const int* __restrict__ coord,
+                                                  const int* __restrict__ parent, const int* __restrict__ col,
+                                                  const int* __restrict__ child, uint32_t* key, uint32_t* val, DevCounts* counts) {
+    const int lane = threadIdx.x & 31;
+    const int k = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (k >= cap || counts->overflow) return;
     const int first = level_off[2], ntgt = counts->nb32 - first;
-    if (k == 0) counts->ntgt32 = ntgt;
+    if (k == 0 && lane == 0) counts->ntgt32 = ntgt;
     if (k >= ntgt) {
-        key[k] = 1u << 30;
-        val[k] = 0xFFFFFFFFu;
+        if (lane == 0) {
+            key[k] = 1u << 30;
+            val[k] = 0xFFFFFFFFu;
+        }
         return;
     }
     const int b = first + k;
     const int tx = coord[3 * b] & 1, ty = coord[3 * b + 1] & 1, tz = coord[3 * b + 2] & 1;
-    const int par = parent[b];
-    uint32_t mask = 0;
-    for (int D = 0; D < 27; ++D) {
-        const int Q = col[27 * par + D];
-        if (Q < 0) continue;
-        const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
+    const int Q = lane < 27 ? col[27 * (size_t)parent[b] + lane] : -1;
+    bool any = false;
+    if (Q >= 0) {
+        const int4 c0 = __ldg(reinterpret_cast<const int4*>(child + 8 * (size_t)Q));
+        const int4 c1 = __ldg(reinterpret_cast<const int4*>(child + 8 * (size_t)Q) + 1);
+        const int ch[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const int Dx = lane % 3 - 1, Dy = (lane / 3) % 3 - 1, Dz = lane / 9 - 1;
+#pragma unroll
         for (int s = 0; s < 8; ++s) {
             const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
-            if (max(abs(ox), max(abs(oy), abs(oz))) > 1 && child[8 * Q + s] >= 0) {
-                mask |= 1u << (26 - D);
-                break;
-            }
+            any |= ch[s] >= 0 && max(abs(ox), max(abs(oy), abs(oz))) > 1;
         }
     }
-    key[k] = ((uint32_t)(tx | (ty << 1) | (tz << 2)) << 27) | mask;
-    val[k] = (uint32_t)b;
+    const unsigned slots = __ballot_sync(FULL, any);   // bit D
+    if (lane == 0) {
+        key[k] = ((uint32_t)(tx | (ty << 1) | (tz << 2)) << 27) | (__brev(slots) >> 5);   // slot D in bit 26 - D
+        val[k] = (uint32_t)b;
+    }
 }
 
 // padded per-octant layout of the M2L targets (sorted by k_tgt_keys' key, octant in
@@ -289,26 +302,37 @@ __global__ void k_tgt_keys(int cap, const int* __restrict__ level_off, const int
 // gs[9..17] = padded group starts, then the FP64 M2L's work split (ogx_m2l64.cuh).
 __global__ void k_target_groups(const uint32_t* key, const DevCounts* counts, int tile, int fill, int* gs) {
     __shared__ int lo_s[9];
-    const int g = threadIdx.x;
+    const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntgt = counts->overflow ? 0 : counts->ntgt32;
-    if (g <= 8) {
-        int lo = 0, hi = ntgt;  // first index with key >= g
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if ((int)(key[mid] >> 27) < g) lo = mid + 1; else hi = mid;
+    if (g <= 8) {   // warp g: the first index with key octant >= g, 32 probes at a time
+        int lo = 0, hi = ntgt;
+        while (hi > lo) {
+            const int step = (hi - lo + 31) / 32, i = lo + lane * step;
+            const bool below = i < hi && (int)(key[i] >> 27) < g;
+            const int c = __popc(__ballot_sync(FULL, below));   // probes below: a prefix
+            if (c == 0) { hi = lo; break; }
+            const int last = lo + (c - 1) * step;
+            hi = min(hi, last + step);
+            lo = last + 1;
         }
-        lo_s[g] = lo;
-        gs[g] = lo;
+        if (lane == 0) {
+            lo_s[g] = lo;
+            gs[g] = lo;
+        }
     }
     __syncthreads();
-    if (g == 0) {
+    if (threadIdx.x == 0) {
         int pad = 0;
         for (int q = 0; q <= 8; ++q) {
             gs[9 + q] = pad;
             if (q < 8) pad += ((lo_s[q + 1] - lo_s[q] + fill - 1) / fill) * tile;
         }
-        int tiles64 = 0;
-        for (int q = 0; q < 8; ++q) tiles64 += (lo_s[q + 1] - lo_s[q] + M2L64_TGT - 1) / M2L64_TGT;
+        int tiles64 = 0, tiles128 = 0;
+        for (int q = 0; q < 8; ++q) {
+            tiles64 += (lo_s[q + 1] - lo_s[q] + M2L64_TGT - 1) / M2L64_TGT;
+            tiles128 += (lo_s[q + 1] - lo_s[q] + 127) / 128;
+        }
+        gs[GS_TILES128] = tiles128;
         gs[GS_SPLIT] = max(1, min(M2L64_MAXSPLIT, (M2L64_ITEMS + tiles64 - 1) / max(tiles64, 1)));
         gs[GS_TILES] = pad / M2L64_TGT;
         gs[GS_TICKET] = 0;
@@ -451,8 +475,7 @@ int lists_build_targets(Handle& h) {
     DevCounts* dc = h.d_counts;
     int* col;
     OGX_TRY(arena_get(h.ws, S_BOX_COL, 27 * (size_t)nb, &col));
-    k_colleagues_bs<<<grid_for(27 * (int64_t)nb, 256), 256, 0, st>>>(nb, h.d_level_off, tv.level, tv.coord, col, dc); ++h.launches;
-    k_colleagues_check<<<grid_for(nb, 4), 128, 0, st>>>(0, nb, tv.leafid, tv.child, tv.center, tv.root, col, dc); ++h.launches;
+    k_colleagues<<<grid_for(27 * (int64_t)nb, 256), 256, 0, st>>>(nb, tv.level, tv.coord, tv.parent, tv.child, col, dc); ++h.launches;
     tv.col = col;
 
     // M2L targets (levels >= 2) grouped by child octant, then by the slot pattern of
@@ -461,13 +484,18 @@ int lists_build_targets(Handle& h) {
     // (which use the scan scratch, not the radix-sort scratch); the main stream joins
     // before the X-list sort, which uses the radix-sort scratch again.
     OGX_CUDA(cudaEventRecord(h.ev_col, st));
+    // nothing of the evaluation waits for the check and the V-pair count: on the side stream
+    // (joined at the evaluation's end)
+    OGX_CUDA(cudaStreamWaitEvent(h.side, h.ev_col, 0));
+    k_colleagues_check<<<grid_for(nb, 4), 128, 0, h.side>>>(0, nb, tv.leafid, tv.child, tv.center, tv.root, col, dc); ++h.launches;
+    OGX_CUDA(cudaEventRecord(h.ev_check, h.side));
     OGX_CUDA(cudaStreamWaitEvent(h.aux, h.ev_col, 0));
     h.stream = h.aux;   // radix_sort_u32 issues on h.stream
     const int tcap = std::max(nb, 1);
     uint32_t *tk, *tb;
     OGX_TRY(arena_get(h.ws, S_TGT_KEY, tcap + 1, &tk));
     OGX_TRY(arena_get(h.ws, S_TGT_BOX, tcap + 1, &tb));
-    k_tgt_keys<<<grid_for(tcap, 256), 256, 0, h.aux>>>(tcap, h.d_level_off, tv.coord, tv.parent, col, tv.child, tk, tb, dc); ++h.launches;
+    k_tgt_keys<<<grid_for(tcap, 4), 128, 0, h.aux>>>(tcap, h.d_level_off, tv.coord, tv.parent, col, tv.child, tk, tb, dc); ++h.launches;
     uint32_t *tk_s, *tb_s;
     const int rc_t = radix_sort_u32(h, S_TGT_KEY, S_TGT_BOX, S_TGT_KEY2, S_TGT_BOX2, tcap, 31, &tk_s, &tb_s);
     h.stream = st;
@@ -483,7 +511,7 @@ int lists_build_targets(Handle& h) {
     OGX_TRY(arena_get(h.ws, S_TGT_TILE, 32, &gs));
     OGX_TRY(arena_get(h.ws, S_TGT_PKEY, npad, &pk));
     OGX_TRY(arena_get(h.ws, S_TGT_PBOX, npad, &pb));
-    k_target_groups<<<1, 32, 0, h.aux>>>(tk_s, dc, tile, fill, gs); ++h.launches;
+    k_target_groups<<<1, 288, 0, h.aux>>>(tk_s, dc, tile, fill, gs); ++h.launches;
     k_target_pad<<<grid_for(npad, 256), 256, 0, h.aux>>>(tb_s, gs, npad, tile, fill, pk, pb); ++h.launches;
     h.tgt_groups = gs;
     h.tgt_tile_key = pk;
@@ -516,7 +544,7 @@ int lists_build_uwx(Handle& h) {
     int* lane_w = lane_uw + 32 * (size_t)nleaf;
     k_uw_warp<false><<<grid_for(nleaf, 4), 128, 0, st>>>(nleaf, tv.leafbox, tv.parent, tv.child, tv.leafid, col, tv.center,
                                                          tv.pcount, tv.root, lane_u, lane_w, ucnt, wcnt, nullptr, nullptr,
-                                                         nullptr, nullptr, dc); ++h.launches;
+                                                         nullptr, nullptr, nullptr, nullptr, nullptr, dc); ++h.launches;
     OGX_TRY(scan2_i32_to_i64(h, ucnt, uoff, wcnt, woff, nleaf));
     int64_t nu, nw;
     if (h.cap_mode) {
@@ -534,12 +562,6 @@ int lists_build_uwx(Handle& h) {
     int *uidx, *widx;
     OGX_TRY(arena_get(h.ws, S_U_IDX, nu + 1, &uidx));
     OGX_TRY(arena_get(h.ws, S_W_IDX, nw + 1, &widx));
-    k_uw_warp<true><<<grid_for(nleaf, 4), 128, 0, st>>>(nleaf, tv.leafbox, tv.parent, tv.child, tv.leafid, col, tv.center,
-                                                        tv.pcount, tv.root, lane_u, lane_w, nullptr, nullptr, uoff, woff, uidx,
-                                                        widx, dc); ++h.launches;
-    tv.u_off = uoff; tv.w_off = woff; tv.u_idx = uidx; tv.w_idx = widx;
-
-    OGX_CUDA(cudaStreamWaitEvent(st, h.ev_tgt, 0));   // target sort done with the radix scratch
     // X lists: W transposed by a stable sort on the W member; keys behind the W total
     // (capacity padding) sort last and are never referenced by x_off
     const int xbits = bits_for(nb);
@@ -551,7 +573,11 @@ int lists_build_uwx(Handle& h) {
     OGX_TRY(arena_get(h.ws, S_X_CNT, nb, &xcnt));
     OGX_TRY(arena_get(h.ws, S_X_OFF, nb + 1, &xoff));
     OGX_CUDA(cudaMemsetAsync(xcnt, 0, sizeof(int) * (size_t)nb, st));
-    k_x_emit<<<grid_for(nleaf, 128), 128, 0, st>>>(nleaf, tv.leafbox, woff, widx, xk, xv, xcnt, dc); ++h.launches;
+    k_uw_warp<true><<<grid_for(nleaf, 4), 128, 0, st>>>(nleaf, tv.leafbox, tv.parent, tv.child, tv.leafid, col, tv.center,
+                                                        tv.pcount, tv.root, lane_u, lane_w, nullptr, nullptr, uoff, woff, uidx,
+                                                        widx, xk, xv, xcnt, dc); ++h.launches;
+    tv.u_off = uoff; tv.w_off = woff; tv.u_idx = uidx; tv.w_idx = widx;
+    OGX_CUDA(cudaStreamWaitEvent(st, h.ev_tgt, 0));   // target sort done with the radix scratch
     if (h.cap_mode) { k_fill_tail_x<<<grid_for(nw, 256), 256, 0, st>>>(xk, dc, nw, (1u << xbits) - 1u); ++h.launches; }
     uint32_t *xk_s, *xv_s;
     OGX_TRY(radix_sort_u32(h, S_X_KEY, S_X_VAL, S_X_KEY2, S_X_VAL2, nw, xbits, &xk_s, &xv_s));

@@ -226,13 +226,14 @@ __global__ void __launch_bounds__(M64<P>::THREADS, M64<P>::MINB)
 }
 
 // Lown of every target = its ranges' sums in range order / side (split above 1)
-__global__ void __launch_bounds__(256) k_m2l64_sum(TreeView tv, M2L64Args ar, int K, double* __restrict__ lown) {
-    const int S = ar.gs[GS_SPLIT];
+__global__ void __launch_bounds__(256) k_m2l64_sum(TreeView tv, M2L64Args ar, int K, int slices, double* __restrict__ lown) {
+    const int S = slices > 0 ? m2l_tc_split(ar.gs[GS_TILES128], slices) : ar.gs[GS_SPLIT];
     if (tv_over(tv) || S == 1) return;
     const int ntgt = tv.cnt->ntgt32;
     const int64_t total = (int64_t)ntgt * K;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int j = (int)(i / K), d = (int)(i - (int64_t)j * K);
+        if (slices > 0 && d == 0) continue;
         double v = 0.0;
 #pragma unroll 9
         for (int z = 0; z < S; ++z) v += ar.part[(size_t)z * total + i];
@@ -245,12 +246,12 @@ template <int P>
 int launch(Handle& h, const double* M, double* Lown) {
     using C = M64<P>;
     M2L64Args a;
-    OGX_TRY(m2l64_args(h, &a));
+    OGX_TRY(m2l64_args(h, 0, &a));
     OGX_CUDA(smem_optin((const void*)k_m2l_fp64<P>, C::SMEM));
     const int tiles = h.ntgt_pad / M2L64_TGT;
     const int grid = (int)std::min<int64_t>((int64_t)tiles * M2L64_MAXSPLIT, C::MINB * h.num_sms);
     k_m2l_fp64<P><<<grid, C::THREADS, C::SMEM, h.stream>>>(h.tv, a, h.d_m2l, M, Lown); ++h.launches;
-    return m2l64_sum_launch(h, a, Lown, h.stream);
+    return m2l64_sum_launch(h, a, 0, Lown, h.stream);
 }
 
 }  // namespace
@@ -258,18 +259,19 @@ int launch(Handle& h, const double* M, double* Lown) {
 int m2l64_pad_rows(int p) { return ((p + 1) * (p + 1) + 3) / 4 * 4; }
 int m2l64_pad_cols(int p) { return ((p + 1) * (p + 1) + 7) / 8 * 8 + 4; }
 
-int m2l64_args(Handle& h, M2L64Args* a) {
+int m2l64_args(Handle& h, int slices, M2L64Args* a) {
     a->tgt_key = h.tgt_tile_key;
     a->tgt_box = h.tgt_tile_box;
     a->sorted_box = h.tgt_box;
     a->gs = h.tgt_groups;
-    return arena_get(h.ws, S_M2L_PART, m2l64_partial_rows(h.ntgt) * num_dofs(h.prm.p), &a->part);
+    const size_t rows = slices > 0 ? m2l_tc_partial_rows(h.ntgt, slices) : m2l64_partial_rows(h.ntgt);
+    return arena_get(h.ws, S_M2L_PART, rows * num_dofs(h.prm.p), &a->part);
 }
 
-int m2l64_sum_launch(Handle& h, const M2L64Args& a, double* Lown, cudaStream_t st) {
+int m2l64_sum_launch(Handle& h, const M2L64Args& a, int slices, double* Lown, cudaStream_t st) {
     const int K = num_dofs(h.prm.p);
     const int grid = (int)std::min<int64_t>(((int64_t)h.ntgt * K + 255) / 256, 8 * h.num_sms);
-    k_m2l64_sum<<<grid, 256, 0, st>>>(h.tv, a, K, Lown); ++h.launches;
+    k_m2l64_sum<<<grid, 256, 0, st>>>(h.tv, a, K, slices, Lown); ++h.launches;
     OGX_CUDA(cudaGetLastError());
     return OGX_OK;
 }

@@ -15,7 +15,7 @@ constexpr int M2L64_TGT = 64;        // targets per tile; the target layout is p
 constexpr int M2L64_ITEMS = 1184;    // items wanted: 4 per CTA slot of 2 x 148
 constexpr int M2L64_MAXSPLIT = 27;
 // k_target_groups' words behind the group starts gs[0..17]
-constexpr int GS_SPLIT = 18, GS_TILES = 19, GS_TICKET = 20, GS_FILL = 21;
+constexpr int GS_SPLIT = 18, GS_TILES = 19, GS_TICKET = 20, GS_FILL = 21, GS_TILES128 = 22;
 
 // V children that slot D offers a target of octant t: the 8 children less the adjacent ones
 __host__ __device__ __forceinline__ int m2l64_slot_count(int D, int t) {
@@ -37,13 +37,40 @@ __host__ __device__ __forceinline__ int m2l64_first_slot(int z, int S, int t) {
     return D;
 }
 
-// partial rows (of K doubles) that S ranges of at most ntgt targets can need: S <= 27,
-// S < M2L64_ITEMS / tiles + 1, and S = 1 (no partial rows) from M2L64_ITEMS tiles on (a
-// capacity is at most twice the targets it was taken from)
+// partial rows (of K doubles) that any tree of at most ntgt targets can need (a captured
+// step's tree may be smaller than its capacity): S <= 27, S < M2L64_ITEMS / tiles + 1, and
+// S = 1 (none) from M2L64_ITEMS tiles on
 inline size_t m2l64_partial_rows(int64_t ntgt) {
-    if (ntgt >= 2ll * M2L64_TGT * M2L64_ITEMS) return 0;
-    const int64_t a = M2L64_MAXSPLIT * ntgt, b = (int64_t)M2L64_TGT * M2L64_ITEMS + ntgt;
+    const int64_t full = (int64_t)M2L64_TGT * M2L64_ITEMS;
+    const int64_t a = M2L64_MAXSPLIT * ntgt, b = full + (ntgt < full ? ntgt : full);
     return (size_t)(a < b ? a : b);
+}
+
+// Ranges of the tensor-core M2L for `tiles` 128-target tiles of `slices` column slices each
+// (one CTA per SM): the fewest waves of work, where a CTA costs 1 / S of a tile and 0.045 of
+// one for its set-up and partial sums (17,000 of 500,000 cycles at p = 8, and the rows).
+__host__ __device__ __forceinline__ int m2l_tc_split(int tiles, int slices) {
+    const int n = tiles * slices;
+    int best = 1;
+    float cost = 1e30f;
+    for (int s = 1; s <= M2L64_MAXSPLIT && (s == 1 || n * s <= 888); ++s) {
+        const float c = (float)((n * s + 147) / 148) * (1.0f / (float)s + 0.045f);
+        if (c < cost * 0.999f) { cost = c; best = s; }
+    }
+    return best;
+}
+// partial rows (of K doubles) that any tree of at most ntgt targets can need
+inline size_t m2l_tc_partial_rows(int64_t ntgt, int slices) {
+    size_t rows = 0;
+    const int64_t most = (ntgt + 127) / 128 + 8;
+    for (int64_t n = 1; n <= most && n * slices <= 444; ++n) {
+        const int s = m2l_tc_split((int)n, slices);
+        if (s > 1) {
+            const size_t r = (size_t)s * (size_t)(128 * n < ntgt ? 128 * n : ntgt);
+            if (r > rows) rows = r;
+        }
+    }
+    return rows;
 }
 
 struct M2L64Args {
@@ -54,9 +81,10 @@ struct M2L64Args {
 };
 
 int m2l_fp64_launch(Handle& h, const double* M, double* Lown);   // the plain form's M2L, on h.stream
-// adds the ranges' sums (split above 1) into Lown
-int m2l64_sum_launch(Handle& h, const M2L64Args& a, double* Lown, cudaStream_t st);
-int m2l64_args(Handle& h, M2L64Args* a);
+// the ranges' sums (split above 1) into Lown; slices > 0: those of the tensor-core M2L (dofs
+// 1 .. K - 1)
+int m2l64_sum_launch(Handle& h, const M2L64Args& a, int slices, double* Lown, cudaStream_t st);
+int m2l64_args(Handle& h, int slices, M2L64Args* a);
 // operators [343][K padded to 4][NP + 4] of the plain form, zero padded, for d_m2l
 int m2l64_pad_rows(int p);
 int m2l64_pad_cols(int p);

@@ -268,7 +268,7 @@ int launch_rot(Handle& h, const double* M, double* Lown) {
     constexpr size_t rsm = RotCfg<P>::SMEM;
     OGX_CUDA(smem_optin((const void*)k_m2l_rot<P>, (int)rsm));
     M2L64Args a;
-    OGX_TRY(m2l64_args(h, &a));
+    OGX_TRY(m2l64_args(h, 0, &a));
     static const int per_sm = [] {
         int b = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_m2l_rot<P>, RotCfg<P>::THREADS, rsm) != cudaSuccess) {
@@ -280,7 +280,7 @@ int launch_rot(Handle& h, const double* M, double* Lown) {
     const int grid = (int)std::min<int64_t>((int64_t)(h.ntgt_pad / ROT_TGT) * M2L64_MAXSPLIT, (int64_t)per_sm * h.num_sms);
     k_m2l_rot<P><<<grid, RotCfg<P>::THREADS, rsm, h.stream>>>(h.tv, a, h.d_rot, M, Lown);
     ++h.launches;
-    return m2l64_sum_launch(h, a, Lown, h.stream);
+    return m2l64_sum_launch(h, a, 0, Lown, h.stream);
 }
 
 }  // namespace

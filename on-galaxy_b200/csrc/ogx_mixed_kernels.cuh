@@ -19,6 +19,9 @@
 //     scaling every multipole row and every operator by a power of two that puts
 //     its largest entry in [0.5, 1), undone exactly per row and combination when
 //     the result is drained;
+//   * a small tree has fewer tiles than SMs (8,192 bodies: 8, each a serial walk of ~150
+//     combinations, 183 us): its tiles are cut into ranges of colleague slots (ogx_m2l64.cuh),
+//     one CTA each, whose sums are added in range order;
 //   * accumulation: FP32 accumulation over all ~6000 MMA steps of a tile loses
 //     ~1e-5 of the (strongly cancelling) far field, so every combination gets a
 //     fresh FP32 accumulator (a ring of buffers in TMEM) that the epilogue warps
@@ -51,6 +54,7 @@
 #include <cuda_fp16.h>
 
 #include "ogx_harmonics.cuh"
+#include "ogx_m2l64.cuh"
 #include "ogx_sm100.cuh"
 
 namespace ogx {
@@ -164,8 +168,7 @@ __device__ __forceinline__ void drain_combo(uint32_t tmem_lane, int a, bool firs
 
 template <int P>
 __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
-    k_m2l_tc(TreeView tv, const uint32_t* __restrict__ tgt_key, const uint32_t* __restrict__ tgt_box,
-             const __half* __restrict__ mhi, const __half* __restrict__ mlo, const float* __restrict__ munscale,
+    k_m2l_tc(TreeView tv, M2L64Args ar, const __half* __restrict__ mhi, const __half* __restrict__ mlo, const float* __restrict__ munscale,
              const uint8_t* __restrict__ btab, const float* __restrict__ ounscale, double* __restrict__ lown, int* err) {
     using C = TcCfg<P>;
     static_assert(C::SUPPORTED, "tensor-core M2L: operand does not fit");
@@ -188,7 +191,13 @@ __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
     __shared__ int s_combo[189];      // present combinations: D | s << 5 | o << 8
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int base = blockIdx.x * 128;
+    const uint32_t* __restrict__ tgt_key = ar.tgt_key;
+    const uint32_t* __restrict__ tgt_box = ar.tgt_box;
     if (tv_over(tv)) return;
+    // this CTA's ranges of colleague slots: [zlo, zhi) of the S ranges (any grid z is correct)
+    const int S = m2l_tc_split(ar.gs[GS_TILES128], C::NSPLIT);
+    const int zlo = S * (int)blockIdx.z / (int)gridDim.z, zhi = S * ((int)blockIdx.z + 1) / (int)gridDim.z;
+    if (zlo == zhi) return;
     if (tid == 0) {
         s_t = (tgt_key[base] == 0xFFFFFFFFu) ? -1 : (int)tgt_key[base];
         s_abort = 0;
@@ -208,6 +217,7 @@ __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
     __syncthreads();
     const int t = s_t;
     if (t < 0) return;
+    const int D0 = m2l64_first_slot(zlo, S, t), D1 = m2l64_first_slot(zhi, S, t);
     // the A operands of every stage start at zero (rows without a source are not copied)
     for (int i = tid; i < C::STAGES * 2 * C::A_BYTES / 16; i += blockDim.x) {
         const int sg = i / (2 * C::A_BYTES / 16), off = i - sg * (2 * C::A_BYTES / 16);
@@ -238,7 +248,7 @@ __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
 #pragma unroll
             for (int i = 0; i < DPT; ++i) {
                 const int D = g + i * NGS;
-                Qv[i] = (D < 27 && par >= 0) ? __ldg(tv.col + 27 * (size_t)par + D) : -1;
+                Qv[i] = (D >= D0 && D < D1 && par >= 0) ? __ldg(tv.col + 27 * (size_t)par + D) : -1;
             }
             int4 cr[DPT][2];
 #pragma unroll
@@ -465,10 +475,65 @@ __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
         for (int g = 0; g < (C::REGACC ? C::MAXG : 1); ++g)
 #pragma unroll
             for (int i = 0; i < 16; ++i) racc[g][i] = 0.0, part[g][i] = 0.f;
+        int z = zlo, zend = m2l64_first_slot(zlo + 1, S, t);   // the range of the current combination, its first slot behind
+        bool fresh = true;                                     // no combination of this range yet
+        // the finished range's sums (zeros where it had no combination) to its row
+        auto flush = [&]() {
+            // to the box's local (one range), else to the range's row of the partial sums
+            // (k_m2l64_sum adds them in range order)
+            const int myb = s_box[row];
+            double inv = 1.0;
+            double* o = nullptr;
+            if (myb >= 0 && S == 1) {
+                inv = 1.0 / (2.0 * tv.center[4 * (size_t)myb + 3]);
+                o = lown + (size_t)myb * C::K;
+            } else if (myb >= 0) {
+                const int pq = base + row - ar.gs[9 + t];
+                o = ar.part + ((size_t)z * tv.cnt->ntgt32 + ar.gs[t] + (int64_t)(pq / 128) * ar.gs[GS_FILL] + pq % 128) * C::K;
+            }
+            if constexpr (C::REGACC) {
+#pragma unroll
+                for (int g = 0; g < C::MAXG; ++g) {
+                    const int c16 = g0 + g;
+                    if (c16 < g1 && myb >= 0) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const int col = c16 * 16 + i, dof = 1 + zs * C::N + col;
+                            if (col < C::N && dof < C::K) o[dof] = racc[g][i] * inv;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) racc[g][i] = 0.0;
+                }
+            } else {
+#pragma unroll 1
+                for (int c16 = g0; c16 < g1; ++c16) {
+                    uint32_t lo[16], hi[16];
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) lo[k] = hi[k] = 0u;
+                    if (!fresh) {
+                        sm100::tmem_ld16(tmem_lane + C::ACC64 + c16 * 32, lo);
+                        sm100::tmem_ld16(tmem_lane + C::ACC64 + c16 * 32 + 16, hi);
+                        sm100::tmem_ld_wait();
+                    }
+                    if (myb >= 0) {
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) {
+                            const int col = c16 * 16 + k, dof = 1 + zs * C::N + col;
+                            if (col < C::N && dof < C::K) o[dof] = __hiloint2double((int)hi[k], (int)lo[k]) * inv;
+                        }
+                    }
+                }
+            }
+            fresh = true;
+            ++z;
+            zend = m2l64_first_slot(z + 1, S, t);
+        };
         for (int k = 0; k < nco && !s_abort; ++k) {
             const int a = k % NBUF;
             // this row's source for combination k and the scales its operands carry
             const int code = s_combo[k];
+            while ((code & 31) >= zend && z + 1 < zhi) flush();
             // combinations come grouped by colleague slot D (the eight children of one
             // colleague, at similar distances): their FP32 results are summed in FP32 and
             // the slot's sum is folded into FP64 once, after its last combination
@@ -510,47 +575,15 @@ __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
                     }
                 }
             } else {
-                drain_combo<C::NPAD, C::DBUF, C::ACC64, C::PAIR>(tmem_lane, a, k == 0, g0, g1, unscale);
+                drain_combo<C::NPAD, C::DBUF, C::ACC64, C::PAIR>(tmem_lane, a, fresh, g0, g1, unscale);
             }
+            fresh = false;
             sm100::tc_fence_before();
             sm100::mbar_arrive(&dempty[a]);
         }
-        if (nco >= 1 && !s_abort) {
-            const int myb = s_box[quarter * 32 + lane];
-            const double inv = (myb >= 0) ? 1.0 / (2.0 * tv.center[4 * myb + 3]) : 0.0;
-            if constexpr (C::REGACC) {
-                if (myb >= 0) {
-#pragma unroll
-                    for (int g = 0; g < C::MAXG; ++g) {
-                        const int c16 = g0 + g;
-                        if (c16 < g1) {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                const int col = c16 * 16 + i, dof = 1 + zs * C::N + col;
-                                if (col < C::N && dof < C::K) lown[(size_t)myb * C::K + dof] += racc[g][i] * inv;
-                            }
-                        }
-                    }
-                }
-            } else {
-                sm100::tc_fence_after();
-#pragma unroll 1
-                for (int c16 = g0; c16 < g1; ++c16) {
-                    uint32_t lo[16], hi[16];
-                    sm100::tmem_ld16(tmem_lane + C::ACC64 + c16 * 32, lo);
-                    sm100::tmem_ld16(tmem_lane + C::ACC64 + c16 * 32 + 16, hi);
-                    sm100::tmem_ld_wait();
-                    if (myb >= 0) {
-#pragma unroll
-                        for (int k = 0; k < 16; ++k) {
-                            const int col = c16 * 16 + k, dof = 1 + zs * C::N + col;
-                            if (col < C::N && dof < C::K)
-                                lown[(size_t)myb * C::K + dof] += __hiloint2double((int)hi[k], (int)lo[k]) * inv;
-                        }
-                    }
-                }
-            }
-        }
+        // (one range and no combination: the local stays zero)
+        if (!s_abort && (nco >= 1 || S > 1))
+            while (z < zhi) flush();
     }
     sm100::tc_fence_before();
     __syncthreads();
@@ -591,31 +624,55 @@ __global__ void __launch_bounds__(128) k_split_mpole(const double* __restrict__ 
     if (lane == 0) munscale[b] = ldexpf(1.0f, e);
 }
 
-// L_0^0 of the M2L (needed only for potentials): FP64 row 0 of every T_o
+// L_0^0 of the M2L (needed only for potentials): FP64 row 0 of every T_o.  Warp per target:
+// lane D lists the V children of colleague slot D, then the lanes run over the coefficients
+// of one source after another (a thread per target read K doubles of 189 sources on its own,
+// 510 us on 262,144 bodies at p = 4).
 template <int P>
-__global__ void __launch_bounds__(128) k_m2l_dof0(TreeView tv, int ntgt_pad, const uint32_t* tgt_key, const uint32_t* tgt_box,
-                                                  const double* row0 /* 343 x K */, const double* M, double* lown) {
-    constexpr int K = (P + 1) * (P + 1);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ntgt_pad || tv_over(tv) || tgt_key[i] == 0xFFFFFFFFu) return;
-    const int b = (int)tgt_box[i], t = (int)tgt_key[i];
-    const int par = tv.parent[b];
-    const int tx = t & 1, ty = (t >> 1) & 1, tz = (t >> 2) & 1;
-    double acc = 0.0;
-    for (int D = 0; D < 27; ++D) {
-        const int Q = tv.col[27 * par + D];
-        if (Q < 0) continue;
-        const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
-        for (int s = 0; s < 8; ++s) {
-            const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
-            if (max(abs(ox), max(abs(oy), abs(oz))) <= 1) continue;
-            const int c = tv.child[8 * Q + s];
-            if (c < 0) continue;
-            const double* r0 = row0 + (size_t)((ox + 3) + 7 * (oy + 3) + 49 * (oz + 3)) * K;
-            for (int k = 0; k < K; ++k) acc = fma(r0[k], M[(size_t)c * K + k], acc);
-        }
+__global__ void __launch_bounds__(128) k_m2l_dof0(TreeView tv, int ntgt_bound, const uint32_t* __restrict__ box,
+                                                  const double* __restrict__ row0 /* 343 x K */, const double* __restrict__ M,
+                                                  double* __restrict__ lown) {
+    constexpr int K = (P + 1) * (P + 1), NPL = (K + 31) / 32;
+    __shared__ int s_src[4][192], s_op[4][192];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 4 + w;
+    if (i >= ntgt_bound || tv_over(tv) || i >= tv.cnt->ntgt32) return;
+    const int b = (int)box[i], par = tv.parent[b];
+    const int tx = tv.coord[3 * (size_t)b] & 1, ty = tv.coord[3 * (size_t)b + 1] & 1, tz = tv.coord[3 * (size_t)b + 2] & 1;
+    const int Q = lane < 27 ? tv.col[27 * (size_t)par + lane] : -1;
+    int4 c0 = make_int4(-1, -1, -1, -1), c1 = c0;
+    if (Q >= 0) {
+        c0 = __ldg(reinterpret_cast<const int4*>(tv.child + 8 * (size_t)Q));
+        c1 = __ldg(reinterpret_cast<const int4*>(tv.child + 8 * (size_t)Q) + 1);
     }
-    lown[(size_t)b * K] += acc / (2.0 * tv.center[4 * b + 3]);
+    const int ch[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+    const int Dx = lane % 3 - 1, Dy = (lane / 3) % 3 - 1, Dz = lane / 9 - 1;
+    int n = 0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
+        const bool v = ch[s] >= 0 && max(abs(ox), max(abs(oy), abs(oz))) > 1;
+        const unsigned m = __ballot_sync(0xffffffffu, v);
+        if (v) {
+            const int q = n + __popc(m & ((1u << lane) - 1u));
+            s_src[w][q] = ch[s];
+            s_op[w][q] = (ox + 3) + 7 * (oy + 3) + 49 * (oz + 3);
+        }
+        n += __popc(m);
+    }
+    __syncwarp();
+    double acc = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) {
+        const double* m = M + (size_t)s_src[w][q] * K;
+        const double* r = row0 + (size_t)s_op[w][q] * K;
+#pragma unroll
+        for (int u = 0; u < NPL; ++u)
+            if (lane + 32 * u < K) acc = fma(__ldg(r + lane + 32 * u), __ldg(m + lane + 32 * u), acc);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) lown[(size_t)b * K] += acc / (2.0 * tv.center[4 * (size_t)b + 3]);
 }
 
 // acc[orig] = G (far + near), pot[orig] = -G (far + near) (AdaptiveFMM3D.hpp:104)

@@ -1,7 +1,7 @@
 // ogx_near.cuh -- the near field (softened P2P over the U lists) of both forms.
 //
 // Replaces the pair loop of AdaptiveFMM3D::computeAccelerations (src3d/AdaptiveFMM3D.hpp:95-103).
-// A one-warp block takes one work item (leaf, chunk of at most 32 targets; k_near_chunks), so
+// A one-warp block takes one work item (leaf, chunk of at most 32 targets; k_leaf_occupancy), so
 // a leaf of many bodies (the eps floor stops splitting in dense cores) spreads over many
 // blocks.  In a chunk of T targets, unit u = lane + 32 r is target u mod T with source part
 // u / T, which takes every G-th source quad of each staged round.  The leaf itself is one
@@ -39,13 +39,6 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
 }
 
 constexpr int NEAR_CAP = 128;    // source bodies staged per round (several U-list entries)
-
-// work items of the near field: ceil(bodies / 32) per leaf (none for capacity padding)
-static __global__ void k_near_chunks(TreeView tv, int* __restrict__ cnt) {
-    const int lf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lf >= tv.nleaf) return;
-    cnt[lf] = (lf < tv_nleaf(tv) && !tv_over(tv)) ? (tv.pcount[tv.leafbox[lf]] + 31) / 32 : 0;
-}
 
 // Number of source parts G for a chunk of T targets: units (target, part) = T G,
 // at most NU, are spread over the 32 lanes in R = ceil(T G / 32) rounds; G maximises

@@ -145,13 +145,24 @@ __device__ __forceinline__ int key_digit(uint64_t hi, uint32_t lo, int level) {
 }
 
 // ---- 3. topology per sorted position ------------------------------------------
-__global__ void k_topo_pairs(const uint64_t* khi, const uint32_t* klo, int64_t n, int thr, int* dfirst, signed char* cplthr) {
+// deep: the keys are sorted by levels 1..16 only (digit passes 3..8); flags a level-16 box
+// that holds more than thr bodies, i.e. bodies whose leaf may lie deeper, for which the
+// order of the lower digits matters.  Keys of one box are contiguous, so such a box
+// has two keys thr apart with the same 48-bit prefix (bits 15..62 of the high word).
+__global__ void k_topo_pairs(const uint64_t* khi, const uint32_t* klo, int64_t n, int thr, bool deep, int* dfirst,
+                             signed char* cplthr, DevCounts* counts) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint64_t hi = khi[i];
     const uint32_t lo = klo[i];
     dfirst[i] = (i == 0) ? 0 : cpl72(khi[i - 1], klo[i - 1], hi, lo) + 1;
-    cplthr[i] = (i + thr < n) ? (signed char)cpl72(hi, lo, khi[i + thr], klo[i + thr]) : (signed char)-1;
+    signed char c = -1;
+    if (i + thr < n) {
+        const uint64_t ht = khi[i + thr];
+        c = (signed char)cpl72(hi, lo, ht, klo[i + thr]);
+        if (deep && (hi >> 15) == (ht >> 15)) counts->deep_flag = 1;
+    }
+    cplthr[i] = c;
 }
 
 constexpr int WM_BLOCK = 1024;
@@ -193,24 +204,37 @@ __global__ void __launch_bounds__(WM_BLOCK) k_topo_levels(const signed char* cpl
     if (threadIdx.x < kMaxDepth + 2 && s_hist[threadIdx.x] != 0) atomicAdd(&counts->level_hist[threadIdx.x], s_hist[threadIdx.x]);
 }
 
+// one warp, lane = level: boxes per level, first box of every level, totals
 __global__ void k_counts_finalize(DevCounts* counts, const int64_t* recoff, const int64_t* leafscan, int64_t n, int* level_off_dev) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    counts->num_boxes = recoff[n];
-    counts->num_leaves = leafscan[n];
-    counts->nb32 = (int32_t)recoff[n];
-    counts->nleaf32 = (int32_t)leafscan[n];
-    int run = 0, maxl = 0;
-    int cum = 0;
-    level_off_dev[0] = 0;
-    for (int l = 0; l <= kMaxDepth; ++l) {
-        run += counts->level_hist[l];   // boxes at level l
+    const int l = threadIdx.x;
+    const int64_t nb = recoff[n], nl = leafscan[n];
+    int run = l <= kMaxDepth ? counts->level_hist[l] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, run, o);
+        if (l >= o) run += y;
+    }
+    if (l > kMaxDepth) run = 0;          // boxes at level l
+    int cum = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL, cum, o);
+        if (l >= o) cum += y;
+    }
+    if (l <= kMaxDepth) {
         counts->level_hist[l] = run;
-        if (run > 0) maxl = l;
-        cum += run;
         level_off_dev[l + 1] = cum;
     }
-    counts->level_hist[kMaxDepth + 1] = 0;
-    counts->max_level = maxl;
+    const unsigned some = __ballot_sync(FULL, run > 0);
+    if (l == 0) {
+        counts->num_boxes = nb;
+        counts->num_leaves = nl;
+        counts->nb32 = (int32_t)nb;
+        counts->nleaf32 = (int32_t)nl;
+        level_off_dev[0] = 0;
+        counts->level_hist[kMaxDepth + 1] = 0;
+        counts->max_level = some ? 31 - __clz((int)some) : 0;
+    }
 }
 
 __global__ void k_emit_records(const int* cnt, const int* dfirst, const int* leaflev, const int64_t* recoff, int64_t n,
@@ -237,9 +261,13 @@ __global__ void k_emit_records(const int* cnt, const int* dfirst, const int* lea
 __global__ void k_boxes(int nb_cap, const uint32_t* reclev, const uint32_t* recpos, const int* level_off, const uint64_t* khi,
                         const uint32_t* klo, const int* leaflev, const int64_t* leafscan, const int* leafstart,
                         const RootInfo* root, int* level, int* coord, double* center, int* parent, int* child, int* leafid,
-                        int* pfirst, int* pcount, int* leafbox, const DevCounts* counts) {
+                        int* pfirst, int* pcount, int* leafbox, int* nlflag, const DevCounts* counts) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nb_cap || counts->overflow) return;
+    if (k >= nb_cap) return;
+    if (counts->overflow) {
+        nlflag[k] = 0;
+        return;
+    }
     if (k >= counts->nb32) {
         level[k] = -1;
         coord[3 * k] = coord[3 * k + 1] = coord[3 * k + 2] = 0;
@@ -248,6 +276,7 @@ __global__ void k_boxes(int nb_cap, const uint32_t* reclev, const uint32_t* recp
         leafid[k] = -1;
         pfirst[k] = 0;
         pcount[k] = 0;
+        nlflag[k] = 0;
         return;
     }
     const int l = (int)reclev[k];
@@ -280,7 +309,9 @@ __global__ void k_boxes(int nb_cap, const uint32_t* reclev, const uint32_t* recp
         pcount[k] = leafstart[lf + 1] - s;
     } else {
         leafid[k] = -1;
+        pcount[k] = 0;
     }
+    nlflag[k] = isleaf ? 0 : 1;
     if (l == 0) { parent[k] = -1; return; }
     // parent: last box of level l-1 whose first position <= s
     int lo_i = level_off[l - 1], hi_i = level_off[l] - 1;
@@ -292,10 +323,11 @@ __global__ void k_boxes(int nb_cap, const uint32_t* reclev, const uint32_t* recp
     child[8 * lo_i + key_digit(hi, lo, l)] = k;
 }
 
-__global__ void k_leaf_occupancy(int nleaf_cap, const int* leafbox, const int* pcount, DevCounts* counts) {
-    if (counts->overflow) return;
+// also the near field's work items per leaf: ceil(bodies / 32) (none for capacity padding)
+__global__ void k_leaf_occupancy(int nleaf_cap, const int* leafbox, const int* pcount, int* nchunk, DevCounts* counts) {
     const int lf = blockIdx.x * blockDim.x + threadIdx.x;
-    int c = (lf < nleaf_cap && lf < counts->nleaf32) ? pcount[leafbox[lf]] : 0;
+    int c = (lf < nleaf_cap && lf < counts->nleaf32 && !counts->overflow) ? pcount[leafbox[lf]] : 0;
+    if (lf < nleaf_cap) nchunk[lf] = (c + 31) / 32;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c = max(c, __shfl_xor_sync(FULL, c, o));
     if ((threadIdx.x & 31) == 0 && c > 0) atomicMax(&counts->max_leaf_occ, c);
@@ -329,40 +361,15 @@ __global__ void k_gather_bodies(const uint32_t* perm, const double* pos, const d
 
 }  // namespace
 
-static // flag the non-leaf boxes and count them per level
-__global__ void k_nonleaf_flags(int nb_cap, const int* __restrict__ leafid, const int* __restrict__ level, int* flag,
-                                DevCounts* counts) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb_cap) return;
-    const int f = !counts->overflow && b < counts->nb32 && leafid[b] < 0;
-    flag[b] = f;
-    if (f) atomicAdd(&counts->nonleaf_level[level[b]], 1);
-}
-
-__global__ void k_nonleaf_emit(int nb, const int* __restrict__ flag, const int64_t* __restrict__ off, int* out) {
+// the non-leaf boxes in box order (level-major) and the first one of every level
+static __global__ void k_nonleaf_emit(int nb, const int* __restrict__ flag, const int64_t* __restrict__ off,
+                                      const int* __restrict__ level_off, int* out, int* nl_off, const DevCounts* counts) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < nb && flag[b]) out[off[b]] = b;
-}
-
-// nl_off[l] = first non-leaf box of level l in the compacted list (exclusive scan of
-// the per-level counts; the list is level-major)
-__global__ void k_nonleaf_offsets(const DevCounts* counts, int* nl_off) {
-    if (threadIdx.x != 0) return;
-    int c = 0;
-    for (int l = 0; l <= kMaxDepth; ++l) {
-        nl_off[l] = c;
-        c += counts->nonleaf_level[l];
+    if (blockIdx.x == 0 && threadIdx.x < kMaxDepth + 2) {
+        const int first = counts->overflow ? 0 : min(level_off[threadIdx.x], nb);
+        nl_off[threadIdx.x] = (int)off[first];
     }
-    nl_off[kMaxDepth + 1] = c;
-}
-
-// After a sort by levels 1..16 only (digit passes 3..8): flags a level-16 box that
-// holds more than thr bodies, i.e. bodies whose leaf may lie deeper, for which the
-// order of the lower digits matters.  Keys of one box are contiguous, so such a box
-// has two keys thr apart with the same 48-bit prefix (bits 15..62 of the high word).
-__global__ void k_deep_check(const uint64_t* __restrict__ khi, int64_t n, int thr, DevCounts* counts) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i + thr < n && (khi[i] >> 15) == (khi[i + thr] >> 15)) counts->deep_flag = 1;
 }
 
 inline int grid_for(int64_t n, int b) { return (int)((n + b - 1) / b); }
@@ -441,8 +448,7 @@ int tree_build(Handle& h, const double* d_pos, const double* d_mass, int64_t n) 
         if (attempt > 0) OGX_CUDA(cudaMemsetAsync(dc, 0, sizeof(DevCounts), st));
         k_keys<<<grid_for(n, 256), 256, 0, st>>>(d_pos, n, root, khi_in, klo_in, kidx_in); ++h.launches;
         OGX_TRY(radix_sort_key72(h, n, first_pass, &khi, &klo, &kidx));
-        if (first_pass > 0 && n > thr) { k_deep_check<<<grid_for(n, 256), 256, 0, st>>>(khi, n, thr, dc); ++h.launches; }
-        k_topo_pairs<<<grid_for(n, 256), 256, 0, st>>>(khi, klo, n, thr, dfirst, cplthr); ++h.launches;
+        k_topo_pairs<<<grid_for(n, 256), 256, 0, st>>>(khi, klo, n, thr, first_pass > 0, dfirst, cplthr, dc); ++h.launches;
         k_topo_levels<<<grid_for(n, WM_BLOCK), WM_BLOCK, wm_smem, st>>>(cplthr, dfirst, n, thr, root, leaflev, cnt, leafflag, dc); ++h.launches;
         OGX_TRY(scan2_i32_to_i64(h, cnt, recoff, leafflag, leafscan, n));
         k_counts_finalize<<<1, 32, 0, st>>>(dc, recoff, leafscan, n, level_off_dev); ++h.launches;
@@ -495,23 +501,23 @@ int tree_build(Handle& h, const double* d_pos, const double* d_mass, int64_t n) 
     OGX_TRY(arena_get(h.ws, S_BOX_PCOUNT, nb, &pcount));
     OGX_TRY(arena_get(h.ws, S_LEAF_BOX, nleaf, &leafbox));
     OGX_CUDA(cudaMemsetAsync(child, 0xFF, 8 * sizeof(int) * (size_t)nb, st));
-    OGX_CUDA(cudaMemsetAsync(pcount, 0, sizeof(int) * (size_t)nb, st));
+    int* nl_flag;
+    OGX_TRY(arena_get(h.ws, S_NONLEAF_FLAG, nb, &nl_flag));
     k_boxes<<<grid_for(nb, 128), 128, 0, st>>>(nb, reclev, recpos_s, level_off_dev, khi, klo, leaflev, leafscan, leafstart, root,
-                                                level, coord, center, parent, child, leafid, pfirst, pcount, leafbox, dc); ++h.launches;
-    k_leaf_occupancy<<<grid_for(nleaf, 128), 128, 0, st>>>(nleaf, leafbox, pcount, dc); ++h.launches;
+                                                level, coord, center, parent, child, leafid, pfirst, pcount, leafbox, nl_flag, dc); ++h.launches;
+    int* nchunk;
+    OGX_TRY(arena_get(h.ws, S_NEAR_CHUNK, nleaf, &nchunk));
+    k_leaf_occupancy<<<grid_for(nleaf, 128), 128, 0, st>>>(nleaf, leafbox, pcount, nchunk, dc); ++h.launches;
 
     // non-leaf boxes in box order (level-major, so each level's parents are contiguous)
-    int *nl_flag, *nonleaf;
+    int* nonleaf;
     int64_t* nl_off;
-    OGX_TRY(arena_get(h.ws, S_NONLEAF_FLAG, nb, &nl_flag));
     OGX_TRY(arena_get(h.ws, S_NONLEAF_OFF, nb + 1, &nl_off));
     OGX_TRY(arena_get(h.ws, S_NONLEAF, nb, &nonleaf));
-    k_nonleaf_flags<<<grid_for(nb, 256), 256, 0, st>>>(nb, leafid, level, nl_flag, dc); ++h.launches;
     OGX_TRY(scan_i32_to_i64(h, nl_flag, nl_off, nb));
-    k_nonleaf_emit<<<grid_for(nb, 256), 256, 0, st>>>(nb, nl_flag, nl_off, nonleaf); ++h.launches;
     int* nl_loff;
     OGX_TRY(arena_get(h.ws, S_NONLEAF_LOFF, kMaxDepth + 2, &nl_loff));
-    k_nonleaf_offsets<<<1, 32, 0, st>>>(dc, nl_loff); ++h.launches;
+    k_nonleaf_emit<<<grid_for(nb, 256), 256, 0, st>>>(nb, nl_flag, nl_off, level_off_dev, nonleaf, nl_loff, dc); ++h.launches;
     h.d_nonleaf = nonleaf;
     h.d_nonleaf_off = nl_loff;
 

@@ -41,3 +41,21 @@ def test_result_does_not_depend_on_the_tile(ogx, n):
             s.set_tuning(m2l_tile_targets=fill)
             out.append(s.compute_accelerations(pos, mass))
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("p", [4, 6, 9, 10, 12])
+@pytest.mark.parametrize("n", [300, 5000, 60000])
+def test_tensor_core_ranges(ogx, p, n):
+    # FP64 sums in registers (p <= 8), in TMEM (9, 10), column slices (12); 1 to 27 ranges; with
+    # potentials (degree 0).  The batch width changes no bit; 5e-6: the mixed form's bar.
+    pos, _, mass = ogx_ic.plummer(n, seed=p)
+    with ogx.AdaptiveFMM3D(p=p, threshold=24, precision=ogx.PREC_FP64) as s:
+        ref, ref_pot = s.compute_accelerations(pos, mass, with_potential=True)
+    out = []
+    for fill in (128, 32):
+        with ogx.AdaptiveFMM3D(p=p, threshold=24, precision=ogx.PREC_MIXED) as s:
+            s.set_tuning(m2l_tile_targets=fill)
+            out.append(s.compute_accelerations(pos, mass, with_potential=True))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    assert rel_err(ref, out[0][0])[1] <= 5e-6
+    assert abs(out[0][1] - ref_pot).max() <= 5e-6 * abs(ref_pot).max()
