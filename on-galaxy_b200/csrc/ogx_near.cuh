@@ -4,7 +4,7 @@
 // A one-warp block takes one work item (leaf, chunk of at most 32 targets; k_leaf_occupancy), so
 // a leaf of many bodies (the eps floor stops splitting in dense cores) spreads over many
 // blocks.  In a chunk of T targets, unit u = lane + 32 r is target u mod T with source part
-// u / T, which takes every G-th source quad of each staged round.  The leaf itself is one
+// u / T, which takes every G-th source of each staged round.  The leaf itself is one
 // round (with the self pair skipped); the bodies of all other U-list entries are
 // concatenated and staged NEAR_CAP at a time.  The G parts of each target are added in part
 // order in FP64 through shared memory (deterministic).
@@ -14,10 +14,13 @@
 // the two hi parts lie within a factor of two of each other, so s_hi - t_hi is exact
 // (Sterbenz) and d = (s_hi - t_hi) + (s_lo - t_lo) carries the FP32 relative accuracy of |d|
 // itself (absolute error ~2^-48 of the root box), however small |d| is.  Bound: issue slots
-// (the FMA pipe was 45% busy at 75% issue); two sources go together in packed f32x2
-// operations, and the staged sources lie as separate x, y, z, m arrays so that one 16-byte
-// load brings a coordinate of four.  Every round's sum goes into a compensated (Kahan)
-// accumulator.
+// (the FMA pipe was 45% busy at 75% issue); two sources of a part go together in packed
+// f32x2 operations up to the pair's weight, and a part's staged sources lie one after another
+// in separate x, y, z, m arrays so that one 16-byte load brings a coordinate of four.  The
+// sums take the sources one by one: another order of the sums is as exact, but unsoftened
+// close pairs amplify its rounding over a few steps.  (Two targets per operation leave half
+// the lanes of a 32-target chunk idle: 1.5 ms.)  Every round's sum goes into a compensated
+// (Kahan) accumulator.
 // FP64 (plain form): the same items and rounds on pair64 (ogx_pair64.cuh); one warp per
 // chunk walked the list source by source before, half its lanes idle on a 17-body leaf.
 #pragma once
@@ -29,7 +32,6 @@
 
 namespace ogx {
 namespace near_field {
-constexpr int NEAR_UNROLL = 1, NEAR_MINB = 32;
 
 __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
     const float y = v - c;
@@ -59,6 +61,15 @@ __device__ __forceinline__ int near_parts(int T) {
 // KM (kernel): 0 Plummer's (eps2); 1 the spline of support hs (ogx_softening.cuh);
 // 2 (FP32) the spline minus the Newtonian kernel, zero from hs on (the far field's pairs
 // inside the support, OGX_SOFT_SPLINE)
+// The G parts of a staged round: part p holds sources p, p + G, ...; S slots per part
+struct Parts {
+    int G, S;
+    unsigned inv;   // x / G = x * inv >> 16 for x < NEAR_CAP
+    __device__ __forceinline__ explicit Parts(int g) : G(g), S(((NEAR_CAP + g - 1) / g + 3) & ~3), inv((65536u + g - 1) / g) {}
+    __device__ __forceinline__ int div(int q) const { return (int)((unsigned)q * inv >> 16); }
+    __device__ __forceinline__ int count(int p, int n) const { return n > p ? div(n - p - 1) + 1 : 0; }
+};
+
 template <class T>
 struct NearPrm {
     T eps2, hs, hinv;
@@ -68,23 +79,27 @@ struct NearPrm {
 struct Near32 {
     using T = float;
     struct Bodies { const float4 *hi, *lo; };
-    struct alignas(16) Stage { float v[7][NEAR_CAP]; };   // hi x, y, z, lo x, y, z, mass
+    // hi x, y, z, lo x, y, z, mass; a part's sources lie one after another (G S <= 168 slots for the G that near_parts gives)
+    struct alignas(16) Stage { float v[7][192]; };
     struct Target { float h[3], l[3]; };
     struct Acc { float s[4], c[4]; };
 
-    __device__ static __forceinline__ void put(Stage& st, const Bodies& b, int q, int j) {
+    __device__ static __forceinline__ void put(Stage& st, const Parts& pa, const Bodies& b, int q, int j) {
         const float4 h = b.hi[j], l = b.lo[j];
-        st.v[0][q] = h.x; st.v[1][q] = h.y; st.v[2][q] = h.z;
-        st.v[3][q] = l.x; st.v[4][q] = l.y; st.v[5][q] = l.z;
-        st.v[6][q] = h.w;
+        const int i = pa.div(q), e = (q - i * pa.G) * pa.S + i;
+        st.v[0][e] = h.x; st.v[1][e] = h.y; st.v[2][e] = h.z;
+        st.v[3][e] = l.x; st.v[4][e] = l.y; st.v[5][e] = l.z;
+        st.v[6][e] = h.w;
     }
-    // sources n .. next multiple of 4: no mass, far away (a finite distance, no zero)
-    __device__ static __forceinline__ void pad(Stage& st, int n, int lane) {
-        const int q = n + lane;
-        if (lane < 3 && q < ((n + 3) & ~3)) {
-            st.v[0][q] = 1e18f;
+    // every part up to a multiple of 4: no mass, far away (a finite distance, no zero)
+    __device__ static __forceinline__ void pad(Stage& st, const Parts& pa, int n, int lane) {
+        for (int i = lane; i < 4 * pa.G; i += 32) {
+            const int p = i >> 2, c = pa.count(p, n), k = (c & ~3) + (i & 3);
+            if ((c & 3) && k >= c) {
+                st.v[0][p * pa.S + k] = 1e18f;
 #pragma unroll
-            for (int a = 1; a < 7; ++a) st.v[a][q] = 0.f;
+                for (int a = 1; a < 7; ++a) st.v[a][p * pa.S + k] = 0.f;
+            }
         }
     }
     __device__ static __forceinline__ Target target(const Bodies& b, int i) {
@@ -97,26 +112,29 @@ struct Near32 {
     }
     __device__ static __forceinline__ double total(const Acc& a, int k) { return (double)a.s[k] - (double)a.c[k]; }
 
-    // sources of quads part, part + G, ... of a round of n; SELF: staged position self_q is the target
+    // the sources of one part of a round of n, in order; SELF: staged position self_q is the target
     template <bool SELF, bool POT, int KM>
-    __device__ static __forceinline__ void round(const Stage& st, int part, int G, int n, int self_q, const Target& t,
+    __device__ static __forceinline__ void round(const Stage& st, const Parts& pa, int part, int n, int self_q, const Target& t,
                                                  const NearPrm<float>& pr, Acc& acc) {
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+        const int quads = (pa.count(part, n) + 3) >> 2, first = part * pa.S >> 2;
+        int self = -1;   // the target's place in this part
+        if (SELF && self_q >= 0 && self_q < n) {
+            const int i = pa.div(self_q);
+            if (self_q - i * pa.G == part) self = i;
+        }
         if constexpr (KM == 0) {
-            f2 nh[3], nl[3], a[4];
+            f2 nh[3], nl[3];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 nh[k] = pack2(-t.h[k], -t.h[k]);
                 nl[k] = pack2(-t.l[k], -t.l[k]);
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) a[k].v = 0ull;
             const f2 e2 = pack2(pr.eps2, pr.eps2);
-            const int quads = (n + 3) >> 2;
-#pragma unroll NEAR_UNROLL
-            for (int q = part; q < quads; q += G) {
+            for (int i = 0; i < quads; ++i) {
                 ulonglong2 s[7];
 #pragma unroll
-                for (int k = 0; k < 7; ++k) s[k] = reinterpret_cast<const ulonglong2*>(st.v[k])[q];
+                for (int k = 0; k < 7; ++k) s[k] = reinterpret_cast<const ulonglong2*>(st.v[k])[first + i];
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
                     f2 d[3];
@@ -126,41 +144,48 @@ struct Near32 {
                     const f2 r2 = fma2(d[0], d[0], fma2(d[1], d[1], fma2(d[2], d[2], e2)));
                     // rsqrtf alone (within 2 ulp): its error, ~1e-7 per pair in random directions,
                     // stays far below the form's budget
-                    float ra, rb;
-                    unpack2(r2, ra, rb);
-                    float ya = rsqrtf(ra), yb = rsqrtf(rb);
+                    float y0, y1, w0, w1, m0, m1;
+                    unpack2(r2, y0, y1);
+                    y0 = rsqrtf(y0);
+                    y1 = rsqrtf(y1);
                     if (SELF) {
-                        if (4 * q + 2 * p == self_q) ya = 0.f;
-                        if (4 * q + 2 * p + 1 == self_q) yb = 0.f;
+                        if (4 * i + 2 * p == self) y0 = 0.f;
+                        if (4 * i + 2 * p + 1 == self) y1 = 0.f;
                     }
-                    const f2 y = pack2(ya, yb);
+                    const f2 y = pack2(y0, y1);
                     const f2 my = mul2(f2{p ? s[6].y : s[6].x}, y);
-                    const f2 w = mul2(mul2(my, y), y);
+                    unpack2(mul2(mul2(my, y), y), w0, w1);
+                    // the sums take the sources one by one, in order
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) a[k] = fma2(w, d[k], a[k]);
-                    if (POT) a[3] = add2(a[3], my);
+                    for (int k = 0; k < 3; ++k) {
+                        float d0, d1;
+                        unpack2(d[k], d0, d1);
+                        a[k] = fmaf(w1, d1, fmaf(w0, d0, a[k]));
+                    }
+                    if (POT) {
+                        unpack2(my, m0, m1);
+                        a[3] = (a[3] + m0) + m1;
+                    }
                 }
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < 3 || POT) kahan_add(acc.s[k], acc.c[k], sum2(a[k]));
         } else {
-            float a[4] = {0.f, 0.f, 0.f, 0.f};
-            const int quads = (n + 3) >> 2;
-            for (int qd = part; qd < quads; qd += G) {
+            for (int i = 0; i < quads; ++i) {
+                float4 s[7];
+#pragma unroll
+                for (int k = 0; k < 7; ++k) s[k] = reinterpret_cast<const float4*>(st.v[k])[first + i];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const int q = 4 * qd + u;
-                    const float dx = (st.v[0][q] - t.h[0]) + (st.v[3][q] - t.l[0]);
-                    const float dy = (st.v[1][q] - t.h[1]) + (st.v[4][q] - t.l[1]);
-                    const float dz = (st.v[2][q] - t.h[2]) + (st.v[5][q] - t.l[2]);
+                    auto el = [&](int k) { return u == 0 ? s[k].x : u == 1 ? s[k].y : u == 2 ? s[k].z : s[k].w; };
+                    const float dx = (el(0) - t.h[0]) + (el(3) - t.l[0]);
+                    const float dy = (el(1) - t.h[1]) + (el(4) - t.l[1]);
+                    const float dz = (el(2) - t.h[2]) + (el(5) - t.l[2]);
                     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    const float mq = st.v[6][q];
+                    const float mq = el(6);
                     if constexpr (KM == 1) {
-                        const bool self = SELF && q == self_q;
+                        const bool me = SELF && 4 * i + u == self;
                         float g, k;
-                        spline_gk<float>(self ? 1.0f : r2, pr.hs, pr.hinv, g, k);
-                        const float m = self ? 0.0f : mq;
+                        spline_gk<float>(me ? 1.0f : r2, pr.hs, pr.hinv, g, k);
+                        const float m = me ? 0.0f : mq;
                         const float w = m * g;
                         a[0] = fmaf(w, dx, a[0]);
                         a[1] = fmaf(w, dy, a[1]);
@@ -178,10 +203,10 @@ struct Near32 {
                     }
                 }
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (k < 3 || POT) kahan_add(acc.s[k], acc.c[k], a[k]);
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < 3 || POT) kahan_add(acc.s[k], acc.c[k], a[k]);
     }
 };
 
@@ -193,11 +218,11 @@ struct Near64 {
     struct Target { double x, y, z; };
     struct Acc { double s[4]; };
 
-    __device__ static __forceinline__ void put(Stage& st, const Bodies& b, int q, int j) {
+    __device__ static __forceinline__ void put(Stage& st, const Parts&, const Bodies& b, int q, int j) {
         st.xy[q] = make_double2(__ldg(b.x + j), __ldg(b.y + j));
         st.zm[q] = make_double2(__ldg(b.z + j), __ldg(b.m + j));
     }
-    __device__ static __forceinline__ void pad(Stage&, int, int) {}
+    __device__ static __forceinline__ void pad(Stage&, const Parts&, int, int) {}
     __device__ static __forceinline__ Target target(const Bodies& b, int i) { return Target{b.x[i], b.y[i], b.z[i]}; }
     __device__ static __forceinline__ void clear(Acc& a) {
 #pragma unroll
@@ -206,19 +231,19 @@ struct Near64 {
     __device__ static __forceinline__ double total(const Acc& a, int k) { return a.s[k]; }
 
     template <bool SELF, bool POT, int KM>
-    __device__ static __forceinline__ void round(const Stage& st, int part, int G, int n, int self_q, const Target& t,
+    __device__ static __forceinline__ void round(const Stage& st, const Parts& pa, int part, int n, int self_q, const Target& t,
                                                  const NearPrm<double>& pr, Acc& acc) {
         double a[4] = {0.0, 0.0, 0.0, 0.0};
         if constexpr (KM == 0) {
 #pragma unroll 4
-            for (int q = part; q < n; q += G) {
+            for (int q = part; q < n; q += pa.G) {
                 if (SELF && q == self_q) continue;
                 const double2 p = st.xy[q], r = st.zm[q];
                 pair64<POT>(p.x - t.x, p.y - t.y, r.x - t.z, r.y, pr.eps2, a);
             }
             if (!sums_finite<POT>(a)) {
                 a[0] = a[1] = a[2] = a[3] = 0.0;
-                for (int q = part; q < n; q += G) {
+                for (int q = part; q < n; q += pa.G) {
                     if (SELF && q == self_q) continue;
                     const double2 p = st.xy[q], r = st.zm[q];
                     pair64_exact<POT>(p.x - t.x, p.y - t.y, r.x - t.z, r.y, pr.eps2, a);
@@ -226,7 +251,7 @@ struct Near64 {
             }
         } else {
             static_assert(KM == 1, "the plain form corrects the far field in k_soft_correct");
-            for (int q = part; q < n; q += G) {
+            for (int q = part; q < n; q += pa.G) {
                 if (SELF && q == self_q) continue;
                 const double2 p = st.xy[q], r = st.zm[q];
                 const double dx = p.x - t.x, dy = p.y - t.y, dz = r.x - t.z;
@@ -249,7 +274,7 @@ struct Near64 {
 // body i, FP64.  The kernel needs only the tree and the lists, so in the mixed form it runs
 // beside the far-field chain.
 template <class N, bool POT, int NU, int KM = 0>
-__global__ void __launch_bounds__(32, sizeof(typename N::T) == 4 ? NEAR_MINB : 20)
+__global__ void __launch_bounds__(32, sizeof(typename N::T) == 4 ? 28 : 20)
     k_leaf_near(TreeView tv, const int64_t* __restrict__ chunk_off, typename N::Bodies bod, NearPrm<typename N::T> pr,
                 double* __restrict__ near) {
     constexpr int R = NU / 32;
@@ -276,6 +301,7 @@ __global__ void __launch_bounds__(32, sizeof(typename N::T) == 4 ? NEAR_MINB : 2
         const int T = min(32, cnt - j0);
         const int G = near_parts<NU>(T);
         const int U = T * G;
+        const Parts pa(G);
         // the lane's units: target tt[r] (index in the leaf), source part pp[r]
         int tt[R], pp[R];
         bool act[R];
@@ -294,12 +320,12 @@ __global__ void __launch_bounds__(32, sizeof(typename N::T) == 4 ? NEAR_MINB : 2
         for (int k0 = 0; k0 < (KM == 2 ? 0 : cnt); k0 += NEAR_CAP) {
             const int n = min(NEAR_CAP, cnt - k0);
             __syncwarp();
-            for (int q = lane; q < n; q += 32) N::put(st, bod, q, f0 + k0 + q);
-            N::pad(st, n, lane);
+            for (int q = lane; q < n; q += 32) N::put(st, pa, bod, q, f0 + k0 + q);
+            N::pad(st, pa, n, lane);
             __syncwarp();
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (act[r]) N::template round<true, POT, KM>(st, pp[r], G, n, j0 + tt[r] - k0, tg[r], pr, acc[r]);
+                if (act[r]) N::template round<true, POT, KM>(st, pa, pp[r], n, j0 + tt[r] - k0, tg[r], pr, acc[r]);
         }
         // the other U-list entries, 32 at a time: lane e holds entry e's first body and
         // count; an inclusive scan of the counts maps a flat source position to its entry
@@ -332,13 +358,13 @@ __global__ void __launch_bounds__(32, sizeof(typename N::T) == 4 ? NEAR_MINB : 2
                         if (__shfl_sync(0xffffffffu, pre, pos + step - 1) <= f) pos += step;
                     const int ep = __shfl_sync(0xffffffffu, pre, pos), ec = __shfl_sync(0xffffffffu, pc, pos);
                     const int j = __shfl_sync(0xffffffffu, pf, pos) + f - (ep - ec);
-                    if (q < n) N::put(st, bod, q, j);
+                    if (q < n) N::put(st, pa, bod, q, j);
                 }
-                N::pad(st, n, lane);
+                N::pad(st, pa, n, lane);
                 __syncwarp();
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    if (act[r]) N::template round<false, POT, KM>(st, pp[r], G, n, -1, tg[r], pr, acc[r]);
+                    if (act[r]) N::template round<false, POT, KM>(st, pa, pp[r], n, -1, tg[r], pr, acc[r]);
             }
         }
         // the parts of every target, in part order, in FP64
