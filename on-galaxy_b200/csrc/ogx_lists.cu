@@ -141,6 +141,12 @@ __global__ void __launch_bounds__(128) k_uw_warp(int nleaf, const int* __restric
                                                  int* widx, uint32_t* xkey, uint32_t* xval, int* xcnt, DevCounts* counts) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int lf = blockIdx.x * 4 + wid;
+    __shared__ unsigned long long s_tot[2];
+    if (!FILL) {
+        if (threadIdx.x < 2) s_tot[threadIdx.x] = 0;
+        __syncthreads();
+    }
+    auto leaf_lists = [&]() {
     if (lf >= nleaf || lf >= counts->nleaf32 || counts->overflow) return;
     const int b = leafbox[lf];
     const double tol = root->tol;
@@ -237,14 +243,24 @@ __global__ void __launch_bounds__(128) k_uw_warp(int nleaf, const int* __restric
             tp += __shfl_xor_sync(FULL, tp, o);
         }
         const bool any_over = __any_sync(FULL, overflow);
+        // totals: one addition per block (one per leaf to the same words took 70 us on the 1M merger)
         if (lane == 0) {
             ucnt[lf] = tu;
             wcnt[lf] = tw;
-            const int64_t pb = pcount[b];
-            atomicAdd((unsigned long long*)&counts->p2p_pairs, (unsigned long long)(pb * tp - pb));
-            atomicAdd((unsigned long long*)&counts->m2p_evals, (unsigned long long)(pb * tw));
-            atomicAdd((unsigned long long*)&counts->p2l_evals, (unsigned long long)(pb * tw));
+            const unsigned long long pb = (unsigned long long)pcount[b];
+            atomicAdd(&s_tot[0], pb * (unsigned long long)tp - pb);
+            atomicAdd(&s_tot[1], pb * (unsigned long long)tw);
             if (any_over) atomicAdd((unsigned long long*)&counts->adj_mismatch, 1ull << 40);
+        }
+    }
+    };
+    leaf_lists();
+    if (!FILL) {
+        __syncthreads();
+        if (threadIdx.x == 0 && s_tot[0] + s_tot[1] > 0) {
+            atomicAdd((unsigned long long*)&counts->p2p_pairs, s_tot[0]);
+            atomicAdd((unsigned long long*)&counts->m2p_evals, s_tot[1]);
+            atomicAdd((unsigned long long*)&counts->p2l_evals, s_tot[1]);
         }
     }
 }
@@ -388,50 +404,76 @@ inline int bits_for(int64_t v) {
 // Adjacency is the U-list predicate (AdaptiveOctree::adjacent, same FP64 operations), so
 // every leaf pair is either in b's U list or a candidate here.  Thread per leaf; pass 1
 // counts, pass 2 writes in the same order.
-constexpr int kSoftStack = 8 * (kMaxDepth + 2);   // > 7 per level + 8: the walk never overflows it
+//
+// Warp per leaf: the 32 boxes on top of a stack in shared memory are tested together, their
+// children pushed, so a walk takes a dozen rounds of loads (a thread per leaf took one box
+// after another, 24 blocks' worth of threads for the 50k merger, 200 us a pass).  A round
+// takes at most 32 boxes and pushes at most 256, and what it pushes is taken first, so at
+// most 224 boxes wait per level.
+constexpr int kSoftStack = 256 * (kMaxDepth + 1);
+constexpr int kSoftSmem = 2 * kSoftStack * (int)sizeof(int);   // two warps per block
 template <bool EMIT>
-__global__ void __launch_bounds__(128) k_soft_lists(int nleaf, const int* __restrict__ leafbox, const int* __restrict__ child,
-                                                    const int* __restrict__ leafid, const double* __restrict__ ctr,
-                                                    const RootInfo* __restrict__ root, double hs, int* cnt,
-                                                    const int64_t* __restrict__ off, int* idx, const DevCounts* counts) {
-    const int lf = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(64) k_soft_lists(int nleaf, const int* __restrict__ leafbox, const int* __restrict__ child,
+                                                   const int* __restrict__ leafid, const double* __restrict__ ctr,
+                                                   const RootInfo* __restrict__ root, double hs, int* cnt,
+                                                   const int64_t* __restrict__ off, int* idx, const DevCounts* counts) {
+    extern __shared__ int s_soft[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lf = blockIdx.x * 2 + wid;
     if (lf >= nleaf) return;
     if (lf >= counts->nleaf32 || counts->overflow) {
-        if (!EMIT) cnt[lf] = 0;
+        if (!EMIT && lane == 0) cnt[lf] = 0;
         return;
     }
+    int* stack = s_soft + wid * kSoftStack;
     const int b = leafbox[lf];
     const double tol = root->tol;
     const double bx = ctr[4 * b], by = ctr[4 * b + 1], bz = ctr[4 * b + 2], bh = ctr[4 * b + 3];
     const double hs2 = hs * hs;
-    int stack[kSoftStack];
-    int sp = 0, n = 0;
+    const unsigned lt = (1u << lane) - 1u;
+    int sp = 1, n = 0;
     const int64_t o = EMIT ? off[lf] : 0;
-    stack[sp++] = 0;   // the root
+    if (lane == 0) stack[0] = 0;   // the root
+    __syncwarp();
     while (sp > 0) {
-        const int c = stack[--sp];
-        const double ch = ctr[4 * c + 3];
-        // gap between the two boxes along each axis (0 where they overlap)
-        const double gx = fmax(0.0, fabs(ctr[4 * c] - bx) - (ch + bh));
-        const double gy = fmax(0.0, fabs(ctr[4 * c + 1] - by) - (ch + bh));
-        const double gz = fmax(0.0, fabs(ctr[4 * c + 2] - bz) - (ch + bh));
-        if (gx * gx + gy * gy + gz * gz >= hs2) continue;
-        if (leafid[c] >= 0) {
+        const int take = min(32, sp);
+        const int c = lane < take ? stack[sp - 1 - lane] : -1;
+        __syncwarp();   // read before the pushes below overwrite
+        sp -= take;
+        int leaf = -1;
+        int4 k0 = make_int4(-1, -1, -1, -1), k1 = k0;
+        bool in = false, adj = false;
+        if (c >= 0) {
+            const double2 c01 = __ldg(reinterpret_cast<const double2*>(ctr) + 2 * (size_t)c);
+            const double2 c23 = __ldg(reinterpret_cast<const double2*>(ctr) + 2 * (size_t)c + 1);
+            leaf = __ldg(leafid + c);
+            k0 = __ldg(reinterpret_cast<const int4*>(child + 8 * (size_t)c));
+            k1 = __ldg(reinterpret_cast<const int4*>(child + 8 * (size_t)c) + 1);
+            const double ch = c23.y;
+            // gap between the two boxes along each axis (0 where they overlap)
+            const double gx = fmax(0.0, fabs(c01.x - bx) - (ch + bh));
+            const double gy = fmax(0.0, fabs(c01.y - by) - (ch + bh));
+            const double gz = fmax(0.0, fabs(c23.x - bz) - (ch + bh));
+            in = !(gx * gx + gy * gy + gz * gz >= hs2);
             const double lim = __dadd_rn(__dadd_rn(ch, bh), tol);
-            const bool adj = fabs(__dsub_rn(ctr[4 * c], bx)) <= lim && fabs(__dsub_rn(ctr[4 * c + 1], by)) <= lim &&
-                             fabs(__dsub_rn(ctr[4 * c + 2], bz)) <= lim;
-            if (!adj) {
-                if (EMIT) idx[o + n] = c;
-                ++n;
-            }
-        } else {
-            for (int s = 7; s >= 0; --s) {
-                const int k = child[8 * c + s];
-                if (k >= 0 && sp < kSoftStack) stack[sp++] = k;
-            }
+            adj = fabs(__dsub_rn(c01.x, bx)) <= lim && fabs(__dsub_rn(c01.y, by)) <= lim && fabs(__dsub_rn(c23.x, bz)) <= lim;
         }
+        const bool found = in && leaf >= 0 && !adj;
+        const unsigned mf = __ballot_sync(FULL, found);
+        if (EMIT && found) idx[o + n + __popc(mf & lt)] = c;
+        n += __popc(mf);
+        const bool open = in && leaf < 0;
+        const int kid[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const bool push = open && kid[s] >= 0;
+            const unsigned m = __ballot_sync(FULL, push);
+            if (push) stack[sp + __popc(m & lt)] = kid[s];
+            sp += __popc(m);
+        }
+        __syncwarp();
     }
-    if (!EMIT) cnt[lf] = n;
+    if (!EMIT && lane == 0) cnt[lf] = n;
 }
 
 }  // namespace
@@ -446,7 +488,9 @@ int soft_lists_build(Handle& h) {
     OGX_TRY(arena_get(h.ws, S_SOFT_CNT, nleaf, &cnt));
     OGX_TRY(arena_get(h.ws, S_SOFT_OFF, nleaf + 1, &off));
     const double hs = spline_support(h.prm.eps);
-    k_soft_lists<false><<<grid_for(nleaf, 128), 128, 0, st>>>(nleaf, tv.leafbox, tv.child, tv.leafid, tv.center, tv.root, hs,
+    OGX_CUDA(smem_optin((const void*)k_soft_lists<false>, kSoftSmem));
+    OGX_CUDA(smem_optin((const void*)k_soft_lists<true>, kSoftSmem));
+    k_soft_lists<false><<<grid_for(nleaf, 2), 64, kSoftSmem, st>>>(nleaf, tv.leafbox, tv.child, tv.leafid, tv.center, tv.root, hs,
                                                               cnt, nullptr, nullptr, h.d_counts); ++h.launches;
     OGX_TRY(scan_i32_to_i64(h, cnt, off, nleaf));
     int64_t ns = 0;
@@ -454,7 +498,7 @@ int soft_lists_build(Handle& h) {
     OGX_CUDA(cudaStreamSynchronize(st));
     int* idx;
     OGX_TRY(arena_get(h.ws, S_SOFT_IDX, ns + 1, &idx));
-    k_soft_lists<true><<<grid_for(nleaf, 128), 128, 0, st>>>(nleaf, tv.leafbox, tv.child, tv.leafid, tv.center, tv.root, hs,
+    k_soft_lists<true><<<grid_for(nleaf, 2), 64, kSoftSmem, st>>>(nleaf, tv.leafbox, tv.child, tv.leafid, tv.center, tv.root, hs,
                                                              nullptr, off, idx, h.d_counts); ++h.launches;
     tv.s_off = off;
     tv.s_idx = idx;

@@ -13,27 +13,43 @@
 
 namespace ogx {
 
+// the spline inside the support, u = r / h in [0, 1), iu = 1 / u (read from u = 1/2 on)
 template <class T>
-__device__ __forceinline__ void spline_gk(T r2, T h, T hinv, T& g, T& k) {
-    if (r2 >= h * h) {
-        T y;
-        if constexpr (sizeof(T) == 4) y = rsqrtf(r2); else y = rsqrt(r2);
-        g = y * y * y;
-        k = y;
-        return;
-    }
-    T r;
-    if constexpr (sizeof(T) == 4) r = sqrtf(r2); else r = sqrt(r2);
-    const T u = r * hinv;
+__device__ __forceinline__ void spline_inside(T u, T iu, T hinv, T& g, T& k) {
     const T u2 = u * u;
     const T hinv3 = hinv * hinv * hinv;
     if (u < T(0.5)) {
         g = hinv3 * (T(32.0 / 3.0) + u2 * (T(32.0) * u - T(38.4)));
         k = hinv * (T(2.8) - u2 * (T(16.0 / 3.0) + u2 * (T(6.4) * u - T(9.6))));
     } else {
-        const T iu = T(1) / u;
         g = hinv3 * (T(64.0 / 3.0) - T(48.0) * u + T(38.4) * u2 - T(32.0 / 3.0) * u2 * u - T(1.0 / 15.0) * iu * iu * iu);
         k = hinv * (T(3.2) - T(1.0 / 15.0) * iu - u2 * (T(32.0 / 3.0) + u * (T(-16.0) + u * (T(9.6) - T(32.0 / 15.0) * u))));
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void spline_gk(T r2, T h, T hinv, T& g, T& k) {
+    // FP32: 1/r from rsqrtf and one Newton step gives r = r2 / r and 1/u = h / r without the
+    // square root and the division (a third of the pair)
+    if constexpr (sizeof(T) == 4) {
+        T y = rsqrtf(r2);
+        if (r2 >= h * h) {
+            g = y * y * y;
+            k = y;
+            return;
+        }
+        y = fmaf(y, T(0.5) * fmaf(-r2 * y, y, T(1)), y);
+        const T r = r2 > T(0) ? r2 * y : T(0);
+        spline_inside<T>(r * hinv, h * y, hinv, g, k);
+    } else {
+        if (r2 >= h * h) {
+            const T y = rsqrt(r2);
+            g = y * y * y;
+            k = y;
+            return;
+        }
+        const T u = sqrt(r2) * hinv;
+        spline_inside<T>(u, T(1) / u, hinv, g, k);
     }
 }
 
