@@ -14,11 +14,16 @@
 #include <vector>
 
 #include "ogx_m2l64.cuh"
+#include "ogx_sm100.cuh"
 
 namespace ogx {
 namespace {
 
 constexpr int ROT_TGT = M2L64_TGT;   // targets per CTA
+
+__device__ __forceinline__ void cp_async8_zfill(void* sdst, const void* gsrc, uint32_t valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sm100::smem_u32(sdst)), "l"(gsrc), "r"(valid) : "memory");
+}
 
 // ---- M2L by rotations (the third form) ------------------------------------------------
 // T_o = Q_o^-1 Z_|o| Q_o (build_rot_pack): per tile of ROT_TGT targets sharing octant t
@@ -39,7 +44,12 @@ struct RotCfg {
     static constexpr int QSZ = (P + 1) * (2 * P + 1) * (2 * P + 3) / 3;   // sum_n (2n+1)^2
     static constexpr int ZSZ = (P + 1) * (P + 2) * (2 * P + 3) / 6;       // sum_m (P+1-m)^2
     static constexpr int PACK = 2 * QSZ + ZSZ;
-    static constexpr size_t SMEM = (size_t)2 * ROT_TGT * LD * sizeof(double);
+    // the device's packs: Q_o, Q_o^-1 and Z, each from a 16-byte boundary
+    static constexpr int QS = (QSZ + 1) / 2 * 2, ZS = (ZSZ + 1) / 2 * 2, DPACK = 2 * QS + ZS;
+    static constexpr size_t ROWS_BYTES = (size_t)2 * ROT_TGT * LD * sizeof(double);
+    // factors staged in shared memory where they fit beside the rows (p <= 11)
+    static constexpr bool STAGE = ROWS_BYTES + DPACK * sizeof(double) <= 212 * 1024;
+    static constexpr size_t SMEM = ROWS_BYTES + (STAGE ? DPACK * sizeof(double) : 0);
     // rows per thread: each factor entry loaded feeds RB FMAs (2 where the registers allow)
     static constexpr int RB = P <= 10 ? 2 : 1;
     static constexpr int ROWS = ROT_TGT / RB;          // threads of one block group
@@ -74,7 +84,7 @@ struct RotCfg {
 
 // stage A (FWD) or C (!FWD) for degree block N: rows N^2 .. N^2 + 2N of source a
 template <int P, int N, bool FWD>
-__device__ __forceinline__ void rot_deg_block(const double* __restrict__ F, const double* x_in, double* y_out,
+__device__ __forceinline__ void rot_deg_block(const double* F, const double* x_in, double* y_out,
                                               double (&acc)[RotCfg<P>::RB][RotCfg<P>::NACC]) {
     constexpr int w = 2 * N + 1, off = N * (2 * N - 1) * (2 * N + 1) / 3, pos = RotCfg<P>::deg_pos(N);
     constexpr int RB = RotCfg<P>::RB, RS = RotCfg<P>::ROWS * RotCfg<P>::LD;   // row stride of the RB rows
@@ -90,7 +100,7 @@ __device__ __forceinline__ void rot_deg_block(const double* __restrict__ F, cons
         for (int q = 0; q < RB; ++q) v[q] = FWD ? 0.0 : acc[q][pos + r];
 #pragma unroll
         for (int c = 0; c < w; ++c) {
-            const double f = __ldg(F + off + r * w + c);
+            const double f = RotCfg<P>::STAGE ? F[off + r * w + c] : __ldg(F + off + r * w + c);
 #pragma unroll
             for (int q = 0; q < RB; ++q) v[q] = fma(f, x[q][c], v[q]);
         }
@@ -104,7 +114,7 @@ __device__ __forceinline__ void rot_deg_block(const double* __restrict__ F, cons
 
 // stage B for order block M: z = Z_M y over degrees M..P, re and im parts
 template <int P, int M>
-__device__ __forceinline__ void rot_ord_block(const double* __restrict__ Z, const double* y_in, double* z_out) {
+__device__ __forceinline__ void rot_ord_block(const double* Z, const double* y_in, double* z_out) {
     constexpr int L = P + 1 - M;
     constexpr int zoff = RotCfg<P>::ZSZ - L * (L + 1) * (2 * L + 1) / 6;
     constexpr int NP = M == 0 ? 1 : 2;                      // parts re, im: same block
@@ -124,7 +134,7 @@ __device__ __forceinline__ void rot_ord_block(const double* __restrict__ Z, cons
         for (int q = 0; q < RB * NP; ++q) v[q] = 0.0;
 #pragma unroll
         for (int d = 0; d < L; ++d) {
-            const double f = __ldg(Z + zoff + jr * L + d);
+            const double f = RotCfg<P>::STAGE ? Z[zoff + jr * L + d] : __ldg(Z + zoff + jr * L + d);
 #pragma unroll
             for (int q = 0; q < RB * NP; ++q) v[q] = fma(f, yv[q][d], v[q]);
         }
@@ -149,19 +159,26 @@ __device__ __forceinline__ void rot_ord_stage(std::integer_sequence<int, Ms...>,
 
 // Work items and split sums as in the plain form (ogx_m2l64.cuh): a small tree's tiles are
 // cut into ranges of colleague slots so that they fill the SMs.
+// Bound: a combination's 64 rows take 2,223 FMAs each at p = 8, 2,200 cycles of the SM's FP64
+// pipe; reading every factor and every source row from L2 at the point of use took about ten
+// times that.  The next combination's factors and sources now come by cp.async while this one
+// runs: its Q once stage A is done with this one's, its Z and its rows (into the buffer that
+// stage C does not read) once stage B is, its Q^-1 after stage C.
 template <int P>
 __global__ void __launch_bounds__(RotCfg<P>::THREADS) k_m2l_rot(TreeView tv, M2L64Args ar, const double* __restrict__ pack,
                                                         const double* __restrict__ mpole, double* lown) {
     using R = RotCfg<P>;
     constexpr int K = R::K, LD = R::LD, RB = R::RB, TH = R::THREADS;
-    extern __shared__ double s_rot[];
-    double* s_m = s_rot;                    // [64][LD] sources, later z
-    double* s_y = s_rot + ROT_TGT * LD;     // [64][LD] y = Q m
-    __shared__ int s_pcol[27][ROT_TGT];
-    __shared__ int s_src[ROT_TGT];
+    extern __shared__ __align__(16) double s_rot[];
+    double* s_x = s_rot;                    // [64][LD] sources, then z
+    double* s_y = s_rot + ROT_TGT * LD;     // [64][LD] y = Q m, then the next sources
+    double* s_f = s_rot + 2 * ROT_TGT * LD; // factors (STAGE): Q, Q^-1, Z
+    __shared__ int s_Q[27][ROT_TGT];
+    __shared__ uint32_t s_mask[7];          // bit 8 D + s: some target of the tile has that source
+    __shared__ int s_combo[189];            // present combinations: D | s << 5 | o << 8
     __shared__ int s_tgt[ROT_TGT];
-    __shared__ int s_item;
-    const int tid = threadIdx.x;
+    __shared__ int s_item, s_n;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int ga = tid / R::ROWS, ra = tid % R::ROWS;   // block group; rows ra, ra + ROWS, ...
     if (tv_over(tv)) return;
     const int S = ar.gs[GS_SPLIT], tiles = ar.gs[GS_TILES];
@@ -169,6 +186,7 @@ __global__ void __launch_bounds__(RotCfg<P>::THREADS) k_m2l_rot(TreeView tv, M2L
     for (;;) {
         __syncthreads();
         if (tid == 0) s_item = atomicAdd(ar.gs + GS_TICKET, 1);
+        if (tid < 7) s_mask[tid] = 0;
         __syncthreads();
         const int item = s_item;
         if (item >= tiles * S) return;
@@ -178,45 +196,95 @@ __global__ void __launch_bounds__(RotCfg<P>::THREADS) k_m2l_rot(TreeView tv, M2L
         const int D0 = m2l64_first_slot(zr, S, t), D1 = m2l64_first_slot(zr + 1, S, t);
         if (tid < ROT_TGT) s_tgt[tid] = ((int)ar.tgt_key[base + tid] == t) ? (int)ar.tgt_box[base + tid] : -1;
         __syncthreads();
+        const int tx = t & 1, ty = (t >> 1) & 1, tz = (t >> 2) & 1;
         for (int i = tid; i < (D1 - D0) * ROT_TGT; i += TH) {
             const int D = D0 + i / ROT_TGT, r = i % ROT_TGT, b = s_tgt[r];
-            s_pcol[D][r] = b >= 0 ? tv.col[27 * (size_t)tv.parent[b] + D] : -1;
+            const int Q = b >= 0 ? tv.col[27 * (size_t)tv.parent[b] + D] : -1;
+            s_Q[D][r] = Q;
+            uint32_t bits = 0;
+            if (Q >= 0) {
+                const int4 c0 = __ldg(reinterpret_cast<const int4*>(tv.child + 8 * (size_t)Q));
+                const int4 c1 = __ldg(reinterpret_cast<const int4*>(tv.child + 8 * (size_t)Q) + 1);
+                const int ch[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+                const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
+                    if (ch[s] >= 0 && max(abs(ox), max(abs(oy), abs(oz))) > 1) bits |= 1u << s;
+                }
+            }
+            bits = __reduce_or_sync(0xffffffffu, bits);   // whole warps share a slot
+            if (lane == 0 && bits) atomicOr(&s_mask[D >> 2], bits << (8 * (D & 3)));
         }
         __syncthreads();
-        const int tx = t & 1, ty = (t >> 1) & 1, tz = (t >> 2) & 1;
+        if (tid < 32) {   // the present combinations in (D, s) order
+            int n = 0;
+            for (int w = 0; w < 7; ++w) {
+                const uint32_t m = s_mask[w];
+                if (m >> lane & 1) {
+                    const int c = 32 * w + lane, D = c >> 3, s = c & 7;
+                    const int ox = 2 * (D % 3 - 1) + (s & 1) - tx, oy = 2 * ((D / 3) % 3 - 1) + ((s >> 1) & 1) - ty,
+                              oz = 2 * (D / 9 - 1) + ((s >> 2) & 1) - tz;
+                    s_combo[n + __popc(m & ((1u << lane) - 1u))] = D | (s << 5) | (((ox + 3) + 7 * (oy + 3) + 49 * (oz + 3)) << 8);
+                }
+                n += __popc(m);
+            }
+            if (lane == 0) s_n = n;
+        }
+        __syncthreads();
+        const int nco = s_n;
+        // copies of combination k's factors [f0, f0 + count) and of its source rows (absent: zeros)
+        auto factors = [&](int k, int f0, int count) {
+            if (!R::STAGE || k >= nco) return;
+            const double* src = pack + (size_t)(s_combo[k] >> 8) * R::DPACK + f0;
+            for (int i = tid; i < count / 2; i += TH) sm100::cp_async16(s_f + f0 + 2 * i, src + 2 * i);
+        };
+        auto rows = [&](int k, double* dst) {
+            if (k >= nco) return;
+            const int code = s_combo[k], lr = tid / (TH / ROT_TGT);   // TH / 64 threads per row
+            const int Q = s_Q[code & 31][lr];
+            const int b = Q >= 0 ? __ldg(tv.child + 8 * (size_t)Q + ((code >> 5) & 7)) : -1;
+            const double* src = mpole + (size_t)max(b, 0) * K;
+            for (int kk = tid % (TH / ROT_TGT); kk < K; kk += TH / ROT_TGT)
+                cp_async8_zfill(dst + lr * LD + kk, src + kk, b >= 0 ? 8u : 0u);
+        };
         double acc[RB][R::NACC];
 #pragma unroll
         for (int q = 0; q < RB; ++q)
 #pragma unroll
             for (int i = 0; i < R::NACC; ++i) acc[q][i] = 0.0;
         using Seq = std::make_integer_sequence<int, P + 1>;
-        for (int D = D0; D < D1; ++D) {
-            const int Dx = D % 3 - 1, Dy = (D / 3) % 3 - 1, Dz = D / 9 - 1;
-            for (int s = 0; s < 8; ++s) {
-                const int ox = 2 * Dx + (s & 1) - tx, oy = 2 * Dy + ((s >> 1) & 1) - ty, oz = 2 * Dz + ((s >> 2) & 1) - tz;
-                if (max(abs(ox), max(abs(oy), abs(oz))) <= 1) continue;  // adjacent: not in V
-                int mysrc = -1;
-                if (tid < ROT_TGT) {
-                    const int Q = s_pcol[D][tid];
-                    mysrc = (Q >= 0) ? tv.child[8 * Q + s] : -1;
-                    s_src[tid] = mysrc;
-                }
-                if (!__syncthreads_or(mysrc >= 0)) continue;
-                for (int idx = tid; idx < ROT_TGT * K; idx += TH) {
-                    const int r = idx / K, kk = idx - r * K;
-                    const int src = s_src[r];
-                    s_m[r * LD + kk] = (src >= 0) ? mpole[(size_t)src * K + kk] : 0.0;
-                }
-                __syncthreads();
-                const double* pk = pack + (size_t)((ox + 3) + 7 * (oy + 3) + 49 * (oz + 3)) * R::PACK;
-                rot_deg_stage<P, true>(Seq{}, ga, pk, s_m + ra * LD, s_y + ra * LD, acc);              // y = Q m
-                __syncthreads();
-                rot_ord_stage<P>(Seq{}, ga, pk + 2 * R::QSZ, s_y + ra * LD, s_m + ra * LD);            // z = Z y
-                __syncthreads();
-                rot_deg_stage<P, false>(Seq{}, ga, pk + R::QSZ, s_m + ra * LD, nullptr, acc);          // acc += Q^-1 z
-                __syncthreads();
-            }
+        double *x = s_x, *y = s_y;
+        factors(0, 0, R::QS);
+        factors(0, 2 * R::QS, R::ZS);
+        rows(0, x);
+        sm100::cp_async_commit();
+        sm100::cp_async_wait<0>();
+        __syncthreads();
+        factors(0, R::QS, R::QS);
+        sm100::cp_async_commit();
+        for (int k = 0; k < nco; ++k) {
+            const double* pk = R::STAGE ? s_f : pack + (size_t)(s_combo[k] >> 8) * R::DPACK;
+            rot_deg_stage<P, true>(Seq{}, ga, pk, x + ra * LD, y + ra * LD, acc);              // y = Q m
+            __syncthreads();
+            factors(k + 1, 0, R::QS);
+            sm100::cp_async_commit();
+            rot_ord_stage<P>(Seq{}, ga, pk + 2 * R::QS, y + ra * LD, x + ra * LD);            // z = Z y
+            sm100::cp_async_wait<1>();                                                       // this combination's Q^-1
+            __syncthreads();
+            factors(k + 1, 2 * R::QS, R::ZS);
+            rows(k + 1, y);
+            sm100::cp_async_commit();
+            rot_deg_stage<P, false>(Seq{}, ga, pk + R::QS, x + ra * LD, nullptr, acc);         // acc += Q^-1 z
+            sm100::cp_async_wait<0>();
+            __syncthreads();
+            factors(k + 1, R::QS, R::QS);
+            sm100::cp_async_commit();
+            double* w = x;
+            x = y;
+            y = w;
         }
+        sm100::cp_async_wait_all();
 #pragma unroll
         for (int q = 0; q < RB; ++q) {
             const int r0 = ra + q * R::ROWS, b = s_tgt[r0];
@@ -243,8 +311,17 @@ std::shared_ptr<const std::vector<double>> rot_packs() {
     static std::shared_ptr<const std::vector<double>> cached;
     std::lock_guard<std::mutex> lk(mu);
     if (cached) return cached;
-    auto v = std::make_shared<std::vector<double>>((size_t)343 * RotCfg<P>::PACK, 0.0);
-    for (int o = 0; o < 343; ++o) build_rot_pack(P, o, v->data() + (size_t)o * RotCfg<P>::PACK);
+    using R = RotCfg<P>;
+    auto v = std::make_shared<std::vector<double>>((size_t)343 * R::DPACK, 0.0);
+    std::vector<double> pk(R::PACK);
+    for (int o = 0; o < 343; ++o) {
+        std::fill(pk.begin(), pk.end(), 0.0);
+        build_rot_pack(P, o, pk.data());
+        double* d = v->data() + (size_t)o * R::DPACK;
+        std::copy(pk.begin(), pk.begin() + R::QSZ, d);
+        std::copy(pk.begin() + R::QSZ, pk.begin() + 2 * R::QSZ, d + R::QS);
+        std::copy(pk.begin() + 2 * R::QSZ, pk.end(), d + 2 * R::QS);
+    }
     cached = v;
     return cached;
 }
