@@ -40,10 +40,11 @@ int Arena::get(Slot s, size_t bytes, void** out) {
             ptr[s] = nullptr;
             cap[s] = 0;
         }
-        // operator tables keep their size; everything else may grow with the next system
+        // operator tables keep their size; everything else may grow with the next system (the
+        // M2L's partial rows, a generous bound, by less)
         const bool table = s == S_OPS_M2L || s == S_OPS_M2M || s == S_OPS_L2L || s == S_MIX_TOPS || s == S_MIX_ROW0 ||
                            s == S_ROT_PACK;
-        size_t nb = table ? bytes : bytes + bytes / 4;
+        size_t nb = table ? bytes : bytes + bytes / (s == S_M2L_PART ? 8 : 4);
         nb = (nb + 255) & ~(size_t)255;
         const cudaError_t e = cudaMalloc(&ptr[s], nb);
         if (e != cudaSuccess) {

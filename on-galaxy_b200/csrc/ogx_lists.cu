@@ -349,6 +349,7 @@ __global__ void k_target_groups(const uint32_t* key, const DevCounts* counts, in
             tiles128 += (lo_s[q + 1] - lo_s[q] + 127) / 128;
         }
         gs[GS_TILES128] = tiles128;
+        for (int sl = 1; sl <= 3; ++sl) gs[GS_TC_SPLIT + sl - 1] = m2l_tc_split(tiles128, sl);
         gs[GS_SPLIT] = max(1, min(M2L64_MAXSPLIT, (M2L64_ITEMS + tiles64 - 1) / max(tiles64, 1)));
         gs[GS_TILES] = pad / M2L64_TGT;
         gs[GS_TICKET] = 0;

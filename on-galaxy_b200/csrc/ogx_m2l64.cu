@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(M64<P>::THREADS, M64<P>::MINB)
 
 // Lown of every target = its ranges' sums in range order / side (split above 1)
 __global__ void __launch_bounds__(256) k_m2l64_sum(TreeView tv, M2L64Args ar, int K, int slices, double* __restrict__ lown) {
-    const int S = slices > 0 ? m2l_tc_split(ar.gs[GS_TILES128], slices) : ar.gs[GS_SPLIT];
+    const int S = ar.gs[slices > 0 ? GS_TC_SPLIT + slices - 1 : GS_SPLIT];
     if (tv_over(tv) || S == 1) return;
     const int ntgt = tv.cnt->ntgt32;
     const int64_t total = (int64_t)ntgt * K;

@@ -12,10 +12,10 @@
 namespace ogx {
 
 constexpr int M2L64_TGT = 64;        // targets per tile; the target layout is padded to 128
-constexpr int M2L64_ITEMS = 1184;    // items wanted: 4 per CTA slot of 2 x 148
+constexpr int M2L64_ITEMS = 888;     // items wanted: 3 per CTA slot of 2 x 148 (2.5: 0.2 ms more of tail at 262,144 bodies)
 constexpr int M2L64_MAXSPLIT = 27;
 // k_target_groups' words behind the group starts gs[0..17]
-constexpr int GS_SPLIT = 18, GS_TILES = 19, GS_TICKET = 20, GS_FILL = 21, GS_TILES128 = 22;
+constexpr int GS_SPLIT = 18, GS_TILES = 19, GS_TICKET = 20, GS_FILL = 21, GS_TILES128 = 22, GS_TC_SPLIT = 23 /* for 1, 2, 3 slices */;
 
 // V children that slot D offers a target of octant t: the 8 children less the adjacent ones
 __host__ __device__ __forceinline__ int m2l64_slot_count(int D, int t) {

@@ -195,7 +195,8 @@ __global__ void __launch_bounds__(TcCfg<P>::THREADS, 1)
     const uint32_t* __restrict__ tgt_box = ar.tgt_box;
     if (tv_over(tv)) return;
     // this CTA's ranges of colleague slots: [zlo, zhi) of the S ranges (any grid z is correct)
-    const int S = m2l_tc_split(ar.gs[GS_TILES128], C::NSPLIT);
+    static_assert(C::NSPLIT <= 3, "k_target_groups writes the split for up to three slices");
+    const int S = ar.gs[GS_TC_SPLIT + C::NSPLIT - 1];
     const int zlo = S * (int)blockIdx.z / (int)gridDim.z, zhi = S * ((int)blockIdx.z + 1) / (int)gridDim.z;
     if (zlo == zhi) return;
     if (tid == 0) {

@@ -47,25 +47,32 @@ constexpr int NEAR_CAP = 128;    // source bodies staged per round (several U-li
 // the busy fraction T G / (32 R) (ties: the smaller G).  With NU = 64 a 17-body leaf
 // gets G = 3 (80% busy; one target per lane would leave 47% of the lanes idle), a
 // 5-body leaf G = 6 (94%).
-template <int NU>
-__device__ __forceinline__ int near_parts(int T) {
-    int best = 1, bu = 0;
-    for (int G = 1; G <= 32 && T * G <= NU; ++G) {
-        const int U = T * G;
-        const int u = (U << 10) / (32 * ((U + 31) >> 5));   // busy fraction, fixed point
-        if (u > bu) { bu = u; best = G; }
+struct PartTable {
+    unsigned char g[2][33];   // [units 32, 64][targets]
+    constexpr PartTable() : g() {
+        for (int w = 0; w < 2; ++w)
+            for (int T = 1; T <= 32; ++T) {
+                int best = 1, bu = 0;
+                for (int G = 1; G <= 32 && T * G <= 32 * (w + 1); ++G) {
+                    const int U = T * G;
+                    const int u = (U << 10) / (32 * ((U + 31) >> 5));   // busy fraction, fixed point
+                    if (u > bu) { bu = u; best = G; }
+                }
+                g[w][T] = (unsigned char)best;
+            }
     }
-    return best;
-}
+};
+static __constant__ const PartTable c_parts{};
 
 // KM (kernel): 0 Plummer's (eps2); 1 the spline of support hs (ogx_softening.cuh);
 // 2 (FP32) the spline minus the Newtonian kernel, zero from hs on (the far field's pairs
 // inside the support, OGX_SOFT_SPLINE)
-// The G parts of a staged round: part p holds sources p, p + G, ...; S slots per part
+// The G parts of a staged round: part p holds sources p, p + G, ...; S slots per part (4 mod 8,
+// so that the 16-byte loads of up to eight parts meet different banks)
 struct Parts {
     int G, S;
     unsigned inv;   // x / G = x * inv >> 16 for x < NEAR_CAP
-    __device__ __forceinline__ explicit Parts(int g) : G(g), S(((NEAR_CAP + g - 1) / g + 3) & ~3), inv((65536u + g - 1) / g) {}
+    __device__ __forceinline__ explicit Parts(int g) : G(g), S((((NEAR_CAP + g - 1) / g + 3) & ~7) + 4), inv((65536u + g - 1) / g) {}
     __device__ __forceinline__ int div(int q) const { return (int)((unsigned)q * inv >> 16); }
     __device__ __forceinline__ int count(int p, int n) const { return n > p ? div(n - p - 1) + 1 : 0; }
 };
@@ -79,8 +86,8 @@ struct NearPrm {
 struct Near32 {
     using T = float;
     struct Bodies { const float4 *hi, *lo; };
-    // hi x, y, z, lo x, y, z, mass; a part's sources lie one after another (G S <= 168 slots for the G that near_parts gives)
-    struct alignas(16) Stage { float v[7][192]; };
+    // hi x, y, z, lo x, y, z, mass; a part's sources lie one after another (G S <= 252 slots for the G of the table)
+    struct alignas(16) Stage { float v[7][256]; };
     struct Target { float h[3], l[3]; };
     struct Acc { float s[4], c[4]; };
 
@@ -299,7 +306,7 @@ __global__ void __launch_bounds__(32, sizeof(typename N::T) == 4 ? 28 : 20)
         if (KM == 2 && u0 == u1) continue;
         const int j0 = 32 * (int)(w - chunk_off[lf]);
         const int T = min(32, cnt - j0);
-        const int G = near_parts<NU>(T);
+        const int G = c_parts.g[NU / 32 - 1][T];
         const int U = T * G;
         const Parts pa(G);
         // the lane's units: target tt[r] (index in the leaf), source part pp[r]

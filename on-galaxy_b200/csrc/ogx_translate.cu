@@ -38,7 +38,7 @@ struct Tr {
     static constexpr int NTW = (NT + PARTS - 1) / PARTS;      // tiles of one part
     static constexpr int LDN = 8 * NT + 4;                    // operator rows (m2l64_pad_cols)
     static constexpr int LDA = (K4 % 16 == 4 || K4 % 16 == 12) ? K4 : K4 + 4;
-    static constexpr int UB = NTW <= 3 ? 8 : 4;               // steps of operator rows in flight
+    static constexpr int UB = 4;                              // steps of operator rows in flight
 };
 
 __device__ __forceinline__ int deg_of(int dof) {
@@ -131,7 +131,7 @@ __device__ __forceinline__ void level_items(const int* __restrict__ nl_off, int 
 
 // item = (level, group of 16 parents, octant); warp = column part
 template <int P>
-__global__ void __launch_bounds__(32 * Tr<P>::PARTS) k_l2l(TreeView tv, const int* __restrict__ nonleaf, const int* __restrict__ nl_off,
+__global__ void __launch_bounds__(32 * Tr<P>::PARTS, Tr<P>::NTW <= 3 ? 4 : 2) k_l2l(TreeView tv, const int* __restrict__ nonleaf, const int* __restrict__ nl_off,
                                                       int nlev, const double* __restrict__ ops, double* local,
                                                       const double* __restrict__ lown, int* ready, int* ticket, int* err) {
     using C = Tr<P>;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * Tr<P>::PARTS) k_l2l(TreeView tv, const in
 
 // item = (level, group of 16 parents, column part); warp = octant
 template <int P>
-__global__ void __launch_bounds__(256) k_m2m(TreeView tv, const int* __restrict__ nonleaf, const int* __restrict__ nl_off, int nlev,
+__global__ void __launch_bounds__(256, 2) k_m2m(TreeView tv, const int* __restrict__ nonleaf, const int* __restrict__ nl_off, int nlev,
                                              const double* __restrict__ ops, double* mpole, int* ready, int* ticket, int* err) {
     using C = Tr<P>;
     constexpr int K = C::K, W = 8 * C::NTW;
@@ -283,8 +283,8 @@ int level_boxes(const Handle& h, int l) {
 }
 
 // One launch: CTAs for the widest level's items (taking a quarter of the next level's boxes
-// for a level's parents), at most two per SM.  Any number is correct; more would only wait
-// and hold the SMs that other systems need.
+// for a level's parents), at most four (M2M, of eight warps: two) per SM.  Any number is
+// correct; more would only wait and hold the SMs that other systems need.
 template <int P>
 int translate(Handle& h, bool down, Slot slot, double* M, double* L, const double* Lown) {
     const int nlev = h.max_level;   // parent levels 0 .. max_level-1
@@ -299,7 +299,7 @@ int translate(Handle& h, bool down, Slot slot, double* M, double* L, const doubl
     OGX_TRY(arena_get(h.ws, slot, nready, &ready));
     OGX_CUDA(cudaMemsetAsync(ready, 0, sizeof(int) * nready, h.stream));
     int* ticket = ready + h.tv.nb;
-    const int grid = std::min(items, 2 * h.num_sms);
+    const int grid = std::min(items, (down ? 4 : 2) * h.num_sms);
     if (down)
         k_l2l<P><<<grid, 32 * Tr<P>::PARTS, 0, h.stream>>>(h.tv, h.d_nonleaf, h.d_nonleaf_off, nlev, h.d_l2l, L, Lown, ready, ticket,
                                                            h.d_err);

@@ -23,7 +23,7 @@ def test_every_order_matches_the_oracle(ogx, oracle, p):
 
 @pytest.mark.parametrize("n, thr", [(70, 8), (3001, 16), (40000, 8), (150000, 4)])
 def test_every_split_matches_the_oracle(ogx, oracle, n, thr):
-    # 70 bodies: a tile or two; 150,000 at leaf 4: above 1,184 tiles, no split
+    # 70 bodies: a tile or two; 150,000 at leaf 4: above 888 tiles, no split
     pos, _, mass = ogx_ic.plummer(n, seed=n)
     ref = oracle.adaptive_fmm(pos, mass, p=2, thr=thr, with_pot=False)
     for prec in (ogx.PREC_FP64, ogx.PREC_FP64_ROT):
