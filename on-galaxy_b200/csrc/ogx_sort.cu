@@ -5,11 +5,11 @@
 //   1. bodies by their 72-bit octant path (9 passes of 8 bits),
 //   2. bodies by leaf id, starting from the original order, so that inside a
 //      leaf the bodies keep their original index order (2-3 passes).
-// Ranking is the same everywhere: a warp ranks 32 keys with __match_any_sync,
+// Ranking is the same everywhere: a warp ranks 32 keys by votes (digit_peers),
 // keeps per-warp digit counters in shared memory and warps are ordered by their
 // contiguous sub-tiles, so a pass is stable.
 //
-// Up to 131,072 items, all passes run in ONE launch of a thread-block cluster: every CTA
+// Up to 65,536 items, all passes run in ONE launch of a thread-block cluster: every CTA
 // keeps its items in registers and shared memory, digit counts are exchanged and items
 // scattered through distributed shared memory, with two cluster barriers per pass.  These
 // sizes are bound by latency, not by memory: as four launches per pass (histogram, two
@@ -25,6 +25,20 @@ namespace {
 
 namespace cg = cooperative_groups;
 constexpr unsigned FULL = 0xffffffffu;
+
+// lanes of the warp whose digit equals this lane's (8 bits; 0xFFFFFFFF: no item), by a vote
+// per bit: nine votes, where __match_any_sync takes a turn per distinct digit
+__device__ __forceinline__ unsigned digit_peers(uint32_t d) {
+    unsigned m = __ballot_sync(FULL, d <= 0xFFu);
+    if (d > 0xFFu) m = ~m;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool one = (d >> b) & 1u;
+        const unsigned v = __ballot_sync(FULL, one);
+        m &= one ? v : ~v;
+    }
+    return m;
+}
 
 struct Key32 {
     uint32_t* k;
@@ -74,20 +88,22 @@ struct Key72 {
 };
 
 // ---- one launch, all passes: a cluster of CTAs ------------------------------------------
-constexpr int RC_THREADS = 1024;
-constexpr int RC_WARPS = RC_THREADS / 32;
-constexpr int RC_MAX_CTAS = 16;
-constexpr int RC_MAX = RC_MAX_CTAS * RC_THREADS * 8;   // 131,072 items
+// A pass is bound by the instructions of one SM (about 700 per warp), so small inputs take
+// small CTAs on more SMs: 8,192 bodies (15 passes) 297 -> 257 us per evaluation, 50,000 with
+// the spline 670 -> 600 (CTAs of 1,024 threads before).  100,001 bodies (FP64 rotation form)
+// alone take 2.12 ms with clusters of 16 x 1,024 x 8 and 2.02 ms with tiles, which spread
+// over more SMs: the line is 16 CTAs of 512 threads.
+constexpr int RC_MAX = 65536;   // 16 CTAs of 512 threads x 8 items
 
-template <class KO, int IPT>
-constexpr int rc_smem() { return RC_THREADS * IPT * (int)(KO::BYTES + 4) + RC_WARPS * 256 * 4; }
+template <class KO, int RC_THREADS, int IPT>
+constexpr int rc_smem() { return RC_THREADS * IPT * (int)(KO::BYTES + 4) + RC_THREADS / 32 * 256 * 4; }
 
-template <class KO, int IPT>
+template <class KO, int RC_THREADS, int IPT>
 __global__ void __launch_bounds__(RC_THREADS) rs_cluster(KO kin, KO kout, const uint32_t* vin, uint32_t* vout, int n,
                                                          int first_pass, int npasses) {
-    constexpr int TILE = RC_THREADS * IPT;
+    constexpr int TILE = RC_THREADS * IPT, RC_WARPS = RC_THREADS / 32, NQ = RC_THREADS / 256;
     extern __shared__ __align__(16) unsigned char rc_raw[];
-    __shared__ uint32_t s_cnt[256], s_base[256], s_quarter[4][256], s_warp[8];
+    __shared__ uint32_t s_cnt[256], s_base[256], s_quarter[NQ][256], s_warp[8];
     typename KO::Smem sk = KO::smem(rc_raw, TILE);
     uint32_t* sv = reinterpret_cast<uint32_t*>(rc_raw + (size_t)TILE * KO::BYTES);
     uint32_t(*wcnt)[256] = reinterpret_cast<uint32_t(*)[256]>(sv + TILE);
@@ -115,7 +131,7 @@ __global__ void __launch_bounds__(RC_THREADS) rs_cluster(KO kin, KO kout, const 
         for (int r = 0; r < IPT; ++r) {
             const bool valid = local0 + 32 * r < left;
             const uint32_t d = valid ? KO::digit(key[r], pass) : 0xFFFFFFFFu;
-            const unsigned peers = __match_any_sync(FULL, d);
+            const unsigned peers = digit_peers(d);
             uint32_t c = 0;
             if (valid) c = wcnt[w][d];
             __syncwarp();
@@ -124,13 +140,13 @@ __global__ void __launch_bounds__(RC_THREADS) rs_cluster(KO kin, KO kout, const 
             loc[r] = c + __popc(peers & lt);
         }
         __syncthreads();
-        {   // counters -> offsets inside the CTA's digit, a quarter of the warps per thread
+        {   // counters -> offsets inside the CTA's digit, eight warps per thread
             const int d = t & 255, q = t >> 8;
             uint32_t run = 0;
 #pragma unroll
-            for (int k = 0; k < RC_WARPS / 4; ++k) {
-                const uint32_t c = wcnt[q * (RC_WARPS / 4) + k][d];
-                wcnt[q * (RC_WARPS / 4) + k][d] = run;
+            for (int k = 0; k < RC_WARPS / NQ; ++k) {
+                const uint32_t c = wcnt[q * (RC_WARPS / NQ) + k][d];
+                wcnt[q * (RC_WARPS / NQ) + k][d] = run;
                 run += c;
             }
             s_quarter[q][d] = run;
@@ -139,7 +155,7 @@ __global__ void __launch_bounds__(RC_THREADS) rs_cluster(KO kin, KO kout, const 
         if (t < 256) {
             uint32_t run = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < NQ; ++q) {
                 const uint32_t c = s_quarter[q][t];
                 s_quarter[q][t] = run;
                 run += c;
@@ -174,7 +190,7 @@ __global__ void __launch_bounds__(RC_THREADS) rs_cluster(KO kin, KO kout, const 
         for (int r = 0; r < IPT; ++r) {
             if (local0 + 32 * r < left) {
                 const uint32_t d = KO::digit(key[r], pass);
-                const uint32_t pos = s_base[d] + s_quarter[w / (RC_WARPS / 4)][d] + wcnt[w][d] + loc[r];
+                const uint32_t pos = s_base[d] + s_quarter[w / (RC_WARPS / NQ)][d] + wcnt[w][d] + loc[r];
                 if (last) {
                     kout.store(pos, key[r]);
                     vout[pos] = val[r];
@@ -218,7 +234,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_hist(KO keys, int64_t n, int pa
     }
 #pragma unroll
     for (int r = 0; r < IPT; ++r) {
-        const unsigned peers = __match_any_sync(FULL, d[r]);
+        const unsigned peers = digit_peers(d[r]);
         if (d[r] < 256 && lane == __ffs(peers) - 1) atomicAdd(&h[d[r]], (uint32_t)__popc(peers));
     }
     __syncthreads();
@@ -295,7 +311,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(KO kin, KO kout, const 
     for (int r = 0; r < IPT; ++r) {
         const bool valid = base + r * 32 < n;
         const uint32_t d = valid ? KO::digit(key[r], pass) : 0xFFFFFFFFu;
-        const unsigned peers = __match_any_sync(FULL, d);
+        const unsigned peers = digit_peers(d);
         uint32_t c = 0;
         if (valid) c = wcnt[w][d];
         __syncwarp();
@@ -469,12 +485,11 @@ int scan2_i32_to_i64(Handle& h, const int* in_a, int64_t* out_a, const int* in_b
     return scan_arrays(h, sp, 2, n);
 }
 
-// The cluster sort: IPT items per thread and the fewest CTAs (a power of two) that hold n.
-// CTAs of 4,096 items while a cluster of 8 holds them (fewer rounds per pass), else of 8,192.
-template <class KO, int IPT>
+// The cluster sort with the fewest CTAs (a power of two) that hold n.
+template <class KO, int RC_THREADS, int IPT>
 static int cluster_sort(Handle& h, KO a, KO b, const uint32_t* va, uint32_t* vb, int64_t n, int npasses, int first_pass) {
-    auto kern = rs_cluster<KO, IPT>;
-    constexpr int smem = rc_smem<KO, IPT>();
+    auto kern = rs_cluster<KO, RC_THREADS, IPT>;
+    constexpr int smem = rc_smem<KO, RC_THREADS, IPT>();
     OGX_CUDA(smem_optin((const void*)kern, smem));
     int ctas = 1;
     while ((int64_t)ctas * RC_THREADS * IPT < n) ctas *= 2;
@@ -516,8 +531,9 @@ static int radix_passes(Handle& h, KO a, KO b, uint32_t* va, uint32_t* vb, int64
                         int first_pass = 0) {
     if (n <= RC_MAX) {
         *which = 1;
-        if (n <= 8 * RC_THREADS * 4) return cluster_sort<KO, 4>(h, a, b, va, vb, n, npasses, first_pass);
-        return cluster_sort<KO, 8>(h, a, b, va, vb, n, npasses, first_pass);
+        if (n <= 8 * 256 * 4) return cluster_sort<KO, 256, 4>(h, a, b, va, vb, n, npasses, first_pass);
+        if (n <= 16 * 256 * 8) return cluster_sort<KO, 256, 8>(h, a, b, va, vb, n, npasses, first_pass);
+        return cluster_sort<KO, 512, 8>(h, a, b, va, vb, n, npasses, first_pass);
     }
     *which = (npasses - first_pass) & 1;  // 0: result in a, 1: result in b
     // tiles of 2,048 while 4,096 would leave SMs without one

@@ -9,8 +9,9 @@ from helpers import assert_same_tree_arrays, canonical_rank
 pytestmark = pytest.mark.gpu
 
 
-# 4,096 items per CTA up to 32,768, 8,192 up to 131,072, tiles of 2,048 up to 606,208, then 4,096
-@pytest.mark.parametrize("n", [33, 4095, 4097, 8193, 32767, 32769, 65537, 131071, 131072, 131073, 262145, 606209])
+# 1,024 items per CTA up to 8,192, 2,048 up to 32,768, 4,096 up to 65,536, tiles of 2,048 up to
+# 606,208, then 4,096
+@pytest.mark.parametrize("n", [33, 1023, 1025, 4097, 8192, 8193, 16385, 32767, 32769, 65535, 65536, 65537, 131073, 606209])
 def test_tree_matches_the_oracle(ogx, oracle, n):
     rng = np.random.Generator(np.random.PCG64(n))
     pos = rng.standard_normal((n, 3)) * rng.random((n, 1)) ** 3   # clustered, no velocities needed
