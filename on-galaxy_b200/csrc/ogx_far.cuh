@@ -15,7 +15,7 @@
 // In FP32 two columns m, m + 1 go together in packed pairs (f32x2: the FMA pipe's rate at
 // half the issue slots): step i of the pair is T_{m+i,m} and T_{m+1+i,m+1}.
 // Bound: FP32 issue slots (the records come from shared memory as warp-wide broadcasts).
-// M2P + L2P of the 1M merger (p = 8, 14.4M evaluations, serialised): 1.33 -> 0.79 ms; in
+// M2P + L2P of the 1M merger (p = 8, 14.4M evaluations, serialised): 1.33 -> 0.72 ms; in
 // FP64 the 262,144-body galaxy: 1.30 -> 0.41 ms (one warp per leaf had walked the W list
 // of a leaf in turn, 199 boxes at most).
 #pragma once
@@ -113,68 +113,92 @@ __host__ __device__ constexpr double rec_b(int n, int m) {
     return (double)((n - 1) * (n - 1) - m * m) / (double)((2 * n - 1) * (2 * n - 3));
 }
 
-// out = {sum_axis x, y, z(, phi)} of one body at scaled offset (x, y, z) for a record in
-// shared memory; SING: singular harmonics (M2P), else regular (L2P)
-template <int L, bool POT, bool SING>
-__device__ __forceinline__ void eval(const float4* rec, float x, float y, float z, float (&out)[4]) {
+// out[k] = {sum_axis x, y, z(, phi)} of NB bodies at scaled offsets (x, y, z)[k] for a record
+// in shared memory, read once for all of them; SING: singular harmonics (M2P), else regular
+// (L2P)
+template <int L, bool POT, bool SING, int NB>
+__device__ __forceinline__ void eval(const float4* rec, float (&x)[NB], float (&y)[NB], float (&z)[NB], float (&out)[NB][4]) {
     using R = Rec<float, L, POT>;
-    float kap = x * x + y * y + z * z, d0 = 1.f;
-    if (SING) {
-        d0 = rsqrtf(kap);
-        kap = d0 * d0;
-        x *= kap; y *= kap; z *= kap;
-    }
-    const f2 z2 = pack2(z, z), nk2 = pack2(-kap, -kap);
-    // (x + iy)^2 carries a column pair to the next
-    const float qr = x * x - y * y, qi = 2.f * x * y;
-    const f2 qr2 = pack2(qr, qr), qi2 = pack2(qi, qi), nqi2 = pack2(-qi, -qi);
-    f2 dr = pack2(d0, d0 * x), di = pack2(0.f, d0 * y);
-    f2 o[4];
+    f2 z2[NB], nk2[NB], qr2[NB], qi2[NB], nqi2[NB], dr[NB], di[NB], o[NB][4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) o[a].v = 0ull;
+    for (int k = 0; k < NB; ++k) {
+        float kap = x[k] * x[k] + y[k] * y[k] + z[k] * z[k], d0 = 1.f;
+        if (SING) {
+            d0 = rsqrtf(kap);
+            kap = d0 * d0;
+            x[k] *= kap; y[k] *= kap; z[k] *= kap;
+        }
+        z2[k] = pack2(z[k], z[k]);
+        nk2[k] = pack2(-kap, -kap);
+        // (x + iy)^2 carries a column pair to the next
+        const float qr = x[k] * x[k] - y[k] * y[k], qi = 2.f * x[k] * y[k];
+        qr2[k] = pack2(qr, qr);
+        qi2[k] = pack2(qi, qi);
+        nqi2[k] = pack2(-qi, -qi);
+        dr[k] = pack2(d0, d0 * x[k]);
+        di[k] = pack2(0.f, d0 * y[k]);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) o[k][a].v = 0ull;
+    }
     const ulonglong2* r = reinterpret_cast<const ulonglong2*>(rec);
     int e = 0;
 #pragma unroll
     for (int m = 0; m <= L; m += 2) {
-        f2 s[R::V], t0 = pack2(1.f, 1.f), t1 = z2;
+        f2 s[NB][R::V], t0[NB], t1[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            t0[k] = pack2(1.f, 1.f);
+            t1[k] = z2[k];
+        }
 #pragma unroll
         for (int i = 0; i <= L - m; ++i, ++e) {
-            f2 c[R::V], t = t1;
+            f2 c[R::V];
 #pragma unroll
             for (int a = 0; a < R::V / 2; ++a) {
                 const ulonglong2 w = r[e * (R::V / 2) + a];
                 c[2 * a].v = w.x;
                 c[2 * a + 1].v = w.y;
             }
-            if (i == 0) {
 #pragma unroll
-                for (int a = 0; a < R::V; ++a) s[a] = c[a];
-                continue;
-            }
-            if (i >= 2) {
-                const f2 b = pack2((float)rec_b(m + i, m), (float)rec_b(m + 1 + i, m + 1));
-                t = fma2(z2, t1, mul2(mul2(b, nk2), t0));
-                t0 = t1;
-                t1 = t;
-            }
+            for (int k = 0; k < NB; ++k) {
+                if (i == 0) {
 #pragma unroll
-            for (int a = 0; a < R::V; ++a) s[a] = fma2(c[a], t, s[a]);
+                    for (int a = 0; a < R::V; ++a) s[k][a] = c[a];
+                    continue;
+                }
+                f2 t = t1[k];
+                if (i >= 2) {
+                    const f2 b = pack2((float)rec_b(m + i, m), (float)rec_b(m + 1 + i, m + 1));
+                    t = fma2(z2[k], t1[k], mul2(mul2(b, nk2[k]), t0[k]));
+                    t0[k] = t1[k];
+                    t1[k] = t;
+                }
+#pragma unroll
+                for (int a = 0; a < R::V; ++a) s[k][a] = fma2(c[a], t, s[k][a]);
+            }
         }
 #pragma unroll
-        for (int a = 0; a < R::V / 2; ++a) o[a] = fma2(s[2 * a], dr, fma2(s[2 * a + 1], di, o[a]));
-        if (m + 2 <= L) {
-            const f2 nr = fma2(dr, qr2, mul2(di, nqi2));
-            di = fma2(dr, qi2, mul2(di, qr2));
-            dr = nr;
+        for (int k = 0; k < NB; ++k) {
+#pragma unroll
+            for (int a = 0; a < R::V / 2; ++a) o[k][a] = fma2(s[k][2 * a], dr[k], fma2(s[k][2 * a + 1], di[k], o[k][a]));
+            if (m + 2 <= L) {
+                const f2 nr = fma2(dr[k], qr2[k], mul2(di[k], nqi2[k]));
+                di[k] = fma2(dr[k], qi2[k], mul2(di[k], qr2[k]));
+                dr[k] = nr;
+            }
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) out[a] = a < R::V / 2 ? sum2(o[a]) : 0.f;
+    for (int k = 0; k < NB; ++k)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) out[k][a] = a < R::V / 2 ? sum2(o[k][a]) : 0.f;
 }
 
-template <int L, bool POT, bool SING>
-__device__ __forceinline__ void eval(const float4* rec, double x, double y, double z, double (&out)[4]) {
+template <int L, bool POT, bool SING, int NB>
+__device__ __forceinline__ void eval(const float4* rec, double (&xs)[NB], double (&ys)[NB], double (&zs)[NB], double (&outs)[NB][4]) {
+    static_assert(NB == 1, "the FP64 pipe, not the records' reads, bounds this form");
     using R = Rec<double, L, POT>;
+    double x = xs[0], y = ys[0], z = zs[0], (&out)[4] = outs[0];
     double kap = x * x + y * y + z * z, dr = 1.0, di = 0.0;
     if (SING) {
         dr = rsqrt(kap);
@@ -221,29 +245,34 @@ __device__ __forceinline__ void eval(const float4* rec, double x, double y, doub
     }
 }
 
-// ---- tasks: the (body, W box) pairs of a block of at most 64 bodies, W-major, taken in
-// rounds of at most 32 (lane = task).  A round covers at most RW W boxes, whose records
+// ---- tasks: the (NB bodies, W box) pairs of a block of at most 64 bodies, W-major, taken in
+// rounds of at most 32 (lane = task).  Heavy
+// leaves in FP32 take NB = 2: one read of a record's coefficients serves two bodies (with one
+// the shared-memory pipe was 76% busy, the FMA pipe 39%; 1M merger 547 -> 388 us).  A light
+// leaf's few tasks then fill 20 lanes of 32 instead of 25 (230 -> 275 us): NB = 1.  A round covers at most RW W boxes, whose records
 // one warp stages in shared memory.
 template <class T> struct Res;
 template <> struct Res<float> { using V = float4; };
 template <> struct Res<double> { using V = double4; };
 
-constexpr int FAR_RW = 3;          // boxes of a round: 32 tasks of leaves of 16 bodies and more span at most 3
+template <class T> constexpr int FAR_HEAVY_NB = sizeof(T) == 4 ? 2 : 1;   // bodies of a heavy leaf's task
+constexpr int FAR_RW = 3;          // boxes of a round: 32 tasks, 16 and more per box, span at most 3
 constexpr int FAR_HW = 8;          // warps of a heavy leaf's CTA
 
 // Leaves with more M2P tasks (bodies x W boxes) than this are taken by a CTA of FAR_HW
 // warps (k_leaf_far_heavy), so that one leaf with a long W list does not decide the
 // kernel's length.  In small trees (fewer leaves than warps the GPU holds) and in FP64 a
-// task costs more of the kernel's length, so the line is lower.
+// task costs more of the kernel's length, so the line is lower.  (512 instead of 1,024: 1M
+// merger 3.66 -> 3.67 ms, three 262,144-body systems of order 4 1.06 -> 1.08.)
 template <class T>
 __device__ __forceinline__ int64_t heavy_line(const TreeView& tv) { return sizeof(T) == 8 || tv_nleaf(tv) < 4096 ? 256 : 1024; }
 
 // shared memory of one warp
-template <int P, bool POT, class T>
+template <int P, bool POT, class T, int NB>
 struct alignas(16) WarpSmem {
     static constexpr int RF4 = Rec<T, P + 1, POT>::F4;
     float4 rec[FAR_RW * RF4];
-    typename Res<T>::V res[32];
+    typename Res<T>::V res[32 * NB];
     double hdr[FAR_RW][4];       // FP64: box centre, 1 / side; FP32: floats {offset xyz, scale, 1 / side}
 };
 
@@ -266,63 +295,79 @@ __device__ __forceinline__ void put_body(Bodies<float>& s, int j, double x, doub
 }
 
 // W box header, written by one lane per box.  FP32: the box's centre offset from the leaf in
-// its own side (a small dyadic number, exact), and the ratio of the sides (a power of two)
-__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double,
+// its own side (a small dyadic number, exact), and the ratio of the sides (a power of two,
+// 2^up; winv = 2^up / side of the leaf is exact too, where a division took thirty operations)
+__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double winv, int,
                                            double) {
-    h[0] = cx - c01.x; h[1] = cy - c01.y; h[2] = cz - c23.x; h[3] = 1.0 / (2.0 * c23.y);
+    h[0] = cx - c01.x; h[1] = cy - c01.y; h[2] = cz - c23.x; h[3] = winv;
 }
-__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double side,
-                                           float) {
+__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double winv,
+                                           int up, float) {
     float* f = reinterpret_cast<float*>(h);
-    const double winv = 1.0 / (2.0 * c23.y);
     f[0] = (float)((cx - c01.x) * winv);
     f[1] = (float)((cy - c01.y) * winv);
     f[2] = (float)((cz - c23.x) * winv);
-    f[3] = (float)(side * winv);
+    f[3] = __int_as_float((127 + up) << 23);   // 0 <= up <= 24
     f[4] = (float)winv;
 }
+// v * 2^up
+__device__ __forceinline__ double scale2(double v, int up) { return v * __hiloint2double((1023 + up) << 20, 0); }
 
-template <int L, bool POT>
-__device__ __forceinline__ double4 m2p_task(const float4* rec, const double (&h)[4], const Bodies<double>& s, int j) {
-    const double w = h[3];
-    double o[4];
-    eval<L, POT, true>(rec, (s.x[0][j] + h[0]) * w, (s.x[1][j] + h[1]) * w, (s.x[2][j] + h[2]) * w, o);
-    const double w2 = w * w;
-    return make_double4(o[0] * w2, o[1] * w2, o[2] * w2, POT ? o[3] * w : 0.0);
-}
-template <int L, bool POT>
-__device__ __forceinline__ float4 m2p_task(const float4* rec, const double (&hd)[4], const Bodies<float>& s, int j) {
-    const float* h = reinterpret_cast<const float*>(hd);
-    const float sc = h[3], w = h[4];
-    float u[3], o[4];
+// results of the bodies j[k] for a W box
+template <int L, bool POT, int NB>
+__device__ __forceinline__ void m2p_task(const float4* rec, const double (&h)[4], const Bodies<double>& s, const int (&j)[NB],
+                                         double4 (&res)[NB]) {
+    const double w = h[3], w2 = w * w;
+    double u[3][NB], o[NB][4];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) u[a] = fmaf(s.l[a][j], sc, fmaf(s.h[a][j], sc, h[a]));
-    eval<L, POT, true>(rec, u[0], u[1], u[2], o);
-    const float w2 = w * w;
-    return make_float4(o[0] * w2, o[1] * w2, o[2] * w2, POT ? o[3] * w : 0.f);
+    for (int k = 0; k < NB; ++k)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) u[a][k] = (s.x[a][j[k]] + h[a]) * w;
+    eval<L, POT, true, NB>(rec, u[0], u[1], u[2], o);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) res[k] = make_double4(o[k][0] * w2, o[k][1] * w2, o[k][2] * w2, POT ? o[k][3] * w : 0.0);
+}
+template <int L, bool POT, int NB>
+__device__ __forceinline__ void m2p_task(const float4* rec, const double (&hd)[4], const Bodies<float>& s, const int (&j)[NB],
+                                         float4 (&res)[NB]) {
+    const float* h = reinterpret_cast<const float*>(hd);
+    const float sc = h[3], w = h[4], w2 = w * w;
+    float u[3][NB], o[NB][4];
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) u[a][k] = fmaf(s.l[a][j[k]], sc, fmaf(s.h[a][j[k]], sc, h[a]));
+    eval<L, POT, true, NB>(rec, u[0], u[1], u[2], o);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) res[k] = make_float4(o[k][0] * w2, o[k][1] * w2, o[k][2] * w2, POT ? o[k][3] * w : 0.f);
 }
 
 // The rounds first, first + stride, ... of a block of nbk bodies and nw W boxes; every body
 // sums its own task results in task order into acc (FP64; lane owns bodies lane, lane + 32).
-template <int P, bool POT, class T>
+template <int P, bool POT, int NB, class T>
 __device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restrict__ hrec, int64_t w0, int nw, int nbk, int first,
-                                           int stride, const Bodies<T>& sb, double cx, double cy, double cz, double side,
-                                           WarpSmem<P, POT, T>& sm, int lane, double (&acc)[2][4]) {
+                                           int stride, const Bodies<T>& sb, double cx, double cy, double cz, double inv, int level,
+                                           WarpSmem<P, POT, T, NB>& sm, int lane, double (&acc)[2][4]) {
     using R = Rec<T, P + 1, POT>;
     constexpr int RF4 = R::F4;
-    const int total = nbk * nw;
-    // tasks of a round: at most FAR_RW boxes (whole ones for leaves of fewer than 16 bodies)
-    const int Q = nbk >= 16 ? 32 : (FAR_RW * nbk <= 32 ? FAR_RW : FAR_RW - 1) * nbk;
+    const int nt1 = (nbk + NB - 1) / NB;   // tasks of a box: bodies j, j + nt1, ...
+    const int total = nt1 * nw;
+    // tasks of a round: at most FAR_RW boxes (whole ones where a box has fewer than 16)
+    const int Q = nt1 >= 16 ? 32 : (FAR_RW * nt1 <= 32 ? FAR_RW : FAR_RW - 1) * nt1;
     int b0 = first * Q;
-    // this lane's task: box w, body j
-    int w = (b0 + lane) / nbk, j = b0 + lane - w * nbk;
-    const int dq = stride * Q / nbk, dr = stride * Q - dq * nbk;
-    for (; b0 < total; b0 += stride * Q) {
-        const int nt = min(Q, total - b0);
-        const int wa = __shfl_sync(0xffffffffu, w, 0), nrec = __shfl_sync(0xffffffffu, w, nt - 1) - wa + 1;
-        const int ja = __shfl_sync(0xffffffffu, j, 0);
-        int c = 0;
-        if (lane < nrec) c = tv.w_idx[w0 + wa + lane];
+    // this lane's task: box w, first body j
+    int w = (b0 + lane) / nt1, j = b0 + lane - w * nt1;
+    const int dq = stride * Q / nt1, dr = stride * Q - dq * nt1;
+    // the round's boxes wa .. wa + nrec - 1, box index c of lane's one: known a round ahead, so
+    // a round waits for its records only
+    int nt = min(Q, total - b0), wa = 0, nrec = 0, c = 0;
+    auto boxes = [&]() {
+        wa = __shfl_sync(0xffffffffu, w, 0);
+        nrec = __shfl_sync(0xffffffffu, w, max(nt, 1) - 1) - wa + 1;
+        c = (nt > 0 && lane < nrec) ? tv.w_idx[w0 + wa + lane] : 0;
+    };
+    boxes();
+    while (b0 < total) {
         for (int q = 0; q < nrec; ++q) {
             const float4* src = reinterpret_cast<const float4*>(hrec + (size_t)__shfl_sync(0xffffffffu, c, q) * R::SIZE);
 #pragma unroll
@@ -332,27 +377,41 @@ __device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restri
         if (lane < nrec) {
             const double2 c01 = __ldg(reinterpret_cast<const double2*>(tv.center) + 2 * (size_t)c);
             const double2 c23 = __ldg(reinterpret_cast<const double2*>(tv.center) + 2 * (size_t)c + 1);
-            put_header(sm.hdr[lane], c01, c23, cx, cy, cz, side, T(0));
+            const int up = __ldg(tv.level + c) - level;
+            put_header(sm.hdr[lane], c01, c23, cx, cy, cz, scale2(inv, up), up, T(0));
         }
+        const int wr = w - wa, jr = j, ja = __shfl_sync(0xffffffffu, j, 0), ntr = nt;
+        b0 += stride * Q;
+        w += dq;
+        j += dr;
+        if (j >= nt1) { j -= nt1; ++w; }
+        nt = min(Q, total - b0);
+        boxes();   // of the next round
         sm100::cp_async_wait_all();
         __syncwarp();
-        if (lane < nt) sm.res[lane] = m2p_task<P + 1, POT>(sm.rec + (w - wa) * RF4, sm.hdr[w - wa], sb, j);
+        if (lane < ntr) {
+            int jb[NB];
+            typename Res<T>::V v[NB];
+#pragma unroll
+            for (int k = 0; k < NB; ++k) jb[k] = jr + k * nt1 < nbk ? jr + k * nt1 : jr;
+            m2p_task<P + 1, POT, NB>(sm.rec + wr * RF4, sm.hdr[wr], sb, jb, v);
+#pragma unroll
+            for (int k = 0; k < NB; ++k) sm.res[32 * k + lane] = v[k];
+        }
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int jo = lane + 32 * q;
             if (jo < nbk) {
-                for (int k = jo >= ja ? jo - ja : jo - ja + nbk; k < nt; k += nbk) {
-                    const auto v = sm.res[k];
+                const int half = NB > 1 && jo >= nt1, jt = jo - half * nt1;
+                for (int k = jt >= ja ? jt - ja : jt - ja + nt1; k < ntr; k += nt1) {
+                    const auto v = sm.res[32 * half + k];
                     acc[q][0] += v.x; acc[q][1] += v.y; acc[q][2] += v.z;
                     if (POT) acc[q][3] += v.w;
                 }
             }
         }
         __syncwarp();   // the next round's copies overwrite the records and results
-        w += dq;
-        j += dr;
-        if (j >= nbk) { j -= nbk; ++w; }
     }
 }
 
@@ -369,13 +428,17 @@ __device__ __forceinline__ void l2p_block(const T* __restrict__ g, int nbk, cons
     for (int q = 0; q < 2; ++q) {
         const int j = lane + 32 * q;
         if (j < nbk) {
-            T o[4];
-            if constexpr (sizeof(T) == 4) eval<L, POT, false>(srec, sb.h[0][j], sb.h[1][j], sb.h[2][j], o);
-            else eval<L, POT, false>(srec, sb.x[0][j] * inv, sb.x[1][j] * inv, sb.x[2][j] * inv, o);
-            acc[q][0] += (double)o[0] * inv;
-            acc[q][1] += (double)o[1] * inv;
-            acc[q][2] += (double)o[2] * inv;
-            if (POT) acc[q][3] += (double)o[3];
+            T u[3][1], o[1][4];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                if constexpr (sizeof(T) == 4) u[a][0] = sb.h[a][j];
+                else u[a][0] = sb.x[a][j] * inv;
+            }
+            eval<L, POT, false, 1>(srec, u[0], u[1], u[2], o);
+            acc[q][0] += (double)o[0][0] * inv;
+            acc[q][1] += (double)o[0][1] * inv;
+            acc[q][2] += (double)o[0][2] * inv;
+            if (POT) acc[q][3] += (double)o[0][3];
         }
     }
     __syncwarp();
@@ -400,7 +463,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? 20 : 12) k_leaf_far(TreeV
     const int nw = DO_M2P ? (int)(tv.w_off[lf + 1] - w0) : 0;
     if (DO_M2P && (int64_t)cnt * nw > heavy_line<T>(tv)) return;
     const double cx = tv.center[4 * b], cy = tv.center[4 * b + 1], cz = tv.center[4 * b + 2];
-    const double side = 2.0 * tv.center[4 * b + 3], inv = 1.0 / side;
+    const double inv = 1.0 / (2.0 * tv.center[4 * b + 3]);
     for (int jb = 0; jb < cnt; jb += 64) {
         const int nbk = min(64, cnt - jb);
         double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
@@ -416,8 +479,8 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? 20 : 12) k_leaf_far(TreeV
             l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, inv, reinterpret_cast<float4*>(s_far_dyn), lane, acc);
         if constexpr (DO_M2P)
             if (nw > 0)
-                m2p_rounds<P, POT, T>(tv, hrec, w0, nw, nbk, 0, 1, sb, cx, cy, cz, side,
-                                      *reinterpret_cast<WarpSmem<P, POT, T>*>(s_far_dyn), lane, acc);
+                m2p_rounds<P, POT, 1, T>(tv, hrec, w0, nw, nbk, 0, 1, sb, cx, cy, cz, inv, tv.level[b],
+                                         *reinterpret_cast<WarpSmem<P, POT, T, 1>*>(s_far_dyn), lane, acc);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int j = lane + 32 * q;
@@ -433,7 +496,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? 20 : 12) k_leaf_far(TreeV
 template <int P, bool POT, bool DO_M2P, class T>
 constexpr size_t leaf_far_smem() {
     constexpr size_t a = sizeof(float4) * Rec<T, rec_degree<P, 1, POT>(), POT>::F4;
-    return DO_M2P ? (sizeof(WarpSmem<P, POT, T>) > a ? sizeof(WarpSmem<P, POT, T>) : a) : a;
+    return DO_M2P ? (sizeof(WarpSmem<P, POT, T, 1>) > a ? sizeof(WarpSmem<P, POT, T, 1>) : a) : a;
 }
 
 // list of the heavy leaves (order irrelevant: every leaf's result is computed
@@ -450,7 +513,7 @@ __global__ void k_far_heavy_list(TreeView tv, int* __restrict__ list, int* count
 // themselves.  Warp w runs the rounds w, w + FAR_HW, ...; warp 0 also the L2P; the warps'
 // per-body partial sums are added in warp order through shared memory (deterministic).
 template <int P, bool POT, bool DO_L2P, class T>
-__global__ void __launch_bounds__(32 * FAR_HW, sizeof(T) == 4 ? 3 : 2) k_leaf_far_heavy(TreeView tv, const T* __restrict__ hrec,
+__global__ void __launch_bounds__(32 * FAR_HW, 2) k_leaf_far_heavy(TreeView tv, const T* __restrict__ hrec,
                                                                                        const T* __restrict__ grec,
                                                                                        double* __restrict__ far,
                                                                                        const int* __restrict__ list, int* ctr) {
@@ -460,7 +523,8 @@ __global__ void __launch_bounds__(32 * FAR_HW, sizeof(T) == 4 ? 3 : 2) k_leaf_fa
     __shared__ int s_lf;
     double* s_part = reinterpret_cast<double*>(s_far_dyn);   // [FAR_HW][64][4], over the records once the rounds are done
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    WarpSmem<P, POT, T>& sm = reinterpret_cast<WarpSmem<P, POT, T>*>(s_far_dyn)[wid];
+    using Smem = WarpSmem<P, POT, T, FAR_HEAVY_NB<T>>;
+    Smem& sm = reinterpret_cast<Smem*>(s_far_dyn)[wid];
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -475,7 +539,7 @@ __global__ void __launch_bounds__(32 * FAR_HW, sizeof(T) == 4 ? 3 : 2) k_leaf_fa
         const int64_t w0 = tv.w_off[lf];
         const int nw = (int)(tv.w_off[lf + 1] - w0);
         const double cx = tv.center[4 * b], cy = tv.center[4 * b + 1], cz = tv.center[4 * b + 2];
-        const double side = 2.0 * tv.center[4 * b + 3], inv = 1.0 / side;
+        const double inv = 1.0 / (2.0 * tv.center[4 * b + 3]);
         for (int jb = 0; jb < cnt; jb += 64) {
             const int nbk = min(64, cnt - jb);
             __syncthreads();
@@ -487,7 +551,7 @@ __global__ void __launch_bounds__(32 * FAR_HW, sizeof(T) == 4 ? 3 : 2) k_leaf_fa
             double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
             if constexpr (DO_L2P)
                 if (wid == 0) l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, inv, sm.rec, lane, acc);
-            m2p_rounds<P, POT, T>(tv, hrec, w0, nw, nbk, wid, FAR_HW, sb, cx, cy, cz, side, sm, lane, acc);
+            m2p_rounds<P, POT, FAR_HEAVY_NB<T>, T>(tv, hrec, w0, nw, nbk, wid, FAR_HW, sb, cx, cy, cz, inv, tv.level[b], sm, lane, acc);
             __syncthreads();
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
@@ -509,7 +573,7 @@ __global__ void __launch_bounds__(32 * FAR_HW, sizeof(T) == 4 ? 3 : 2) k_leaf_fa
 }
 template <int P, bool POT, class T>
 constexpr size_t leaf_far_heavy_smem() {
-    constexpr size_t a = FAR_HW * sizeof(WarpSmem<P, POT, T>), b = sizeof(double) * FAR_HW * 64 * 4;
+    constexpr size_t a = FAR_HW * sizeof(WarpSmem<P, POT, T, FAR_HEAVY_NB<T>>), b = sizeof(double) * FAR_HW * 64 * 4;
     return a > b ? a : b;
 }
 

@@ -113,7 +113,7 @@ __device__ __forceinline__ bool near_item(const TreeView& tv, const int64_t* chu
 // over the pairs closer than hs (the difference is zero beyond).  The far field took these
 // pairs with the Newtonian kernel; with this sum they carry the spline kernel's force.
 // Warp per leaf, lanes over the leaf's bodies, FP64 (the plain form; the mixed form runs
-// the FP32 near-field kernel over the same lists, mixed::k_leaf_near32<.., 2>).
+// the FP32 near-field kernel over the same lists, k_leaf_near<Near32, .., 2>).
 template <bool POT>
 __global__ void __launch_bounds__(128) k_soft_correct(TreeView tv, const int64_t* __restrict__ chunk_off, double hs, double hinv,
                                                       double* out) {
