@@ -345,13 +345,14 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(KO kin, KO kout, const 
 }
 
 // ---- generic exclusive scan int32 -> int64 (out has n+1 entries) --------------
-// Two arrays of one length at a time (grid y); up to SC_ONE entries in one launch (one
-// CTA walks them, its loads a chunk ahead), else per-tile sums and a second launch in
-// which every tile adds the sums before it.
+// Two arrays of one length at a time (grid y); up to SC_ONE entries in one launch, in
+// which every tile's CTA sums the entries before it itself (one CTA walking eight tiles in
+// turn took 9 us, a barrier chain per tile; 8 steps of 30,011 bodies 4.27 -> 4.18 ms); else per-tile sums and a second launch in which
+// every tile adds the sums before it.
 constexpr int SC_THREADS = 1024;
 constexpr int SC_IPT = 4;
 constexpr int SC_TILE = SC_THREADS * SC_IPT;
-constexpr int64_t SC_ONE = 8 * SC_TILE;
+constexpr int64_t SC_ONE = 32 * SC_TILE;
 
 struct ScanPair {
     const int* in[2];
@@ -393,29 +394,32 @@ __device__ __forceinline__ void sc_load(const int* in, int64_t b, int64_t n, int
 }
 
 __global__ void __launch_bounds__(SC_THREADS) sc_one(ScanPair sp, int64_t n) {
-    __shared__ int64_t sh[32];
+    __shared__ int64_t sh[32], s_before[32];
     const int* in = sp.in[blockIdx.y];
     int64_t* out = sp.out[blockIdx.y];
-    int64_t carry = 0;
+    const int64_t t0 = (int64_t)blockIdx.x * SC_TILE, b = t0 + (int64_t)threadIdx.x * SC_IPT;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int v[SC_IPT];
-    sc_load(in, (int64_t)threadIdx.x * SC_IPT, n, v);
-    for (int64_t t0 = 0; t0 < n; t0 += SC_TILE) {
-        const int64_t b = t0 + (int64_t)threadIdx.x * SC_IPT;
-        int nx[SC_IPT];
-        sc_load(in, b + SC_TILE, n, nx);
-        int64_t s = 0, tot;
+    sc_load(in, b, n, v);
+    int64_t before = 0, s = 0, tot;
+#pragma unroll 16
+    for (int64_t i = threadIdx.x; i < t0; i += SC_THREADS) before += in[i];
 #pragma unroll
-        for (int k = 0; k < SC_IPT; ++k) s += v[k];
-        int64_t run = carry + block_excl_scan_i64(s, sh, &tot);
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(FULL, before, o);
+    if (lane == 0) s_before[w] = before;
 #pragma unroll
-        for (int k = 0; k < SC_IPT; ++k) {
-            if (b + k < n) out[b + k] = run;
-            run += v[k];
-            v[k] = nx[k];
-        }
-        carry += tot;
+    for (int k = 0; k < SC_IPT; ++k) s += v[k];
+    const int64_t mine = block_excl_scan_i64(s, sh, &tot);
+    int64_t carry = s_before[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) carry += __shfl_xor_sync(FULL, carry, o);
+    int64_t run = carry + mine;
+#pragma unroll
+    for (int k = 0; k < SC_IPT; ++k) {
+        if (b + k < n) out[b + k] = run;
+        run += v[k];
     }
-    if (threadIdx.x == 0) out[n] = carry;
+    if (blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) out[n] = carry + tot;
 }
 
 __global__ void __launch_bounds__(SC_THREADS) sc_partials(ScanPair sp, int64_t n) {
@@ -459,7 +463,7 @@ static int scan_arrays(Handle& h, ScanPair sp, int count, int64_t n) {
         return OGX_OK;
     }
     if (n <= SC_ONE) {
-        sc_one<<<dim3(1, count), SC_THREADS, 0, h.stream>>>(sp, n); ++h.launches;
+        sc_one<<<dim3((unsigned)((n + SC_TILE - 1) / SC_TILE), count), SC_THREADS, 0, h.stream>>>(sp, n); ++h.launches;
     } else {
         const int nparts = (int)((n + SC_TILE - 1) / SC_TILE);
         OGX_TRY(arena_get(h.ws, S_SCAN_TMP, 2 * (size_t)nparts, &sp.part[0]));

@@ -32,3 +32,17 @@ def test_deep_cluster_takes_all_key_levels(ogx, oracle):
             s.compute_accelerations(pos, np.ones(n))
             got = s.tree()
         assert_same_tree_arrays(ref, got, f"deep n={n}")
+
+
+# boxes and leaves up to 4,096 in one scan tile, up to 131,072 in the one-launch scan, above
+# that in two launches
+@pytest.mark.parametrize("n, thr, boxes", [(3001, 1, (4097, 8192)), (40009, 2, (32769, 131072)), (130003, 2, (131073, 400000))])
+def test_scans_of_many_boxes(ogx, oracle, n, thr, boxes):
+    rng = np.random.Generator(np.random.PCG64(n))
+    pos = rng.random((n, 3))
+    ref = oracle.tree(pos, thr)
+    assert boxes[0] <= len(ref["boxes"]) <= boxes[1]
+    with ogx.AdaptiveFMM3D(p=1, threshold=thr) as s:
+        s.compute_accelerations(pos, np.ones(n))
+        got = s.tree()
+    assert_same_tree_arrays(ref, got, f"n={n} thr={thr}")
