@@ -104,19 +104,24 @@ static std::shared_ptr<HostOps> host_ops(int p, bool m2l) {
     return ops;
 }
 
+// The M2L operators are kept apart from the others: a handle of another form meets the plain
+// form too (ogx_ic_merger solves the circular-velocity field with it), also after evaluations
+// of its own.
 int ensure_operator_tables(Handle& h) {
-    if (h.ops_p == h.prm.p) return OGX_OK;
-    auto ops = host_ops(h.prm.p, false);
-    OGX_TRY(arena_get(h.ws, S_OPS_M2M, ops->m2m.size(), &h.d_m2m));
-    OGX_TRY(arena_get(h.ws, S_OPS_L2L, ops->l2l.size(), &h.d_l2l));
-    OGX_CUDA(upload_now(h.d_m2m, ops->m2m.data(), ops->m2m.size() * sizeof(double)));
-    OGX_CUDA(upload_now(h.d_l2l, ops->l2l.data(), ops->l2l.size() * sizeof(double)));
-    if (h.prm.precision == OGX_PREC_FP64) {
+    if (h.ops_p != h.prm.p) {
+        auto ops = host_ops(h.prm.p, false);
+        OGX_TRY(arena_get(h.ws, S_OPS_M2M, ops->m2m.size(), &h.d_m2m));
+        OGX_TRY(arena_get(h.ws, S_OPS_L2L, ops->l2l.size(), &h.d_l2l));
+        OGX_CUDA(upload_now(h.d_m2m, ops->m2m.data(), ops->m2m.size() * sizeof(double)));
+        OGX_CUDA(upload_now(h.d_l2l, ops->l2l.data(), ops->l2l.size() * sizeof(double)));
+        h.ops_p = h.prm.p;
+    }
+    if (h.prm.precision == OGX_PREC_FP64 && h.m2l_ops_p != h.prm.p) {
         auto m2l = host_ops(h.prm.p, true);
         OGX_TRY(arena_get(h.ws, S_OPS_M2L, m2l->m2l.size(), &h.d_m2l));
         OGX_CUDA(upload_now(h.d_m2l, m2l->m2l.data(), m2l->m2l.size() * sizeof(double)));
+        h.m2l_ops_p = h.prm.p;
     }
-    h.ops_p = h.prm.p;
     return OGX_OK;
 }
 

@@ -227,7 +227,8 @@ struct Handle {
     int max_level = 0;
     int64_t n = 0;
     // operator tables for prm.p (host built, device resident)
-    int ops_p = -1;
+    int ops_p = -1;           // order of d_m2m, d_l2l
+    int m2l_ops_p = -1;       // order of d_m2l (uploaded when the plain form first runs)
     // k-major, rows and columns padded with zeros (m2l64_pad_rows, m2l64_pad_cols)
     double* d_m2l = nullptr;  // 343 operators
     double* d_m2m = nullptr;  // 8

@@ -277,6 +277,7 @@ int m2l64_sum_launch(Handle& h, const M2L64Args& a, int slices, double* Lown, cu
 }
 
 int m2l_fp64_launch(Handle& h, const double* M, double* Lown) {
+    if (!h.d_m2l || h.m2l_ops_p != h.prm.p) return OGX_ERR_STATE;   // no operators on the device
     switch (h.prm.p) {
         case 1: return launch<1>(h, M, Lown);
         case 2: return launch<2>(h, M, Lown);

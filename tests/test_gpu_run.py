@@ -58,6 +58,32 @@ def test_ic_merger_is_deterministic_and_follows_the_profiles(ogx):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("form", ["mixed", "fp64rot", "fp64"])
+def test_ic_merger_on_a_handle_that_has_evaluated(ogx, form):
+    """The circular-velocity field is the plain form's, whatever the handle's form is and whatever
+    ran on it before: the same bits as on a fresh handle, and the handle's own form after it."""
+    import ogx_ic
+    prec = {"mixed": ogx.PREC_MIXED, "fp64rot": ogx.PREC_FP64_ROT, "fp64": ogx.PREC_FP64}[form]
+    pos, vel, mass = ogx_ic.plummer(3000, seed=2)
+    kw = dict(p=6, threshold=32, precision=prec)
+    with ogx.AdaptiveFMM3D(**kw) as s:
+        s.ic_merger(4000, seed=3)
+        fresh = s.download()
+    with ogx.AdaptiveFMM3D(**kw) as s:
+        before = s.compute_accelerations(pos, mass)
+        s.ic_merger(4000, seed=3)
+        used = s.download()
+        again = s.compute_accelerations(pos, mass)
+    with ogx.AdaptiveFMM3D(**kw) as s:
+        s.upload(pos, vel, mass)
+        s.ic_merger(4000, seed=3)
+        uploaded = s.download()
+    for a, b, c in zip(fresh, used, uploaded):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
+    assert np.array_equal(before, again)
+
+
+@pytest.mark.gpu
 def test_diagnostics_match_host_sums_and_direct_potential_energy(ogx, oracle):
     n_per = 3000
     with ogx.AdaptiveFMM3D(eps=0.0, p=8, threshold=32) as s:
