@@ -25,9 +25,13 @@ FMM_TOL = 1e-12
 
 
 @pytest.fixture(scope="module")
-def reference():
-    from oracle_lib import Reference
-    return Reference()
+def reference(oracle):
+    """The reference's own octree where its sources were present at build time, else the oracle's,
+    which equals it box for box and list for list (test_oracle_pins.py)."""
+    import os
+
+    from oracle_lib import REF_SO, Reference
+    return Reference() if os.path.exists(REF_SO) else oracle
 
 
 @pytest.fixture(scope="module")
