@@ -46,42 +46,21 @@ template <class T> struct Vec;
 template <> struct Vec<float> { using V = f2; static constexpr int W = 2; };
 template <> struct Vec<double> { using V = double; static constexpr int W = 1; };
 
-// box centre: FP64, or relative to the root centre as hi + lo FP32
-template <class T> struct Center;
-template <> struct Center<double> {
+// A body's offset from the box centre is one FP64 difference, scaled in FP64 and rounded to T
+// once: taken from the near field's hi + lo FP32 pairs it carried three FP32 roundings.
+template <class T>
+struct Center {
     double c[3], inv;
     __device__ __forceinline__ Center(const TreeView& tv, int b) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) c[a] = tv.center[4 * (size_t)b + a];
         inv = 1.0 / (2.0 * tv.center[4 * (size_t)b + 3]);
     }
-    __device__ __forceinline__ void body(const TreeView& tv, int i, double& x, double& y, double& z, double& q) const {
-        x = (tv.px[i] - c[0]) * inv;
-        y = (tv.py[i] - c[1]) * inv;
-        z = (tv.pz[i] - c[2]) * inv;
-        q = tv.pm[i];
-    }
-};
-template <> struct Center<float> {
-    float h[3], l[3], inv, inv_lo;
-    __device__ __forceinline__ Center(const TreeView& tv, int b) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const double v = tv.center[4 * (size_t)b + a] - tv.root->c[a];
-            h[a] = (float)v;
-            l[a] = (float)(v - (double)h[a]);
-        }
-        const double v = 1.0 / (2.0 * tv.center[4 * (size_t)b + 3]);
-        inv = (float)v;
-        inv_lo = (float)(v - (double)inv);
-    }
-    __device__ __forceinline__ float scaled(float d) const { return fmaf(d, inv, d * inv_lo); }
-    __device__ __forceinline__ void body(const TreeView& tv, int i, float& x, float& y, float& z, float& q) const {
-        const float4 a = __ldg(tv.rhi + i), b = __ldg(tv.rlo + i);
-        x = scaled((a.x - h[0]) + (b.x - l[0]));
-        y = scaled((a.y - h[1]) + (b.y - l[1]));
-        z = scaled((a.z - h[2]) + (b.z - l[2]));
-        q = a.w;
+    __device__ __forceinline__ void body(const TreeView& tv, int i, T& x, T& y, T& z, T& q) const {
+        x = (T)((tv.px[i] - c[0]) * inv);
+        y = (T)((tv.py[i] - c[1]) * inv);
+        z = (T)((tv.pz[i] - c[2]) * inv);
+        q = (T)tv.pm[i];
     }
 };
 
