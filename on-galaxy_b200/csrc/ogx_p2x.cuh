@@ -11,7 +11,7 @@
 // holds NB bodies of a chunk at a time (FP32: in f32x2 pairs), walks the columns m and adds
 // its bodies' terms of one (n, m) at once, so no lane keeps the K sums (81 registers a lane
 // at p = 8, and another kernel that staged whole rows above p = 9); the lanes' sums meet in
-// FP64 through shared memory.
+// FP64 through shared memory, in FP32 after every 32 bodies of a lane at the latest.
 // The bodies of the X list's leaves form one flat sequence (lane e of a group of 32 entries
 // holds entry e; a scan of the counts maps positions to entries), so all lanes are busy
 // however the leaves are sized and a chunk's loads are in flight together.
@@ -181,6 +181,27 @@ __global__ void __launch_bounds__(32) k_p2x(TreeView tv, int ntargets, double* _
     const Center<T> cen(tv, b);
     bool first = true;
     int cols = sums<T>();   // columns of s_red in use
+    // The columns' sums, in FP64: added up at the end, and in FP32 after every 32 bodies of a
+    // column too (lane = coefficients lane, lane + 32, ...), so that a chain of FP32 additions
+    // is no longer in a leaf of thousands of bodies than in one of a thousand.
+    constexpr int NPL = (K + 31) / 32, FLUSH = 32 / NB;
+    double sum[NPL];
+#pragma unroll
+    for (int u = 0; u < NPL; ++u) sum[u] = 0.0;
+    auto flush = [&]() {
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < NPL; ++u) {
+            const int d = lane + 32 * u;
+            if (d < K) {
+#pragma unroll 8
+                for (int r = 0; r < cols; ++r) sum[u] += (double)s_red[d * LD + r];
+            }
+        }
+        __syncwarp();   // the next chunk overwrites the columns
+        first = true;
+    };
+    int held = 0;           // chunks in the columns
     for (int64_t eb = e0; eb < e1; eb += 32) {
         int pf = 0, pc = 0;
         if (MODE == 0) {
@@ -220,17 +241,19 @@ __global__ void __launch_bounds__(32) k_p2x(TreeView tv, int ntargets, double* _
             if (MODE == 0 && sizeof(T) == 4 && first) cols = min(sums<T>(), (total + NB - 1) / NB);
             add_chunk<P, MODE == 1, T, NB>(x, y, z, q, s_red, lane, first);
             first = false;
+            if (sizeof(T) == 4 && ++held == FLUSH) {
+                flush();
+                held = 0;
+            }
         }
     }
-    __syncwarp();
+    if (!first) flush();
     const double scale = MODE == 1 ? 1.0 / (2.0 * tv.center[4 * (size_t)b + 3]) : 1.0;
-    for (int d = lane; d < K; d += 32) {
-        double v = 0.0;
-        if (!first) {
-#pragma unroll 8
-            for (int r = 0; r < cols; ++r) v += (double)s_red[d * LD + r];
-        }
-        v *= __ldg(&g_harm.sd[d]);   // s_nm, negative for the imaginary part (the conjugate)
+#pragma unroll
+    for (int u = 0; u < NPL; ++u) {
+        const int d = lane + 32 * u;
+        if (d >= K) continue;
+        const double v = sum[u] * __ldg(&g_harm.sd[d]);   // s_nm, negative for the imaginary part (the conjugate)
         if (MODE == 0) out[(size_t)b * K + d] = v;
         else out[(size_t)b * K + d] += v * scale;
     }

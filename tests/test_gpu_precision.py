@@ -15,6 +15,44 @@ def _rms(ref, got):
     return float(np.sqrt(((got - ref) ** 2).sum() / (ref ** 2).sum()))
 
 
+@pytest.mark.parametrize("p", [4, 8, 12])
+def test_leaf_of_many_thousand_bodies(ogx, p):
+    """60,000 bodies of one mass in one leaf (the eps floor) act on massless bodies far away, so
+    every force goes through the leaf's P2M sums.  A chain of 32 FP32 additions of equal terms is
+    off by at most 4.9e-7 (16.5 half ulps), its bodies' masses by 6e-8, the translations by 4e-7
+    in the same direction at worst: 1e-6.  One FP32 chain over the whole leaf gave 6.5e-6."""
+    rng = np.random.default_rng(p)
+    pos = np.concatenate([[0.31, -0.27, 0.44] + 0.02 * (rng.random((60000, 3)) - 0.5),
+                          [-0.6, 0.55, -0.3] + 0.8 * (rng.random((3000, 3)) - 0.5)])
+    mass = np.concatenate([np.full(60000, 1.0 / 60000), np.zeros(3000)])
+    out = {}
+    for form in (ogx.PREC_FP64, ogx.PREC_MIXED):
+        with ogx.AdaptiveFMM3D(p=p, threshold=64, eps=0.25, precision=form) as s:
+            acc, pot = s.compute_accelerations(pos, mass, with_potential=True)
+            assert s.stats()["max_leaf_occupancy"] >= 60000
+        out[form] = acc[60000:], pot[60000:]
+    for a, b in zip(out[ogx.PREC_FP64], out[ogx.PREC_MIXED]):
+        assert _rms(a, b) <= 1e-6
+
+
+@pytest.mark.parametrize("p", [4, 12])
+def test_x_lists_of_many_thousand_bodies(ogx, p):
+    """Leaves of up to 4,096 bodies round a deep cluster of massless ones: P2L over X lists of
+    thousands of bodies, and heavy leaves' M2P the other way.  5e-7: chains of 32 FP32 additions
+    and the translations, as above (random terms: 1e-7 measured at p = 4)."""
+    rng = np.random.default_rng(p)
+    pos = np.concatenate([2.0 * rng.random((120000, 3)) - 1.0,
+                          [0.21, -0.13, 0.32] + 0.004 * rng.standard_normal((20000, 3))])
+    mass = np.concatenate([np.full(120000, 1.0 / 120000), np.zeros(20000)])
+    out = []
+    for form in (ogx.PREC_FP64, ogx.PREC_MIXED):
+        with ogx.AdaptiveFMM3D(p=p, threshold=4096, precision=form) as s:
+            out.append(s.compute_accelerations(pos, mass, with_potential=True))
+            assert s.stats()["p2l_evals"] > 100000
+    for a, b in zip(*out):
+        assert _rms(a[120000:], b[120000:]) <= 5e-7
+
+
 @pytest.mark.parametrize("kind, n, p, thr, eps", [("plummer", 8192, 6, 64, 0.0), ("galaxy", 60000, 8, 64, 0.0), ("galaxy", 60000, 8, 64, 0.05),
                                                   ("cube", 20000, 10, 128, 0.0), ("plummer", 20000, 12, 64, 0.0)])
 def test_mixed_form_keeps_its_bits(ogx, kind, n, p, thr, eps):
