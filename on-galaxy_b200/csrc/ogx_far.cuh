@@ -273,80 +273,38 @@ struct alignas(16) WarpSmem {
     static constexpr int RF4 = Rec<T, P + 1, POT>::F4;
     float4 rec[FAR_RW * RF4];
     typename Res<T>::V res[32 * NB];
-    double hdr[FAR_RW][4];       // FP64: box centre, 1 / side; FP32: floats {offset xyz, scale, 1 / side}
+    double hdr[FAR_RW][4];       // box centre, 1 / side
 };
 
-// bodies of a block relative to the leaf centre: FP64 (x - c); FP32 ((x - c) / side) as hi + lo
-template <class T> struct Bodies;
-template <> struct Bodies<double> { double x[3][64]; };
-template <> struct Bodies<float> { float h[3][64], l[3][64]; };
+// Positions of a block's bodies.  An offset from a box is one FP64 difference, scaled in FP64
+// and rounded to T once: through the leaf's centre it took two roundings, the first
+// magnified by the ratio of the sides for a W box many levels below its leaf.
+struct Bodies { double x[3][64]; };
 
-__device__ __forceinline__ void put_body(Bodies<double>& s, int j, double x, double y, double z, double) {
-    s.x[0][j] = x; s.x[1][j] = y; s.x[2][j] = z;
-}
-__device__ __forceinline__ void put_body(Bodies<float>& s, int j, double x, double y, double z, double inv) {
-    const double v[3] = {x * inv, y * inv, z * inv};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float h = (float)v[a];
-        s.h[a][j] = h;
-        s.l[a][j] = (float)(v[a] - (double)h);
-    }
-}
-
-// W box header, written by one lane per box.  FP32: the box's centre offset from the leaf in
-// its own side (a small dyadic number, exact), and the ratio of the sides (a power of two,
-// 2^up; winv = 2^up / side of the leaf is exact too, where a division took thirty operations)
-__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double winv, int,
-                                           double) {
-    h[0] = cx - c01.x; h[1] = cy - c01.y; h[2] = cz - c23.x; h[3] = winv;
-}
-__device__ __forceinline__ void put_header(double (&h)[4], double2 c01, double2 c23, double cx, double cy, double cz, double winv,
-                                           int up, float) {
-    float* f = reinterpret_cast<float*>(h);
-    f[0] = (float)((cx - c01.x) * winv);
-    f[1] = (float)((cy - c01.y) * winv);
-    f[2] = (float)((cz - c23.x) * winv);
-    f[3] = __int_as_float((127 + up) << 23);   // 0 <= up <= 24
-    f[4] = (float)winv;
-}
-// v * 2^up
+// 1 / side of a W box `up` levels below one of 1 / side = v: v * 2^up, exact (a division takes
+// thirty operations)
 __device__ __forceinline__ double scale2(double v, int up) { return v * __hiloint2double((1023 + up) << 20, 0); }
 
 // results of the bodies j[k] for a W box
-template <int L, bool POT, int NB>
-__device__ __forceinline__ void m2p_task(const float4* rec, const double (&h)[4], const Bodies<double>& s, const int (&j)[NB],
-                                         double4 (&res)[NB]) {
-    const double w = h[3], w2 = w * w;
-    double u[3][NB], o[NB][4];
+template <class T, int L, bool POT, int NB>
+__device__ __forceinline__ void m2p_task(const float4* rec, const double (&h)[4], const Bodies& s, const int (&j)[NB],
+                                         typename Res<T>::V (&res)[NB]) {
+    const T w = (T)h[3], w2 = w * w;
+    T u[3][NB], o[NB][4];
 #pragma unroll
     for (int k = 0; k < NB; ++k)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) u[a][k] = (s.x[a][j[k]] + h[a]) * w;
+        for (int a = 0; a < 3; ++a) u[a][k] = (T)((s.x[a][j[k]] - h[a]) * h[3]);
     eval<L, POT, true, NB>(rec, u[0], u[1], u[2], o);
 #pragma unroll
-    for (int k = 0; k < NB; ++k) res[k] = make_double4(o[k][0] * w2, o[k][1] * w2, o[k][2] * w2, POT ? o[k][3] * w : 0.0);
-}
-template <int L, bool POT, int NB>
-__device__ __forceinline__ void m2p_task(const float4* rec, const double (&hd)[4], const Bodies<float>& s, const int (&j)[NB],
-                                         float4 (&res)[NB]) {
-    const float* h = reinterpret_cast<const float*>(hd);
-    const float sc = h[3], w = h[4], w2 = w * w;
-    float u[3][NB], o[NB][4];
-#pragma unroll
-    for (int k = 0; k < NB; ++k)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) u[a][k] = fmaf(s.l[a][j[k]], sc, fmaf(s.h[a][j[k]], sc, h[a]));
-    eval<L, POT, true, NB>(rec, u[0], u[1], u[2], o);
-#pragma unroll
-    for (int k = 0; k < NB; ++k) res[k] = make_float4(o[k][0] * w2, o[k][1] * w2, o[k][2] * w2, POT ? o[k][3] * w : 0.f);
+    for (int k = 0; k < NB; ++k) res[k] = typename Res<T>::V{o[k][0] * w2, o[k][1] * w2, o[k][2] * w2, POT ? o[k][3] * w : T(0)};
 }
 
 // The rounds first, first + stride, ... of a block of nbk bodies and nw W boxes; every body
 // sums its own task results in task order into acc (FP64; lane owns bodies lane, lane + 32).
 template <int P, bool POT, int NB, class T>
 __device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restrict__ hrec, int64_t w0, int nw, int nbk, int first,
-                                           int stride, const Bodies<T>& sb, double cx, double cy, double cz, double inv, int level,
+                                           int stride, const Bodies& sb, double inv, int level,
                                            WarpSmem<P, POT, T, NB>& sm, int lane, double (&acc)[2][4]) {
     using R = Rec<T, P + 1, POT>;
     constexpr int RF4 = R::F4;
@@ -378,7 +336,8 @@ __device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restri
             const double2 c01 = __ldg(reinterpret_cast<const double2*>(tv.center) + 2 * (size_t)c);
             const double2 c23 = __ldg(reinterpret_cast<const double2*>(tv.center) + 2 * (size_t)c + 1);
             const int up = __ldg(tv.level + c) - level;
-            put_header(sm.hdr[lane], c01, c23, cx, cy, cz, scale2(inv, up), up, T(0));
+            double* hd = sm.hdr[lane];
+            hd[0] = c01.x; hd[1] = c01.y; hd[2] = c23.x; hd[3] = scale2(inv, up);
         }
         const int wr = w - wa, jr = j, ja = __shfl_sync(0xffffffffu, j, 0), ntr = nt;
         b0 += stride * Q;
@@ -394,7 +353,7 @@ __device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restri
             typename Res<T>::V v[NB];
 #pragma unroll
             for (int k = 0; k < NB; ++k) jb[k] = jr + k * nt1 < nbk ? jr + k * nt1 : jr;
-            m2p_task<P + 1, POT, NB>(sm.rec + wr * RF4, sm.hdr[wr], sb, jb, v);
+            m2p_task<T, P + 1, POT, NB>(sm.rec + wr * RF4, sm.hdr[wr], sb, jb, v);
 #pragma unroll
             for (int k = 0; k < NB; ++k) sm.res[32 * k + lane] = v[k];
         }
@@ -417,7 +376,8 @@ __device__ __forceinline__ void m2p_rounds(const TreeView& tv, const T* __restri
 
 // L2P of the block's bodies (lane owns bodies lane and lane + 32)
 template <int P, bool POT, class T>
-__device__ __forceinline__ void l2p_block(const T* __restrict__ g, int nbk, const Bodies<T>& sb, double inv, float4* srec, int lane,
+__device__ __forceinline__ void l2p_block(const T* __restrict__ g, int nbk, const Bodies& sb, double cx, double cy, double cz,
+                                          double inv, float4* srec, int lane,
                                           double (&acc)[2][4]) {
     constexpr int L = rec_degree<P, 1, POT>();
     using R = Rec<T, L, POT>;
@@ -428,12 +388,7 @@ __device__ __forceinline__ void l2p_block(const T* __restrict__ g, int nbk, cons
     for (int q = 0; q < 2; ++q) {
         const int j = lane + 32 * q;
         if (j < nbk) {
-            T u[3][1], o[1][4];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if constexpr (sizeof(T) == 4) u[a][0] = sb.h[a][j];
-                else u[a][0] = sb.x[a][j] * inv;
-            }
+            T u[3][1] = {{(T)((sb.x[0][j] - cx) * inv)}, {(T)((sb.x[1][j] - cy) * inv)}, {(T)((sb.x[2][j] - cz) * inv)}}, o[1][4];
             eval<L, POT, false, 1>(srec, u[0], u[1], u[2], o);
             acc[q][0] += (double)o[0][0] * inv;
             acc[q][1] += (double)o[0][1] * inv;
@@ -453,7 +408,7 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? 20 : 12) k_leaf_far(TreeV
                                                                            const T* __restrict__ grec, double* __restrict__ far) {
     using GR = Rec<T, rec_degree<P, 1, POT>(), POT>;
     extern __shared__ __align__(16) unsigned char s_far_dyn[];
-    __shared__ Bodies<T> sb;
+    __shared__ Bodies sb;
     const int lane = threadIdx.x;
     const int lf = blockIdx.x;
     if (lf >= tv.nleaf || lf >= tv_nleaf(tv) || tv_over(tv)) return;
@@ -471,15 +426,15 @@ __global__ void __launch_bounds__(32, sizeof(T) == 4 ? 20 : 12) k_leaf_far(TreeV
             __syncwarp();
             for (int j = lane; j < nbk; j += 32) {
                 const int i = f0 + jb + j;
-                put_body(sb, j, tv.px[i] - cx, tv.py[i] - cy, tv.pz[i] - cz, inv);
+                sb.x[0][j] = tv.px[i]; sb.x[1][j] = tv.py[i]; sb.x[2][j] = tv.pz[i];
             }
             __syncwarp();
         }
         if constexpr (DO_L2P)
-            l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, inv, reinterpret_cast<float4*>(s_far_dyn), lane, acc);
+            l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, cx, cy, cz, inv, reinterpret_cast<float4*>(s_far_dyn), lane, acc);
         if constexpr (DO_M2P)
             if (nw > 0)
-                m2p_rounds<P, POT, 1, T>(tv, hrec, w0, nw, nbk, 0, 1, sb, cx, cy, cz, inv, tv.level[b],
+                m2p_rounds<P, POT, 1, T>(tv, hrec, w0, nw, nbk, 0, 1, sb, inv, tv.level[b],
                                          *reinterpret_cast<WarpSmem<P, POT, T, 1>*>(s_far_dyn), lane, acc);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
@@ -519,7 +474,7 @@ __global__ void __launch_bounds__(32 * FAR_HW, 2) k_leaf_far_heavy(TreeView tv, 
                                                                                        const int* __restrict__ list, int* ctr) {
     using GR = Rec<T, rec_degree<P, 1, POT>(), POT>;
     extern __shared__ __align__(16) unsigned char s_far_dyn[];
-    __shared__ Bodies<T> sb;
+    __shared__ Bodies sb;
     __shared__ int s_lf;
     double* s_part = reinterpret_cast<double*>(s_far_dyn);   // [FAR_HW][64][4], over the records once the rounds are done
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -545,13 +500,13 @@ __global__ void __launch_bounds__(32 * FAR_HW, 2) k_leaf_far_heavy(TreeView tv, 
             __syncthreads();
             for (int j = threadIdx.x; j < nbk; j += blockDim.x) {
                 const int i = f0 + jb + j;
-                put_body(sb, j, tv.px[i] - cx, tv.py[i] - cy, tv.pz[i] - cz, inv);
+                sb.x[0][j] = tv.px[i]; sb.x[1][j] = tv.py[i]; sb.x[2][j] = tv.pz[i];
             }
             __syncthreads();
             double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
             if constexpr (DO_L2P)
-                if (wid == 0) l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, inv, sm.rec, lane, acc);
-            m2p_rounds<P, POT, FAR_HEAVY_NB<T>, T>(tv, hrec, w0, nw, nbk, wid, FAR_HW, sb, cx, cy, cz, inv, tv.level[b], sm, lane, acc);
+                if (wid == 0) l2p_block<P, POT, T>(grec + (size_t)lf * GR::SIZE, nbk, sb, cx, cy, cz, inv, sm.rec, lane, acc);
+            m2p_rounds<P, POT, FAR_HEAVY_NB<T>, T>(tv, hrec, w0, nw, nbk, wid, FAR_HW, sb, inv, tv.level[b], sm, lane, acc);
             __syncthreads();
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
