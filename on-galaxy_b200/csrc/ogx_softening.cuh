@@ -29,8 +29,9 @@ __device__ __forceinline__ void spline_inside(T u, T iu, T hinv, T& g, T& k) {
 
 template <class T>
 __device__ __forceinline__ void spline_gk(T r2, T h, T hinv, T& g, T& k) {
-    // FP32: 1/r from rsqrtf and one Newton step gives r = r2 / r and 1/u = h / r without the
-    // square root and the division (a third of the pair)
+    // FP32: 1/r from rsqrtf and one Newton step gives r and 1/u = h / r without the square root
+    // and the division (a third of the pair).  r takes the residual r2 - r^2 as well, which
+    // rounds it correctly but for ties; 1/u carries two roundings where 1 / (r hinv) has three.
     if constexpr (sizeof(T) == 4) {
         T y = rsqrtf(r2);
         if (r2 >= h * h) {
@@ -39,8 +40,8 @@ __device__ __forceinline__ void spline_gk(T r2, T h, T hinv, T& g, T& k) {
             return;
         }
         y = fmaf(y, T(0.5) * fmaf(-r2 * y, y, T(1)), y);
-        const T r = r2 > T(0) ? r2 * y : T(0);
-        spline_inside<T>(r * hinv, h * y, hinv, g, k);
+        const T r = r2 * y;
+        spline_inside<T>(r2 > T(0) ? fmaf(fmaf(-r, r, r2), T(0.5) * y, r) * hinv : T(0), h * y, hinv, g, k);
     } else {
         if (r2 >= h * h) {
             const T y = rsqrt(r2);
