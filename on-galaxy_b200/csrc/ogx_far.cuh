@@ -201,8 +201,10 @@ __device__ __forceinline__ void eval(const float4* rec, double (&xs)[NB], double
     double x = xs[0], y = ys[0], z = zs[0], (&out)[4] = outs[0];
     double kap = x * x + y * y + z * z, dr = 1.0, di = 0.0;
     if (SING) {
-        dr = rsqrt(kap);
+        const double r2 = kap;
+        dr = rsqrt(r2);
         kap = dr * dr;
+        kap = fma(kap, fma(-r2, kap, 1.0), kap);   // 1 / r2 to half an ulp: degree n carries its n-th power
         x *= kap; y *= kap; z *= kap;
     }
 #pragma unroll

@@ -91,7 +91,9 @@ __device__ __forceinline__ void add_chunk(const T (&x)[NB], const T (&y)[NB], co
                 T ir;
                 if constexpr (sizeof(T) == 4) ir = rsqrtf(r2); else ir = rsqrt(r2);
                 w *= ir;
-                r2 = ir * ir;
+                const T k2 = ir * ir;
+                // FP64: 1 / r2 to half an ulp, as in ogx_far.cuh
+                if constexpr (sizeof(T) == 8) r2 = fma(k2, fma(-r2, k2, T(1)), k2); else r2 = k2;
                 a[i] *= r2; b[i] *= r2; c[i] *= r2;
             }
             nb[i] = -b[i];
