@@ -137,14 +137,23 @@ uint64_t fnv1a(const void* data, size_t bytes, uint64_t h = 1469598103934665603u
     return h;
 }
 
-// admission estimate of a job's device footprint: the per-order operator tables
-// (343 M2L matrices of K^2 doubles and the mixed form's padded FP16 hi/lo images,
-// 20 bytes per matrix entry together, with slack) and per body its coordinates,
-// keys, tree, lists and expansions; measured peaks sit below it by 20-50% from
-// 16k to 200k bodies at p = 6, 8 and 12
-double footprint_bytes(int64_t n, int p) {
+// Admission estimate of a job's device footprint: the operator tables of its order and form (a
+// merger's circular velocities take the plain form's 343 M2L operators whatever the job's form
+// is), the partial rows of the M2L's slot ranges (a bound, csrc/ogx_m2l64.cuh), and per body and
+// per box what the arrays of the evaluation take, growth slack included; 4.0 to 4.6
+// boxes per leaf capacity of bodies were measured, 5 are taken.  Measured peaks of 156 jobs (n
+// from 7,000 to 575,000, p = 4, 8, 12, leaf capacities 32 and 64, three forms) lie between 0.44
+// and 0.87 of it; without the leaf capacity and the rows they reached 1.5 times it.
+double footprint_bytes(int64_t n, int p, int leaf_capacity, int precision, bool merger) {
     const double K = (double)(p + 1) * (p + 1);
-    return 48e6 + 343.0 * K * K * 20.0 + (double)n * (1300.0 + 1.5 * K);
+    const double op = (double)(((int)K + 3) / 4 * 4) * (((int)K + 7) / 8 * 8 + 4) * 8.0;   // one padded FP64 operator
+    double tables = 16.0 * op;
+    if (precision == OGX_PREC_FP64 || merger) tables += 343.0 * op;
+    if (precision == OGX_PREC_MIXED) tables += 343.0 * (K + 16.0) * (K + 64.0) * 5.0;      // FP16 hi and lo images, padded
+    if (precision == OGX_PREC_FP64_ROT) tables += 343.0 * (p + 1.0) * (2 * p + 3.0) * (9 * p + 6.0) * (8.0 / 6.0);
+    const double boxes = 5.0 * (double)n / leaf_capacity + 64.0;
+    const double rows = std::min(27.0 * boxes, 56832.0 + std::min(boxes, 56832.0)) * K * 9.0;   // 8 bytes and an eighth
+    return 10e6 + tables + rows + (double)n * 700.0 + boxes * (2400.0 + K * (precision == OGX_PREC_MIXED ? 80.0 : 106.0));
 }
 
 bool g_capture = false;   // --capture: every job replays its captured step (ogx_tuning.capture_steps)
@@ -587,7 +596,7 @@ int main(int argc, char** argv) {
         // lockstep ensemble: every system takes step s before any takes step s + 1
         std::vector<Job*> live;
         for (Job& jb : jobs) {
-            jb.need_bytes = footprint_bytes(jb.n, jb.p);
+            jb.need_bytes = footprint_bytes(jb.n, jb.p, autotune ? std::min(jb.thr, 32) : jb.thr, precision, jb.kind == 1);
             if (in_use + jb.need_bytes > budget) {
                 jb.rejected = true;
                 jb.status = OGX_ERR_INVALID;
@@ -708,7 +717,7 @@ int main(int argc, char** argv) {
     if (!solo) start_pool();
     int admitted = 0;
     for (Job& jb : jobs) {
-        jb.need_bytes = footprint_bytes(jb.n, jb.p);
+        jb.need_bytes = footprint_bytes(jb.n, jb.p, autotune ? std::min(jb.thr, 32) : jb.thr, precision, jb.kind == 1);
         if (jb.need_bytes > budget) {
             // could never fit, even alone: refused at admission, the loop goes on
             jb.rejected = true;

@@ -74,6 +74,21 @@ def test_jobs_give_the_same_bits_alone_and_in_the_mix():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision, thr, extra", [("mixed", 32, ()), ("mixed", 128, ("--capture",)), ("fp64", 32, ()),
+                                                   ("fp64", 64, ("--eps", 0.05, "--softening", "spline")), ("fp64rot", 32, ())])
+def test_the_admission_estimate_covers_every_form_and_leaf_capacity(precision, thr, extra):
+    """Small leaves mean more boxes, a merger needs the plain form's operators whatever its form,
+    and the M2L's partial rows are bounded by the boxes: one job's peak stays below its estimate,
+    and the estimate of a large job below three times its peak."""
+    out = _serve("--jobs", 8, "--rate", 2000, "--solo", "--smin", 1, "--smax", 2, "--nmin", 8000, "--nmax", 320000,
+                 "--orders", "4,8,12", "--seed", 21, "--precision", precision, "--thr", thr, *extra)
+    assert out["failed"] == 0 and out["rejected"] == 0
+    for j in out["jobs_detail"]:
+        assert j["peak_mb"] <= j["need_mb"], j
+        assert j["n"] < 50000 or j["need_mb"] <= 3.0 * j["peak_mb"], j
+
+
+@pytest.mark.gpu
 def test_jobs_above_the_budget_are_refused_and_the_rest_run():
     out = _serve("--jobs", 6, "--rate", 400, "--nmin", 16384, "--nmax", 1 << 20, "--smin", 2, "--smax", 3,
                  "--orders", "8", "--seed", 3, "--hbm-gb", 0.4)
