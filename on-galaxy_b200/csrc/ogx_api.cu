@@ -18,7 +18,6 @@
 #include <mutex>
 #include <thread>
 
-#include "ogx_harmonics.cuh"
 #include "ogx_m2l64.cuh"
 #include "ogx_sm100.cuh"
 

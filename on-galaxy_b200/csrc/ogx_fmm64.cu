@@ -34,8 +34,6 @@ namespace ogx {
 
 namespace {
 
-constexpr unsigned FULL = 0xffffffffu;
-
 // ---- leaf far field (ogx_far.cuh): coefficient records, then M2P over the W lists and L2P.
 // The mixed form's M2P part (L2P = false) needs only the multipoles, so it runs on the side
 // stream beside the M2L and the downward pass; the plain form takes both parts in one.

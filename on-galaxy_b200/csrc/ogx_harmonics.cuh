@@ -1,17 +1,18 @@
-// ogx_harmonics.cuh -- solid harmonics and expansion-coefficient helpers.
+// ogx_harmonics.cuh -- solid-harmonic constants and the layout of expansion coefficients.
 //
 // The reference evaluates Y_n^m through cos/sin/atan2 and the seminormalised
 // Legendre recurrence (src3d/FmmExpansions3D.hpp:75-107) and multiplies by
-// rho^n or rho^-(n+1) afterwards.  Here the same functions are generated
-// directly as solid harmonics in Cartesian form, column by column in m, so a
-// thread never holds more than the current column:
+// rho^n or rho^-(n+1) afterwards.  As solid harmonics in Cartesian form the same
+// functions are
 //   R_n^m = rho^n Y_n^m:           R_m^m = (x+iy) a_m R_{m-1}^{m-1}
 //                                  R_{m+1}^m = z b_m R_m^m
 //                                  R_n^m = z A_nm R_{n-1}^m - r^2 B_nm R_{n-2}^m
 //   S_n^m = Y_n^m / rho^{n+1}:     same recurrences with a factor 1/r^2 per step
 // with a_m = sqrt((2m-1)/2m), b_m = sqrt(2m+1), A_nm = (2n-1)/sqrt(n^2-m^2),
 // B_nm = sqrt((n-1)^2-m^2)/sqrt(n^2-m^2): the reference's Q recurrence
-// multiplied through by rho^n e^{i m phi} (no trigonometric calls).
+// multiplied through by rho^n e^{i m phi} (no trigonometric calls).  The kernels take them
+// as R_n^m = s_nm (x+iy)^m T_nm with real polynomials T_nm of leading coefficient 1
+// (ogx_far.cuh, ogx_p2x.cuh); only the products s_nm of a, b and A are kept here.
 //
 // Real coefficient layout (K = (p+1)^2 doubles): dof(n,0) = n^2,
 // dof(n,m>0) = n^2 + 2m - 1 (real part), n^2 + 2m (imaginary part).
@@ -28,19 +29,13 @@ namespace ogx {
 constexpr int kTab = kDegMax + 2;
 
 struct HarmTables {
-    double a[kTab];
-    double b[kTab];
-    double A[kTab][kTab];
-    double B[kTab][kTab];
     // gradient-coefficient constants (derivative recurrences of FmmExpansions3D.hpp:111-129)
     double gz[kTab][kTab], gp[kTab][kTab], gm[kTab][kTab];  // local  -> degree n (from degree n+1)
     double hz[kTab][kTab], hp[kTab][kTab], hm[kTab][kTab];  // mpole  -> degree n (from degree n-1)
-    // R_n^m = s[n][m] (x+iy)^m T_nm: the product of the recurrence constants (ogx_far.cuh)
+    // R_n^m = s[n][m] (x+iy)^m T_nm: the product of the recurrence constants a, b, A (ogx_far.cuh)
     double s[kTab][kTab];
     // the same per real dof, negative for imaginary parts (conjugate sums, ogx_p2x.cuh)
     double sd[(kPMax + 1) * (kPMax + 1)];
-    // FP32 copies of the recurrence constants for the FP32 kernels (no conversion per use)
-    float fa[kTab], fb[kTab], fA[kTab][kTab], fB[kTab][kTab];
 };
 
 // the reference's derivative coefficients (FmmExpansions3D.hpp:111-129)
@@ -53,30 +48,14 @@ inline double ref_dm_S(int n, int m) { return ((m > 0) ? 1.0 : -1.0) * std::sqrt
 
 // One copy per translation unit (whole-program compilation, no device linking);
 // every unit that launches harmonic kernels calls harm_tables_ready() first.
-static __constant__ HarmTables c_harm;
-// the same tables in global memory, for kernels whose lanes index them divergently
-// (the constant cache serialises lanes that read different addresses)
+// In global memory: the kernels' lanes index them divergently (the constant cache serialises
+// lanes that read different addresses).
 static __device__ HarmTables g_harm;
 
 static inline void fill_harm_tables(HarmTables& t) {
     t = HarmTables{};
-    for (int m = 0; m < kTab; ++m) {
-        t.a[m] = m > 0 ? std::sqrt((2.0 * m - 1.0) / (2.0 * m)) : 1.0;
-        t.b[m] = std::sqrt(2.0 * m + 1.0);
-    }
-    for (int m = 0; m < kTab; ++m) {
-        t.fa[m] = (float)t.a[m];
-        t.fb[m] = (float)t.b[m];
-    }
     for (int n = 0; n < kTab; ++n)
         for (int m = 0; m < kTab; ++m) {
-            if (n >= m + 2) {
-                const double d = std::sqrt((double)(n * n - m * m));
-                t.A[n][m] = (2.0 * n - 1.0) / d;
-                t.B[n][m] = std::sqrt((double)((n - 1) * (n - 1) - m * m)) / d;
-                t.fA[n][m] = (float)t.A[n][m];
-                t.fB[n][m] = (float)t.B[n][m];
-            }
             if (m <= n) {
                 // G_n^m from L_{n+1}^{m}, L_{n+1}^{m-1}, L_{n+1}^{m+1}
                 t.gz[n][m] = ref_cz_R(n + 1, m);
@@ -92,11 +71,11 @@ static inline void fill_harm_tables(HarmTables& t) {
         }
     double am = 1.0;
     for (int m = 0; m < kTab; ++m) {
-        am *= t.a[m];
+        am *= m > 0 ? std::sqrt((2.0 * m - 1.0) / (2.0 * m)) : 1.0;
         double v = am;
         for (int n = m; n < kTab; ++n) {
-            if (n == m + 1) v *= t.b[m];
-            else if (n > m + 1) v *= t.A[n][m];
+            if (n == m + 1) v *= std::sqrt(2.0 * m + 1.0);
+            else if (n > m + 1) v *= (2.0 * n - 1.0) / std::sqrt((double)(n * n - m * m));
             t.s[n][m] = v;
         }
     }
@@ -116,9 +95,8 @@ static inline int harm_tables_ready(int device) {
     if (done[device]) return OGX_OK;
     HarmTables t;
     fill_harm_tables(t);
-    cudaError_t e = cudaMemcpyToSymbol(c_harm, &t, sizeof(t));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_harm, &t, sizeof(t));
-    // the copies from the pageable t may still be in flight on the legacy stream,
+    cudaError_t e = cudaMemcpyToSymbol(g_harm, &t, sizeof(t));
+    // the copy from the pageable t may still be in flight on the legacy stream,
     // which the library's non-blocking streams do not wait for
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
@@ -130,90 +108,6 @@ static inline int harm_tables_ready(int device) {
 }
 
 __host__ __device__ __forceinline__ constexpr int dof_re(int n, int m) { return m == 0 ? n * n : n * n + 2 * m - 1; }
-
-// Visit R_n^m(x,y,z), n <= P (m >= 0), calling f(n, m, re, im) column by column.
-// recurrence constants in the arithmetic type (FP32 kernels read the FP32 copies)
-template <class T> __device__ __forceinline__ T harm_a(int m) {
-    if constexpr (sizeof(T) == 4) return c_harm.fa[m]; else return (T)c_harm.a[m];
-}
-template <class T> __device__ __forceinline__ T harm_b(int m) {
-    if constexpr (sizeof(T) == 4) return c_harm.fb[m]; else return (T)c_harm.b[m];
-}
-template <class T> __device__ __forceinline__ T harm_A(int n, int m) {
-    if constexpr (sizeof(T) == 4) return c_harm.fA[n][m]; else return (T)c_harm.A[n][m];
-}
-template <class T> __device__ __forceinline__ T harm_B(int n, int m) {
-    if constexpr (sizeof(T) == 4) return c_harm.fB[n][m]; else return (T)c_harm.B[n][m];
-}
-
-template <int P, class T, class F>
-__device__ __forceinline__ void for_regular(T x, T y, T z, F&& f) {
-    const T r2 = x * x + y * y + z * z;
-    T dr = 1, di = 0;  // R_m^m
-#pragma unroll
-    for (int m = 0; m <= P; ++m) {
-        if (m > 0) {
-            const T a = harm_a<T>(m);
-            const T nr = a * (x * dr - y * di), ni = a * (x * di + y * dr);
-            dr = nr;
-            di = ni;
-        }
-        f(m, m, dr, di);
-        if (m + 1 <= P) {
-            const T bz = harm_b<T>(m) * z;
-            T pr = dr, pi = di;              // R_{n-2}
-            T cr = bz * dr, ci = bz * di;    // R_{n-1}
-            f(m + 1, m, cr, ci);
-#pragma unroll
-            for (int n = m + 2; n <= P; ++n) {
-                const T A = harm_A<T>(n, m) * z, B = harm_B<T>(n, m) * r2;
-                const T qr = A * cr - B * pr, qi = A * ci - B * pi;
-                pr = cr; pi = ci; cr = qr; ci = qi;
-                f(n, m, cr, ci);
-            }
-        }
-    }
-}
-
-// Visit S_n^m(x,y,z), n <= P (m >= 0).  The origin is excluded by construction
-// (sources and targets of M2P/P2L are in well-separated boxes).
-template <int P, class T, class F>
-__device__ __forceinline__ void for_singular(T x, T y, T z, F&& f) {
-    const T r2 = x * x + y * y + z * z;
-    T ir2, dr, di = 0;         // dr = S_0^0 = 1/rho
-    if constexpr (sizeof(T) == 4) {
-        dr = rsqrtf(r2);       // FP32 path: one rsqrt instead of a division and a square root
-        ir2 = dr * dr;
-    } else {
-        ir2 = T(1) / r2;
-        dr = sqrt(ir2);
-    }
-    const T zr = z * ir2;      // FP32 path: one product per visit instead of two
-#pragma unroll
-    for (int m = 0; m <= P; ++m) {
-        if (m > 0) {
-            const T a = harm_a<T>(m) * ir2;
-            const T nr = a * (x * dr - y * di), ni = a * (x * di + y * dr);
-            dr = nr;
-            di = ni;
-        }
-        f(m, m, dr, di);
-        if (m + 1 <= P) {
-            const T bz = (sizeof(T) == 4) ? harm_b<T>(m) * zr : harm_b<T>(m) * z * ir2;
-            T pr = dr, pi = di;
-            T cr = bz * dr, ci = bz * di;
-            f(m + 1, m, cr, ci);
-#pragma unroll
-            for (int n = m + 2; n <= P; ++n) {
-                const T A = (sizeof(T) == 4) ? harm_A<T>(n, m) * zr : harm_A<T>(n, m) * z * ir2;
-                const T B = harm_B<T>(n, m) * ir2;
-                const T qr = A * cr - B * pr, qi = A * ci - B * pi;
-                pr = cr; pi = ci; cr = qr; ci = qi;
-                f(n, m, cr, ci);
-            }
-        }
-    }
-}
 
 // complex coefficient c_n^m from a real layout (m may be negative)
 template <class T>

@@ -53,7 +53,6 @@
 
 #include <cuda_fp16.h>
 
-#include "ogx_harmonics.cuh"
 #include "ogx_m2l64.cuh"
 #include "ogx_sm100.cuh"
 
