@@ -46,16 +46,6 @@ struct M64 {
     static_assert(SMEM <= 218 * 1024, "stages fit the SM");
 };
 
-// D (16 x 8) += A (16 x 4) B (4 x 8), FP64
-__device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double b) {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-                 : "d"(a0), "d"(a1), "d"(b));
-}
-__device__ __forceinline__ void cp_async8_zfill(void* sdst, const void* gsrc, uint32_t valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sm100::smem_u32(sdst)), "l"(gsrc), "r"(valid) : "memory");
-}
-
 template <int P>
 __global__ void __launch_bounds__(M64<P>::THREADS, M64<P>::MINB)
     k_m2l_fp64(TreeView tv, M2L64Args ar, const double* __restrict__ ops, const double* __restrict__ mpole, double* lown) {
@@ -167,7 +157,7 @@ __global__ void __launch_bounds__(M64<P>::THREADS, M64<P>::MINB)
                     const int r = i / C::KC, q = i - r * C::KC, kk = c * C::KC + q;
                     const int b = src[r];
                     const bool ok = b >= 0 && kk < K;
-                    if (q < kn) cp_async8_zfill(sa + r * C::LDA + q, ok ? mpole + (size_t)b * K + kk : mpole, ok ? 8u : 0u);
+                    if (q < kn) sm100::cp_async8_zfill(sa + r * C::LDA + q, ok ? mpole + (size_t)b * K + kk : mpole, ok ? 8u : 0u);
                 }
                 if (c == 0 && tid < M2L64_TGT) {   // sources of the next combination; the buffer's last reader was chunk u - 1
                     put_source(k + 1, src_next);
@@ -195,7 +185,7 @@ __global__ void __launch_bounds__(M64<P>::THREADS, M64<P>::MINB)
                 const double a0 = sa[k4], a1 = sa[k4 + 8 * C::LDA];
 #pragma unroll
                 for (int i = 0; i < C::NTW; ++i)
-                    dmma(acc[i], a0, a1, sb[k4 * C::LDN + 8 * i]);
+                    sm100::dmma(acc[i], a0, a1, sb[k4 * C::LDN + 8 * i]);
             };
             if (kn == C::KC) {
 #pragma unroll

@@ -21,10 +21,6 @@ namespace {
 
 constexpr int ROT_TGT = M2L64_TGT;   // targets per CTA
 
-__device__ __forceinline__ void cp_async8_zfill(void* sdst, const void* gsrc, uint32_t valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sm100::smem_u32(sdst)), "l"(gsrc), "r"(valid) : "memory");
-}
-
 // ---- M2L by rotations (the third form) ------------------------------------------------
 // T_o = Q_o^-1 Z_|o| Q_o (build_rot_pack): per tile of ROT_TGT targets sharing octant t
 // and per present (D, s) combination (offset o) the 64 source multipoles are staged,
@@ -246,7 +242,7 @@ __global__ void __launch_bounds__(RotCfg<P>::THREADS) k_m2l_rot(TreeView tv, M2L
             const int b = Q >= 0 ? __ldg(tv.child + 8 * (size_t)Q + ((code >> 5) & 7)) : -1;
             const double* src = mpole + (size_t)max(b, 0) * K;
             for (int kk = tid % (TH / ROT_TGT); kk < K; kk += TH / ROT_TGT)
-                cp_async8_zfill(dst + lr * LD + kk, src + kk, b >= 0 ? 8u : 0u);
+                sm100::cp_async8_zfill(dst + lr * LD + kk, src + kk, b >= 0 ? 8u : 0u);
         };
         double acc[RB][R::NACC];
 #pragma unroll

@@ -1,5 +1,5 @@
 // ogx_sm100.cuh -- thin inline-PTX helpers for sm_100a (mbarrier, cp.async,
-// bulk copy, tcgen05 MMA / TMEM).  Every wait is bounded: after kSpinLimit
+// bulk copy, FP64 MMA, tcgen05 MMA / TMEM).  Every wait is bounded: after kSpinLimit
 // polls it reports failure instead of spinning forever.
 #pragma once
 
@@ -53,6 +53,10 @@ __device__ __forceinline__ void cp_async16_zfill(void* sdst, const void* gsrc, u
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(sdst)), "l"(gsrc), "r"(bytes_valid)
                  : "memory");
 }
+// 8-byte cp.async reading `bytes_valid` (0 or 8) bytes and zero-filling the rest
+__device__ __forceinline__ void cp_async8_zfill(void* sdst, const void* gsrc, uint32_t bytes_valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(sdst)), "l"(gsrc), "r"(bytes_valid) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <int N>
@@ -71,6 +75,13 @@ __device__ __forceinline__ void bulk_g2s(void* sdst, const void* gsrc, uint32_t 
                      smem_u32(sdst)),
                  "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
+}
+
+// D (16 x 8) += A (16 x 4) B (4 x 8), FP64
+__device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a0), "d"(a1), "d"(b));
 }
 
 // ---- tcgen05 ------------------------------------------------------------------

@@ -67,13 +67,6 @@ __device__ __forceinline__ void publish(int* flag) {
     asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(flag) : "memory");
 }
 
-// D (16 x 8) += A (16 x 4) B (4 x 8), FP64
-__device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double b) {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
-                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-                 : "d"(a0), "d"(a1), "d"(b));
-}
-
 // one column part of a product: steps [k0, k1) of A (callable: step -> a0, a1) times the
 // operator rows T (this lane's element of step 0, column 0 of the part); `tiles` of its
 // column tiles exist.  `first`: the rows of the first block, loaded by tr_load.
@@ -102,7 +95,7 @@ __device__ __forceinline__ void tr_product(double (&acc)[Tr<P>::NTW][4], double 
 #pragma unroll
         for (int u = 0; u < C::UB; ++u)
 #pragma unroll
-            for (int i = 0; i < C::NTW; ++i) dmma(acc[i], a0[u], a1[u], first[u][i]);
+            for (int i = 0; i < C::NTW; ++i) sm100::dmma(acc[i], a0[u], a1[u], first[u][i]);
 #pragma unroll
         for (int u = 0; u < C::UB; ++u)
 #pragma unroll
