@@ -26,7 +26,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 constexpr int DT_WARPS = 8;
-constexpr int DT_CTAS = 2368;    // CTAs wanted: 4 waves of 148 x 4
+constexpr int DT_CTAS = 16 * SPLIT_SMS;    // CTAs wanted: 4 waves of 4 per SM
 
 // SOFT: the spline kernel of support hs (ogx_softening.cuh) instead of Plummer's eps2
 template <bool POT, bool SOFT>

@@ -36,6 +36,10 @@ constexpr int kHiLevels = 21;     // levels packed in the 64-bit key word
 constexpr int kPMax = 12;         // largest supported expansion order
 constexpr int kDegMax = kPMax + 2;
 
+// SMs that the rules for splitting work count with (the B200's; fixed rather than read from the
+// device, so that a result, which depends on the split's order of sums, does not depend on it)
+constexpr int SPLIT_SMS = 148;
+
 inline int num_dofs(int p) { return (p + 1) * (p + 1); }
 
 // ---- error plumbing ------------------------------------------------------

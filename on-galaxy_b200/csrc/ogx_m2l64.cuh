@@ -12,8 +12,9 @@
 namespace ogx {
 
 constexpr int M2L64_TGT = 64;        // targets per tile; the target layout is padded to 128
-constexpr int M2L64_ITEMS = 888;     // items wanted: 3 per CTA slot of 2 x 148 (2.5: 0.2 ms more of tail at 262,144 bodies)
+constexpr int M2L64_ITEMS = 6 * SPLIT_SMS;   // items wanted: 3 per CTA slot of 2 per SM (2.5: 0.2 ms more of tail at 262,144 bodies)
 constexpr int M2L64_MAXSPLIT = 27;
+constexpr int TC_ITEMS = 6 * SPLIT_SMS;      // most items (tile, slice, range) a split of the tensor-core M2L makes
 // k_target_groups' words behind the group starts gs[0..17]
 constexpr int GS_SPLIT = 18, GS_TILES = 19, GS_TICKET = 20, GS_FILL = 21, GS_TILES128 = 22, GS_TC_SPLIT = 23 /* for 1, 2, 3 slices */;
 
@@ -53,8 +54,8 @@ __host__ __device__ __forceinline__ int m2l_tc_split(int tiles, int slices) {
     const int n = tiles * slices;
     int best = 1;
     float cost = 1e30f;
-    for (int s = 1; s <= M2L64_MAXSPLIT && (s == 1 || n * s <= 888); ++s) {
-        const float c = (float)((n * s + 147) / 148) * (1.0f / (float)s + 0.045f);
+    for (int s = 1; s <= M2L64_MAXSPLIT && (s == 1 || n * s <= TC_ITEMS); ++s) {
+        const float c = (float)((n * s + SPLIT_SMS - 1) / SPLIT_SMS) * (1.0f / (float)s + 0.045f);
         if (c < cost * 0.999f) { cost = c; best = s; }
     }
     return best;
@@ -63,7 +64,7 @@ __host__ __device__ __forceinline__ int m2l_tc_split(int tiles, int slices) {
 inline size_t m2l_tc_partial_rows(int64_t ntgt, int slices) {
     size_t rows = 0;
     const int64_t most = (ntgt + 127) / 128 + 8;
-    for (int64_t n = 1; n <= most && n * slices <= 444; ++n) {
+    for (int64_t n = 1; n <= most && n * slices * 2 <= TC_ITEMS; ++n) {   // more are not split
         const int s = m2l_tc_split((int)n, slices);
         if (s > 1) {
             const size_t r = (size_t)s * (size_t)(128 * n < ntgt ? 128 * n : ntgt);
