@@ -263,9 +263,13 @@ constexpr int FAR_HW = 8;          // warps of a heavy leaf's CTA
 
 // Leaves with more M2P tasks (bodies x W boxes) than this are taken by a CTA of FAR_HW
 // warps (k_leaf_far_heavy), so that one leaf with a long W list does not decide the
-// kernel's length.  In small trees (fewer leaves than warps the GPU holds) and in FP64 a
-// task costs more of the kernel's length, so the line is lower.  (512 instead of 1,024: 1M
-// merger 3.66 -> 3.67 ms, three 262,144-body systems of order 4 1.06 -> 1.08.)
+// kernel's length.  That matters while the leaves are fewer than the warps the GPU holds, and
+// more in FP64, where a task takes longer.  One evaluation alone, lines 1,024 / 512 / 256 / 128
+// (us): 8,192 bodies (516 leaves) 403 / 381 / 373 / 373, 30,011 (1,855) 520 / 513 / 510 / 501;
+// FP64, 16,384 bodies (1,009) 964 / 933 / 917 / 913, 60,000 (3,480) 1,532 / 1,510 / 1,490 / 1,478.
+// In larger trees the lines 1,024, 512 and 256 lie within 1% of one another (1M merger 3.92 / 3.88 /
+// 3.91 ms, 262,144 bodies in FP64 3.31 ms each), and systems that share the GPU do better with
+// fewer heavy CTAs (three of 262,144 bodies, order 4: 1.06 ms at 1,024, 1.08 at 512).
 template <class T>
 __device__ __forceinline__ int64_t heavy_line(const TreeView& tv) { return sizeof(T) == 8 || tv_nleaf(tv) < 4096 ? 256 : 1024; }
 

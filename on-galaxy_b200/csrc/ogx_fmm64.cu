@@ -1,20 +1,22 @@
-// ogx_fmm64.cu -- the plain FP64 form of the adaptive FMM evaluation.
+// ogx_fmm64.cu -- the passes of an adaptive FMM evaluation, in the plain FP64 form (run_fp64, also
+// the third form) and in the mixed form (run_mixed*).
 //
 // Same passes as AdaptiveFMM3D::computeAccelerations (src3d/AdaptiveFMM3D.hpp:29-110)
 // but organised for the GPU:
-//   P2M           warp per leaf: lanes build harmonics of 32 bodies into shared
-//                 memory, then reduce columns (:53-61, FmmExpansions3D.hpp:148-163)
-//   M2M           bottom-up in one launch (groups of parents taken level by level,
-//                 each waiting for its children), warp per child octant,
-//                 level-independent matrices MM_s (:62-71)
-//   M2L           all levels in one launch on the FP64 matrix instructions
-//                 (ogx_m2l64.cu; :78-81; V list implicit in the colleague slots)
-//   P2L           warp per box over its X list (:82, :117-128)
-//   L2L           top-down in one launch, the same way (:75-77)
-//   leaf far      warp per leaf: L2P through gradient coefficients of L, M2P
-//                 over the W list through gradient coefficients of M (:92-93)
-//   leaf near     warp per leaf: softened P2P over the U list, j != i (:95-103),
-//                 then acc[orig] = G (far + near) (:104)
+//   P2M           one-warp block per leaf: a lane takes bodies, adds their terms of one
+//                 coefficient at a time to its column of sums (:53-61, ogx_p2x.cuh)
+//   M2M           bottom-up in one launch (items of 16 parents taken by ticket, each waiting
+//                 for its children) on the FP64 matrix instructions (:62-71, ogx_translate.cu)
+//   M2L           all levels in one launch: FP64 matrix instructions (ogx_m2l64.cu), rotations
+//                 (ogx_m2l_rot.cu) or the tensor cores (ogx_mixed_kernels.cuh); :78-81, the V
+//                 list implicit in the colleague slots
+//   P2L           one-warp block per box over its X list (:82, :117-128, ogx_p2x.cuh)
+//   L2L           top-down in one launch, the same way as M2M (:75-77)
+//   leaf far      L2P and, over the W lists, M2P from coefficient records, a warp per leaf or a
+//                 CTA per heavy leaf (:92-93, ogx_far.cuh)
+//   leaf near     softened P2P over the U list, j != i, a one-warp block per chunk of at most 32
+//                 targets of a leaf (:95-103, ogx_near.cuh)
+//   combine       acc[orig] = G (far + near) (:104)
 // Potentials (pot = -G Phi) are produced alongside when requested.
 #include <algorithm>
 #include <cstring>
@@ -110,8 +112,9 @@ __device__ __forceinline__ bool near_item(const TreeView& tv, const int64_t* chu
 // out[4 i] += sum_j m_j (g(r) - r^-3) (r_j - r_i) and, for potentials, m_j (k(r) - 1/r),
 // over the pairs closer than hs (the difference is zero beyond).  The far field took these
 // pairs with the Newtonian kernel; with this sum they carry the spline kernel's force.
-// Warp per leaf, lanes over the leaf's bodies, FP64 (the plain form; the mixed form runs
-// the FP32 near-field kernel over the same lists, k_leaf_near<Near32, .., 2>).
+// Warp per near-field work item (a leaf's chunk of 32 targets), a lane per target, FP64 (the
+// plain form; the mixed form runs the FP32 near-field kernel over the same lists,
+// k_leaf_near<Near32, .., 2>).
 template <bool POT>
 __global__ void __launch_bounds__(128) k_soft_correct(TreeView tv, const int64_t* __restrict__ chunk_off, double hs, double hinv,
                                                       double* out) {

@@ -403,8 +403,8 @@ inline int bits_for(int64_t v) {
 // field takes their pairs) and whose box lies within the spline's support `hs` of b's
 // box, found by a depth-first walk from the root that skips every box farther than hs.
 // Adjacency is the U-list predicate (AdaptiveOctree::adjacent, same FP64 operations), so
-// every leaf pair is either in b's U list or a candidate here.  Thread per leaf; pass 1
-// counts, pass 2 writes in the same order.
+// every leaf pair is either in b's U list or a candidate here.  Pass 1 counts, pass 2 writes
+// in the same order.
 //
 // Warp per leaf: the 32 boxes on top of a stack in shared memory are tested together, their
 // children pushed, so a walk takes a dozen rounds of loads (a thread per leaf took one box

@@ -81,9 +81,9 @@ def test_galaxy_262k_fp64_form_matches_oracle(ogx, oracle, galaxy262k, p):
 
 
 def test_galaxy_262k_fp64_form_one_launch_translations_match_oracle(ogx, oracle, galaxy262k):
-    """Leaf capacity 16: about 63k boxes, so M2M and L2L each run as one launch over all
-    levels (groups of parents taken by ticket, waiting on per-box ready flags) instead of
-    one launch per level; the FP64 form still equals the oracle to 1e-12."""
+    """Leaf capacity 16: about 63k boxes, so the one launch of M2M and of L2L (groups of parents
+    taken by ticket in level order, waiting on per-box ready flags) takes many groups per CTA;
+    the FP64 form still equals the oracle to 1e-12."""
     pos, mass = galaxy262k
     with ogx.AdaptiveFMM3D(p=4, threshold=16, precision=ogx.PREC_FP64) as s:
         acc = s.compute_accelerations(pos, mass)

@@ -3,11 +3,10 @@ FP64 translations), through the C ABI.
 
 Tolerances (stated per the precision design):
   * vs the FP64 form at the same p and leaf capacity: RMS <= 5e-6, max_rel <= 1e-3.
-    The budget is set by the FP32 near field: leaf-centred FP32 positions carry an
-    absolute error of 2^-24 x leaf size, so a pair at separation r gets a relative
-    force error ~3e-8 x leaf/r (measured on CPU for Plummer N=2000: RMS 2.6e-6);
-    the split M2L (three FP16 products of 11-bit halves, power-of-two scales,
-    FP32 accumulation per combination) contributes ~2^-22 per product;
+    What it shows is 1.5e-7 to 4e-7 (test_gpu_precision.py holds it to 6e-7): FP32 pair sums on
+    double-float coordinates (a pair's difference carries the FP32 relative accuracy of the
+    difference itself), and the split M2L (three FP16 products of 11-bit halves, power-of-two
+    scales, FP32 accumulation per combination), ~2^-22 per product;
   * vs the FP64 direct oracle: RMS within 5e-6 of the FP64 form's own truncation error.
 """
 import numpy as np
