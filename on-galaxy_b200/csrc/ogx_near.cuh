@@ -98,14 +98,14 @@ struct Near32 {
         st.v[3][e] = l.x; st.v[4][e] = l.y; st.v[5][e] = l.z;
         st.v[6][e] = h.w;
     }
-    // every part up to a multiple of 4: no mass, far away (a finite distance, no zero)
+    // every part up to a multiple of 4: no mass, far away on every axis.  (A target at exactly that
+    // point would make 0 / 0 of it; on the x axis alone a pair at +-float(1e18) did.)
     __device__ static __forceinline__ void pad(Stage& st, const Parts& pa, int n, int lane) {
         for (int i = lane; i < 4 * pa.G; i += 32) {
             const int p = i >> 2, c = pa.count(p, n), k = (c & ~3) + (i & 3);
             if ((c & 3) && k >= c) {
-                st.v[0][p * pa.S + k] = 1e18f;
 #pragma unroll
-                for (int a = 1; a < 7; ++a) st.v[a][p * pa.S + k] = 0.f;
+                for (int a = 0; a < 7; ++a) st.v[a][p * pa.S + k] = a == 0 ? 1.0e18f : a == 1 ? 1.1e18f : a == 2 ? 1.3e18f : 0.f;
             }
         }
     }

@@ -125,3 +125,17 @@ def test_mixed_with_leaves_held_large_by_the_eps_floor(ogx, softening):
     mx, rms = rel_err(a64, am)
     assert rms <= 1e-6 and mx <= 1e-3, (mx, rms)
     assert float(np.sqrt(np.mean((pm - p64) ** 2) / np.mean(p64 ** 2))) <= 1e-6
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_bodies_at_large_round_coordinates(ogx, axis):
+    """A pair at +-float32(1e18) on one axis: the near field pads its source parts with massless
+    points about that far away, and a target must not meet one (0 / 0)."""
+    pos = np.zeros((2, 3))
+    pos[:, axis] = np.float64(np.float32(1e18)) * np.array([1.0, -1.0])
+    mass = np.full(2, 1e30)
+    with ogx.AdaptiveFMM3D(p=4, threshold=64, precision=ogx.PREC_MIXED) as s:
+        acc = s.compute_accelerations(pos, mass)
+    ref = np.zeros((2, 3))
+    ref[:, axis] = -np.sign(pos[:, axis]) * 1e30 / (2.0 * pos[0, axis]) ** 2
+    assert rel_err(ref, acc)[0] <= 1e-6
